@@ -130,7 +130,8 @@ def _number(g, n, kind):
     if kind == "f32":
         return _measure(g, n).float()
     if kind == "decimal":
-        return _u32(g, n, 1_000_000).double().div_(100.0)
+        cents = _u32(g, n, 1_000_000).double()
+        return cents.div_(torch.full_like(cents, 100.0))     # a division, not a product with 1 / 100
     if kind == "i64":
         return _i64(g, n)
     return _u32(g, n, U32_RANGE)
