@@ -39,6 +39,7 @@ struct CqlKernelDesc
 extern const CqlKernelDesc cql_kernels_aggregate[];
 extern const CqlKernelDesc cql_kernels_scan[];
 extern const CqlKernelDesc cql_kernels_hash[];
+extern const CqlKernelDesc cql_kernels_group[];
 extern const CqlKernelDesc cql_kernels_join[];
 extern const CqlKernelDesc cql_kernels_sort[];
 extern const CqlKernelDesc cql_kernels_fixed[];

@@ -17,6 +17,7 @@
 // reference's 256 lanes per warp lane) so groups of a few rows do not idle 256 threads each, while
 // the per-lane t-digest centroid (first sample, weight) is computed for the same 256 lane positions.
 #include "cql_internal.cuh"
+#include "cql_bits.cuh"
 #include "cql_fixed.cuh"
 #include <algorithm>
 #include <float.h>
@@ -25,16 +26,6 @@
 #define HASH_THREADS 256
 #define EMPTY_SLOT 0xffffffffu
 #define PAST_END 0xfffffffeu
-
-__device__ __forceinline__ uint32_t hash_u32(uint32_t x)
-{
-  x ^= x >> 16;
-  x *= 0x7feb352du;
-  x ^= x >> 15;
-  x *= 0x846ca68bu;
-  x ^= x >> 16;
-  return x;
-}
 
 // ---------------------------------------------------------------------------------------------
 // aggregate_assign: binding 0 owner row per slot, 1 rows per slot, 2 slot per row, 3 overflow count,
@@ -529,15 +520,8 @@ static int launch_csr_scatter(const CqlLaunch& a, uint32_t gws, uint32_t lws, cu
 
 __device__ __forceinline__ void hll_add(uint32_t* sketch, uint64_t sketch_words, uint32_t slot, uint32_t g, uint32_t nhll, uint32_t p, double value)
 {
-  unsigned long long bits = (unsigned long long)__double_as_longlong(value);
-  uint32_t lo = (uint32_t)bits, hi = (uint32_t)(bits >> 32);
-  uint32_t h = hash_u32(lo ^ hash_u32(hi));
-  uint32_t rest_bits = 32u - p;
-  uint32_t bucket = h >> rest_bits;
-  uint32_t rest = h & ((1u << rest_bits) - 1u);
-  // findMSB: the index of the highest set bit, -1 for zero
-  int msb = rest ? 31 - __clz(rest) : -1;
-  uint32_t rho = msb < 0 ? rest_bits + 1u : rest_bits - (uint32_t)msb;
+  uint32_t bucket, rho;
+  cql_hll_place((unsigned long long)__double_as_longlong(value), p, &bucket, &rho);
   uint64_t idx = ((uint64_t)g * nhll + slot) * (1ull << p) + bucket;
   // registers only grow: a value read at least as large (even a stale one) makes the atomic redundant,
   // and after the first rows almost every value is below its register
@@ -991,31 +975,6 @@ static int launch_group_finish(const CqlLaunch& a, uint32_t gws, uint32_t lws, c
 // integer and FP32 rate): a value becomes the bits of its double, then a fixed-point whole number or an
 // order key.
 
-// the double bits of a 32-bit float (exact: subnormals normalized, infinities and NaN kept)
-__device__ __forceinline__ unsigned long long small_f32_bits(uint32_t b)
-{
-  unsigned long long sign = (unsigned long long)(b >> 31) << 63;
-  uint32_t e = (b >> 23) & 0xffu, m = b & 0x7fffffu;
-  if (e == 0xffu) return sign | 0x7ff0000000000000ull | ((unsigned long long)m << 29);
-  if (e == 0)
-  {
-    if (m == 0) return sign;
-    uint32_t shift = __clz(m) - 8;   // bring the leading one to bit 23
-    m = (m << shift) & 0x7fffffu;
-    return sign | ((unsigned long long)(1023 - 126 - shift) << 52) | ((unsigned long long)m << 29);
-  }
-  return sign | ((unsigned long long)(e - 127 + 1023) << 52) | ((unsigned long long)m << 29);
-}
-
-// the double bits of a whole number below 2^53 in magnitude (exact)
-__device__ __forceinline__ unsigned long long small_int_bits(long long v)
-{
-  if (v == 0) return 0;
-  unsigned long long sign = v < 0 ? 0x8000000000000000ull : 0ull, a = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
-  int p = 63 - __clzll(a);
-  return sign | ((unsigned long long)(1023 + p) << 52) | ((a << (52 - p)) & 0xfffffffffffffull);
-}
-
 // x * 2^s rounded to the nearest whole number (ties away from zero), for a finite double x given by its
 // bits; |x * 2^s| < 2^62 by the choice of s
 __device__ __forceinline__ long long small_fixed(unsigned long long b, int s)
@@ -1137,7 +1096,7 @@ __global__ void __launch_bounds__(HASH_THREADS) k_group_small(CqlLaunch a, uint6
         // the value as a whole number (whole-number columns, exact) and, where needed, as its double's bits
         long long whole = type == 7 ? (long long)(int)(uint32_t)raw[i] : (long long)raw[i];
         unsigned long long b = 0;
-        if (!whole_col) b = type == 3 ? small_f32_bits((uint32_t)raw[i]) : raw[i];
+        if (!whole_col) b = type == 3 ? cql_f32_bits((uint32_t)raw[i]) : raw[i];
         bool finite = whole_col || ((b >> 52) & 0x7ffu) != 0x7ffu;
         if (what & 1u)
         {
@@ -1163,7 +1122,7 @@ __global__ void __launch_bounds__(HASH_THREADS) k_group_small(CqlLaunch a, uint6
         }
         if (what & 2u)
         {
-          if (whole_col) b = small_int_bits(whole);
+          if (whole_col) b = cql_int_bits(whole);
           if (finite || !(b & 0xfffffffffffffull))   // NaN is left out
           {
             if ((b << 1) == 0) b = 0;   // -0.0 compares equal to +0.0
