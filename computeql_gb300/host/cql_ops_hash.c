@@ -14,6 +14,7 @@
  */
 #include "cqlops.h"
 #include "cql_ops_internal.h"
+#include "cql_group_plan.h"
 
 #include <math.h>
 #include <stdio.h>
@@ -856,6 +857,294 @@ static int group_direct(const CqlColumn* key, uint32_t expr_count, const uint32_
   return 1;
 }
 
+/* ---- the exact tables: numeric keys numbered in one 64-bit word, COUNT/SUM/AVG/MIN/MAX in one pass (cql_group_exact) ----
+   Every key becomes a digit: a whole number its distance from its range's start, a float its bits; the digits in
+   mixed radix number the group. The results are the member lists' (or, for whole numbers and decimals, the
+   fixed-point reduce's) with each f64 SUM rounded once from the exact sum, so `path` is reported as before. */
+#define EXACT_DIRECT_MAX (1ull << 24)
+#define EXACT_LOCAL_BYTES (200u * 1024u)
+#define EXACT_TABLE_BYTES (8ull << 30)
+#define EXACT_EMIT_SLOTS 65536u
+#define EXACT_ONE_READ_BYTES (192ull << 10)
+
+static uint64_t pow2_from(uint64_t n)
+{
+  uint64_t p = 1;
+  while (p < n) p <<= 1;
+  return p;
+}
+
+static int exact_type(const CqlColumn* c, uint64_t rows)
+{
+  return c && c->rows == rows && c->width == 0 && c->buffer &&
+         (c->type == CQLOPS_TYPE_U32 || c->type == CQLOPS_TYPE_I32 || c->type == CQLOPS_TYPE_F32 || c->type == CQLOPS_TYPE_F64 ||
+          c->type == CQLOPS_TYPE_U64 || c->type == CQLOPS_TYPE_I64);
+}
+
+/* the keys' digits; the product of their ranges in *out_product (0: 2^64). 0 when they do not fit one word. */
+static int exact_keys(CqlGroupPlan* p, const CqlColumn* keys, uint32_t key_count, uint64_t rows, uint64_t* out_product)
+{
+  unsigned __int128 product = 1, all = (unsigned __int128)1 << 64;
+  p->key_count = key_count;
+  for (uint32_t k = 0; k < key_count; k++)
+  {
+    const CqlColumn* c = &keys[k];
+    if (!exact_type(c, rows)) return 0;
+    uint32_t type = c->type;
+    unsigned __int128 range;
+    uint64_t min = 0;
+    int whole = type == CQLOPS_TYPE_U32 || type == CQLOPS_TYPE_I32 || type == CQLOPS_TYPE_U64 || type == CQLOPS_TYPE_I64;
+    /* (doubles tell whole numbers apart up to 2^53: the keys compare as f64 values) */
+    int ranged = whole && c->has_range && c->zone_min >= -9007199254740992.0 && c->zone_max <= 9007199254740992.0 && c->zone_min <= c->zone_max &&
+                 c->zone_min == floor(c->zone_min) && c->zone_max == floor(c->zone_max);
+    if (ranged)
+    {
+      min = (uint64_t)(int64_t)c->zone_min;
+      range = (unsigned __int128)(uint64_t)((int64_t)c->zone_max - (int64_t)c->zone_min) + 1;
+    }
+    else if (type == CQLOPS_TYPE_U32 || type == CQLOPS_TYPE_F32) range = (unsigned __int128)1 << 32;
+    else if (type == CQLOPS_TYPE_I32)
+    {
+      min = (uint64_t)INT64_C(-2147483648);
+      range = (unsigned __int128)1 << 32;
+    }
+    else
+    {
+      range = all;
+      if (type == CQLOPS_TYPE_U64) type = CQL_EXACT_KEY_U64_AS_F64;
+      if (type == CQLOPS_TYPE_I64) type = CQL_EXACT_KEY_I64_AS_F64;
+    }
+    p->key_type[k] = type;
+    p->key_min[k] = min;
+    p->key_range[k] = (uint64_t)range;   /* 0 for 2^64, which leaves room for no other key */
+    if (range == all && key_count > 1) return 0;
+    product *= range;
+    if (product > all) return 0;
+  }
+  *out_product = (uint64_t)product;
+  return 1;
+}
+
+/* the argument columns, what is kept of each, and the sums' units */
+static int exact_columns(CqlGroupPlan* p, const CqlColumn** cols, uint64_t rows, uint32_t expr_count, const uint32_t* funcs, const CqlColumn* const* args,
+                         int use_fixed, uint32_t fixed_scales)
+{
+  p->expr_count = expr_count;
+  p->decimals = (uint32_t)use_fixed;
+  for (uint32_t e = 0; e < expr_count; e++)
+  {
+    uint32_t f = funcs[e], i = 0;
+    if (f > CQLOPS_FUNC_MAX) return 0;
+    p->expr_func[e] = f;
+    if (f == CQLOPS_FUNC_COUNT) continue;
+    const CqlColumn* c = args[e];
+    if (!exact_type(c, rows)) return 0;
+    while (i < p->column_count && !(cols[i]->buffer == c->buffer && cols[i]->type == c->type)) i++;
+    if (i == p->column_count)
+    {
+      cols[i] = c;
+      p->col_type[i] = c->type;
+      if (c->type == CQLOPS_TYPE_U32 || c->type == CQLOPS_TYPE_I32) p->col_what[i] = CQL_EXACT_WHOLE;
+      else if (use_fixed)
+      {
+        if (c->type != CQLOPS_TYPE_F64) return 0;
+        p->col_what[i] = CQL_EXACT_DECIMAL;
+        p->col_scale[i] = (fixed_scales >> (4 * e)) & 0xfu;
+      }
+      p->column_count++;
+    }
+    p->expr_col[e] = i;
+    uint32_t want = f == CQLOPS_FUNC_MIN ? CQL_EXACT_MIN : f == CQLOPS_FUNC_MAX ? CQL_EXACT_MAX : CQL_EXACT_SUM;
+    if (!(p->col_what[i] & want))
+    {
+      p->col_what[i] |= want;
+      if (want == CQL_EXACT_SUM) p->col_sum[i] = p->sums++;
+      else if (want == CQL_EXACT_MIN) p->col_min[i] = p->mins++;
+      else p->col_max[i] = p->maxs++;
+    }
+  }
+  return 1;
+}
+
+/* the units of the f32/f64 (and 64-bit integer) sums: 2^base with the column's largest exponent at the window's top */
+static int exact_units(CqlGroupPlan* p, const CqlColumn* const* cols, uint64_t rows)
+{
+  double largest[CQL_EXACT_COLUMNS] = { 0 };
+  uint32_t measure = 0;
+  for (uint32_t i = 0; i < p->column_count; i++)
+  {
+    const CqlColumn* c = cols[i];
+    if (!(p->col_what[i] & CQL_EXACT_SUM) || (p->col_what[i] & (CQL_EXACT_WHOLE | CQL_EXACT_DECIMAL))) continue;
+    if (c->has_range && isfinite(c->zone_min) && isfinite(c->zone_max))
+      largest[i] = fabs(c->zone_min) > fabs(c->zone_max) ? fabs(c->zone_min) : fabs(c->zone_max);
+    else if (c->type == CQLOPS_TYPE_U64 || c->type == CQLOPS_TYPE_I64) largest[i] = 18446744073709551616.0;
+    else measure |= 1u << i;
+  }
+  if (measure && !finite_magnitudes(cols, p->column_count, measure, rows, largest)) return 0;
+  int pos_max = 73 - (int)p->low_bits;
+  for (uint32_t i = 0; i < p->column_count; i++)
+  {
+    if (!(p->col_what[i] & CQL_EXACT_SUM) || (p->col_what[i] & (CQL_EXACT_WHOLE | CQL_EXACT_DECIMAL))) continue;
+    uint64_t bits;
+    memcpy(&bits, &largest[i], 8);
+    int e = (int)((bits >> 52) & 0x7ff);
+    int base = (e ? e : 1) - 1075 - pos_max;
+    p->col_base[i] = base < -1074 ? -1074 : base;
+  }
+  return 1;
+}
+
+/* 1 done, 0 failed, -1 the query does not fit (or its data does not: the caller's general path answers it) */
+static int group_exact(const CqlColumn* keys, uint32_t key_count, uint64_t rows, uint32_t expr_count, const uint32_t* funcs,
+                       const CqlColumn* const* args, int use_fixed, uint32_t fixed_scales, uint64_t group_hint, uint64_t max_groups,
+                       uint64_t* out_group_count, uint64_t* out_repr_row, uint64_t* out_counts, double* out_results)
+{
+  CqlGroupPlan p;
+  memset(&p, 0, sizeof(p));
+  const CqlColumn* cols[CQL_EXACT_COLUMNS] = { NULL };
+  uint64_t product = 0;
+  if (rows >= (1ull << 31) || key_count == 0 || !exact_keys(&p, keys, key_count, rows, &product) ||
+      !exact_columns(&p, cols, rows, expr_count, funcs, args, use_fixed, fixed_scales))
+    return -1;
+  while ((1ull << p.low_bits) < rows) p.low_bits++;
+  p.low_bits++;
+  if (!exact_units(&p, cols, rows)) return 0;
+  CqlKernel* k = kernel("cql_group_exact");
+  CqlKernel* ke = kernel("cql_group_exact_emit");
+  CqlKernel* kb = kernel("cql_group_direct_bits");
+  CqlBuffer* pb = pooled("group_exact_plan", sizeof(CqlGroupPlan), CQLCUDA_BUFFER_READ_WRITE);
+  if (!k || !ke || !kb || !pb) return 0;
+  for (uint32_t i = 0; i < CQL_EXACT_KEYS; i++) cqlcuda_kernel_set_arg_buffer(k, i, keys[i < key_count ? i : 0].buffer);
+  for (uint32_t i = 0; i < CQL_EXACT_COLUMNS; i++) cqlcuda_kernel_set_arg_buffer(k, 4 + i, i < p.column_count ? cols[i]->buffer : keys[0].buffer);
+  /* how many groups: the hint, or the ranges' product where that is less */
+  uint64_t expected = group_hint;
+  if (product && (expected == 0 || expected > product)) expected = product <= EXACT_DIRECT_MAX || group_hint ? product : 0;
+  if (group_hint && expected > group_hint) expected = group_hint;
+  p.direct = product && product <= EXACT_DIRECT_MAX && product <= (group_hint ? 2 : 8) * rows;
+  /* A CTA's own table pays while merging it costs less than the rows' own updates would: at most half a merged group a
+     row over all CTAs, and what fits the SM. */
+  int local = 1;
+  uint64_t slot_bytes = (p.direct ? 0 : 8) + 8ull * (p.mins + p.maxs) + 16ull * p.sums + 12;
+  uint64_t table_slots = 0;
+  for (int attempt = 0; attempt < 12; attempt++)
+  {
+    p.local_slots = 0;
+    p.copies_log2 = 0;
+    if (local)
+    {
+      uint64_t n = p.direct ? product : expected ? expected : 1300;
+      while (expected && p.copies_log2 < 5 && (n << (p.copies_log2 + 1)) <= 512 && (p.direct || product >> 58 == 0)) p.copies_log2++;
+      uint64_t s = p.direct ? n << p.copies_log2 : pow2_from((n << p.copies_log2) * 3 / 2);
+      if (!p.direct && s < 256) s = 256;
+      uint64_t bytes = s * slot_bytes;
+      uint64_t per_cta = bytes <= 48 * 1024 ? 256 : bytes <= 104 * 1024 ? 512 : 1024;
+      uint64_t ctas = (rows + per_cta * 4 - 1) / (per_cta * 4), resident = (uint64_t)cqlcuda_sm_count() * (1024 / per_cta);
+      if (ctas > resident) ctas = resident;
+      if (bytes <= EXACT_LOCAL_BYTES && (n << p.copies_log2) * ctas <= rows / 2 + 1024) p.local_slots = (uint32_t)s;
+      else local = 0;
+    }
+    uint64_t most = pow2_from(2 * rows < 1024 ? 1024 : 2 * rows);
+    if (p.direct) table_slots = product;
+    else if (table_slots == 0)
+    {
+      uint64_t want = local ? 2ull * p.local_slots >> p.copies_log2 : expected ? 2 * expected : rows / 16;
+      table_slots = pow2_from(want < 1024 ? 1024 : want);
+    }
+    if (!p.direct && table_slots > most) table_slots = most;
+    if (table_slots > (1ull << 30)) return -1;
+    p.slots = (uint32_t)table_slots;
+    uint64_t ones = cql_exact_ones_bytes(&p), zeros = cql_exact_zero_bytes(&p);
+    if (ones + zeros > EXACT_TABLE_BYTES) return -1;
+    uint64_t cap = table_slots < rows ? table_slots : rows;
+    if (cap > max_groups) cap = max_groups;
+    if (cap == 0) cap = 1;
+    uint64_t counts_at = 64 + cap * 8, results_at = 64 + cap * 16, out_bytes = 64 + cap * (16 + 8ull * expr_count);
+    int listed = p.slots > EXACT_EMIT_SLOTS;
+    CqlBuffer* tab = pooled("group_exact_table", ones + zeros, CQLCUDA_BUFFER_READ_WRITE);
+    CqlBuffer* ob = pooled("group_exact_out", out_bytes, CQLCUDA_BUFFER_READ_WRITE);
+    CqlBuffer* bits = listed ? pooled("group_exact_bits", ((table_slots + 31) / 32) * 4, CQLCUDA_BUFFER_READ_WRITE) : NULL;
+    CqlBuffer* list = listed ? pooled("group_exact_list", cap * 4, CQLCUDA_BUFFER_READ_WRITE) : NULL;
+    if (!tab || !ob || (listed && (!bits || !list))) return 0;
+    cqlcuda_kernel_set_arg_buffer(k, 12, pb);
+    cqlcuda_kernel_set_arg_buffer(k, 13, tab);
+    cqlcuda_kernel_set_arg_buffer_range(k, 14, ob, 16, 4);
+    cqlcuda_kernel_set_arg_u64(k, 0, rows);
+    cqlcuda_kernel_set_arg_u64(k, 1, (uint64_t)p.local_slots | ((uint64_t)p.local_slots * slot_bytes) << 32);
+    cqlcuda_kernel_set_arg_u64(k, 2, p.direct);
+    cqlcuda_kernel_set_arg_u64(k, 3, p.slots);
+    cqlcuda_kernel_set_arg_u64(k, 4, ones + zeros);
+    cqlcuda_kernel_set_arg_buffer(ke, 0, tab);
+    cqlcuda_kernel_set_arg_buffer(ke, 1, pb);
+    cqlcuda_kernel_set_arg_buffer_range(ke, 2, ob, 16, 4);
+    cqlcuda_kernel_set_arg_buffer_range(ke, 3, ob, 0, 4);
+    cqlcuda_kernel_set_arg_buffer_range(ke, 4, ob, 64, cap * 8);
+    cqlcuda_kernel_set_arg_buffer_range(ke, 5, ob, counts_at, cap * 8);
+    cqlcuda_kernel_set_arg_buffer_range(ke, 6, ob, results_at, cap * 8 * expr_count);
+    cqlcuda_kernel_set_arg_buffer(ke, 7, listed ? list : ob);
+    cqlcuda_kernel_set_arg_buffer_range(ke, 8, ob, 32, 4);
+    cqlcuda_kernel_set_arg_u64(ke, 0, cap);
+    cqlcuda_kernel_set_arg_u64(ke, 1, (uint64_t)listed);
+    cqlcuda_kernel_set_arg_u64(ke, 2, expr_count);
+    cqlcuda_kernel_set_arg_u64(ke, 3, p.slots);
+    int one_read = out_bytes <= EXACT_ONE_READ_BYTES;
+    unsigned char head[64];
+    unsigned char* host = one_read ? (unsigned char*)malloc(out_bytes) : head;
+    if (!host) return 0;
+    CqlBatch* b = cqlcuda_batch_begin(sizeof(p), one_read ? out_bytes : 64);
+    cqlcuda_batch_buffer_write(b, pb, &p, sizeof(p));
+    cqlcuda_batch_buffer_fill(b, tab, ones, EMPTY);
+    cqlcuda_batch_fill_range(b, tab, ones, zeros, 0);
+    cqlcuda_batch_buffer_zero(b, ob, 64);
+    cqlcuda_batch_kernel_execute(b, k, (uint32_t)rows, QE_GPU_WORKGROUP_SIZE);
+    int ok = 1;
+    if (listed)
+    {
+      uint64_t cnt_at = ones + (24ull * p.sums + 8ull * p.maxs) * p.slots;
+      cqlcuda_kernel_set_arg_buffer_range(kb, 0, tab, cnt_at, 4ull * p.slots);
+      cqlcuda_kernel_set_arg_buffer(kb, 1, bits);
+      cqlcuda_kernel_set_arg_buffer_range(kb, 2, ob, 32, 4);
+      cqlcuda_kernel_set_arg_u64(kb, 0, p.slots);
+      cqlcuda_batch_kernel_execute(b, kb, p.slots, QE_GPU_WORKGROUP_SIZE);
+      ok = cqlops_bitmap_rows_enqueue(b, bits, 0, p.slots, list);
+    }
+    cqlcuda_batch_kernel_execute(b, ke, p.slots, QE_GPU_WORKGROUP_SIZE);
+    cqlcuda_batch_buffer_read(b, ob, host, one_read ? out_bytes : 64);
+    if (!cqlcuda_batch_end(b)) ok = 0;
+    uint32_t groups = 0, status = 0;
+    memcpy(&groups, host, 4);
+    memcpy(&status, host + 16, 4);
+    int result = !ok ? 0 : status ? -2 : groups > max_groups ? refuse("more groups than the output arrays hold") : 1;
+    if (result == 1 && one_read)
+    {
+      memcpy(out_repr_row, host + 64, (uint64_t)groups * 8);
+      memcpy(out_counts, host + counts_at, (uint64_t)groups * 8);
+      memcpy(out_results, host + results_at, (uint64_t)groups * 8 * expr_count);
+    }
+    if (one_read) free(host);
+    if (result == 1 && !one_read && groups)
+    {
+      b = cqlcuda_batch_begin(0, (uint64_t)groups * (16 + 8ull * expr_count) + 64);
+      cqlcuda_batch_buffer_read_at(b, ob, 64, out_repr_row, (uint64_t)groups * 8);
+      cqlcuda_batch_buffer_read_at(b, ob, counts_at, out_counts, (uint64_t)groups * 8);
+      cqlcuda_batch_buffer_read_at(b, ob, results_at, out_results, (uint64_t)groups * 8 * expr_count);
+      if (!cqlcuda_batch_end(b)) result = 0;
+    }
+    if (result == 1) *out_group_count = groups;
+    if (result != -2) return result;
+    if (status & (CQL_EXACT_RANGE | CQL_EXACT_KEY)) return -1;
+    /* more groups than expected: the table in device memory next, then a larger one */
+    if (p.direct || (!local && table_slots >= most)) return -1;
+    if (local)
+    {
+      local = 0;
+      table_slots = pow2_from(4 * expected > rows / 16 ? 4 * expected : rows / 16);
+      if (table_slots < 4096) table_slots = 4096;
+    }
+    else table_slots *= 8;
+  }
+  return -1;
+}
+
 int cqlops_group_hash(const CqlColumn* keys, uint32_t key_count, uint32_t expr_count, const uint32_t* funcs, const CqlColumn* const* args,
                       const double* params, uint64_t group_hint, uint32_t path, uint64_t max_groups, uint64_t* out_group_count,
                       uint64_t* out_repr_row, uint64_t* out_counts, double* out_results, uint32_t* out_path)
@@ -972,6 +1261,17 @@ int cqlops_group_hash(const CqlColumn* keys, uint32_t key_count, uint32_t expr_c
       if (out_path) *out_path = 1u;
       return 1;
     }
+  }
+  if (path == 0 && key_count > 0 && !has_sketch)
+  {
+    int r = group_exact(keys, key_count, rows, expr_count, funcs, args, use_fixed, fixed_scales, group_hint, max_groups, out_group_count,
+                        out_repr_row, out_counts, out_results);
+    if (r >= 0)
+    {
+      if (r == 1 && out_path) *out_path = use_fixed ? 2u : 1u;
+      return r;
+    }
+    cqlops_note_error("");
   }
   for (uint32_t c = 0; c < key_count; c++)
   {
