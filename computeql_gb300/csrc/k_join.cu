@@ -939,6 +939,344 @@ static int launch_join_dim_fold(const CqlLaunch& a, uint32_t gws, uint32_t lws, 
   return 0;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Join-aggregate by a hash table of the dim keys that carries each key's group (not a reference kernel: the
+// reference's probe, join_probe_native above, totals per dim row and the dim rows are grouped afterwards). With
+// unique dim keys and one small whole-number GROUP BY value (or none), a fact row's match is its group, so the totals
+// are kept per group in shared memory, in up to 32 copies so that the lanes of a warp do not meet, and
+// flushed once per CTA; the smallest kept dim row of each group comes along as a minimum.
+//
+//  cql_join_hash_build  binding 0 visits (u32 dim rows; unbound: rows 0..visits-1), 1 dim keys (u32), 2 dim group
+//                       values (word 12's type), 3 table (8-byte entries, all ones before), 4 error word, 5 the visits'
+//                       groups out (u32; with word 6 = 32); word 0 visits, word 2 1 = visit list given, word 4 log2 of
+//                       the table's size, word 6 the bits of a visit's number in an entry, word 8/9 the smallest group
+//                       value (f64 bits), word 10 group values given, word 12 their type (4 f64, 1 u32, 7 i32), word
+//                       14 the groups. Error bit 0: a key met twice, bit 1: a group value outside the groups.
+//                       An entry is the key (low word) and the group above the visit's number in the high word, or
+//                       the visit's number alone where the two do not fit 31 bits.
+//  cql_join_hash_probe  binding 0 fact keys, 1..4 arguments (u32/i32 words), 5 table, 6 totals out: counts u64 [G], sums
+//                       u64 [G][E], MIN i32 [G][E], MAX i32 [G][E], first visit u32 [G], 7 the visits' groups; word 0
+//                       rows, 2 expressions E, 4 functions, 6 argument per expression (4 bits each), 7 signed arguments
+//                       (bits), 8 log2 table size, 9 the bits of a visit's number, 10 groups G, 11 log2 copies
+//  cql_join_group_range binding 0 visits, 1 group values (f64), 2 result: (smallest, largest as order keys, 1 = a
+//                       value that is no whole number below 9e15), u64 each; word 0 visits, 2 1 = visit list given
+//
+// The probe costs one 8-byte load of a random sector a fact row beside the columns, which bounds it: the L1 takes a
+// warp's 32 different lines one a clock, and past L1 the sectors come from L2. Tables of at most JHASH_STAGED entries are
+// copied into shared memory instead, where 32 random 8-byte loads take a few clocks. Per dim row the totals took two
+// global atomics a row, and the table, its Bloom words, the totals' copies back and the grouping of the dim rows were
+// the host's: 50M rows and 100003 keys took 920 us of kernels and 1.2 ms of host work, now 240 us of kernels; 1M keys
+// 1700 us and 13 ms, now 490; 1500 keys 262 us and 0.2 ms, now 150.
+#define JHASH_THREADS 512
+#define JHASH_UNROLL 6   // with three CTAs an SM: against 8 and two, 231 to 247 us (100003 keys), 457 to 575 us (1M keys)
+#define JHASH_SMEM (96u * 1024u)
+#define JHASH_STAGED 8192u
+#define JHASH_EMPTY 0xffffffffffffffffull
+
+__global__ void __launch_bounds__(JOIN_THREADS) k_join_hash_build(CqlLaunch a, uint64_t visits)
+{
+  const uint32_t* visit_rows = (const uint32_t*)a.buf[0];
+  const uint32_t* dim_keys = (const uint32_t*)a.buf[1];
+  unsigned long long* table = (unsigned long long*)a.buf[3];
+  uint32_t* error = (uint32_t*)a.buf[4];
+  uint32_t* visit_group = (uint32_t*)a.buf[5];
+  bool listed = cql_word(a, 2) != 0, grouped = cql_word(a, 10) != 0;
+  uint32_t log2_size = cql_word(a, 4), visit_bits = cql_word(a, 6), type = cql_word(a, 12), groups = cql_word(a, 14), mask = (1u << log2_size) - 1u;
+  double group_min = __longlong_as_double((long long)a.push[4]);
+  bool group_f64 = type != 1u && type != 7u;
+  uint64_t dim_rows = a.bytes[1] / 4, value_rows = a.bytes[2] / (group_f64 ? 8 : 4);
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < visits; v += (uint64_t)gridDim.x * blockDim.x)
+  {
+    uint64_t row = listed ? visit_rows[v] : v;
+    if (row >= dim_rows || (grouped && row >= value_rows)) continue;
+    uint32_t key = dim_keys[row], g = 0;
+    if (grouped)
+    {
+      double off = (group_f64 ? ((const double*)a.buf[2])[row] : type == 7u ? (double)((const int*)a.buf[2])[row] : (double)((const uint32_t*)a.buf[2])[row]) - group_min;
+      if (!(off >= 0.0 && off < (double)groups))
+      {
+        atomicOr(error, 2u);
+        continue;
+      }
+      g = (uint32_t)off;
+    }
+    uint32_t high = (uint32_t)v;
+    if (visit_bits < 32u) high |= g << visit_bits;
+    else visit_group[v] = g;
+    unsigned long long entry = ((unsigned long long)high << 32) | key;
+    uint32_t slot = (key * 0x9E3779B1u) >> (32u - log2_size);
+    for (uint32_t p = 0; p <= mask; p++)   // at most half the slots are taken
+    {
+      unsigned long long old = atomicCAS(&table[slot], JHASH_EMPTY, entry);
+      if (old == JHASH_EMPTY) break;
+      if ((uint32_t)old == key)
+      {
+        atomicOr(error, 1u);
+        break;
+      }
+      slot = (slot + 1u) & mask;
+    }
+  }
+}
+
+static int launch_join_hash_build(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t visits = a.push[0];
+  uint32_t log2_size = cql_word(a, 4);
+  if (visits == 0) return 0;
+  if (visits > 0xffffffffull || log2_size == 0 || log2_size > 28 || visits * 2 > (1ull << log2_size) || a.bytes[3] < (8ull << log2_size) || a.bytes[4] < 4)
+    return (int)cudaErrorInvalidValue;
+  uint32_t visit_bits = cql_word(a, 6);
+  if (visit_bits >= 32 ? a.bytes[5] < visits * 4
+                       : visits > (1ull << visit_bits) || ((uint64_t)cql_word(a, 14) << visit_bits) > (1ull << 31))
+    return (int)cudaErrorInvalidValue;
+  k_join_hash_build<<<cql_stream_grid((visits + JOIN_THREADS - 1) / JOIN_THREADS, 8), JOIN_THREADS, 0, stream>>>(a, visits);
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
+template <bool PACKED, bool STAGED>
+__global__ void __launch_bounds__(JHASH_THREADS, 3) k_join_hash_probe(CqlLaunch a, uint64_t rows)
+{
+  extern __shared__ __align__(16) uint32_t jhash_mem[];
+  const uint32_t* fact = (const uint32_t*)a.buf[0];
+  const unsigned long long* global_table = (const unsigned long long*)a.buf[5];
+  const uint32_t* visit_group = (const uint32_t*)a.buf[7];
+  const uint32_t exprs = cql_word(a, 2), funcs = cql_word(a, 4), arg_index = cql_word(a, 6), arg_signed = cql_word(a, 7);
+  const uint32_t log2_size = cql_word(a, 8), mask = (1u << log2_size) - 1u, G = cql_word(a, 10), copies_log2 = cql_word(a, 11);
+  const uint32_t visit_bits = cql_word(a, 9), visit_mask = PACKED ? (1u << visit_bits) - 1u : 0xffffffffu;
+  const unsigned long long* staged = (const unsigned long long*)jhash_mem;
+  uint32_t* jsmem = jhash_mem + (STAGED ? 2u * (mask + 1u) : 0u);
+  const uint32_t cells = G << copies_log2, copy = threadIdx.x & ((1u << copies_log2) - 1u);
+  uint32_t used_args = 0, words = 1;   // a cell's words: the count, then per expression a sum's two halves or an extremum
+  for (uint32_t e = 0; e < exprs; e++)
+  {
+    uint32_t f = (funcs >> (4 * e)) & 0xfu;
+    if (f == JFUNC_COUNT) continue;
+    used_args |= 1u << ((arg_index >> (4 * e)) & 0x3u);
+    words += f == JFUNC_SUM ? 2 : 1;
+  }
+  uint32_t* s_first = jsmem + words * cells;
+  for (uint32_t i = threadIdx.x; i < words * cells; i += JHASH_THREADS) jsmem[i] = 0u;
+  for (uint32_t i = threadIdx.x; i < G; i += JHASH_THREADS) s_first[i] = 0xffffffffu;
+  if (STAGED)
+    for (uint32_t i = threadIdx.x; i <= mask; i += JHASH_THREADS) ((unsigned long long*)jhash_mem)[i] = __ldg(&global_table[i]);
+  uint32_t at = 1;
+  __syncthreads();
+  for (uint32_t e = 0; e < exprs; e++)
+  {
+    uint32_t f = (funcs >> (4 * e)) & 0xfu;
+    if (f == JFUNC_COUNT) continue;
+    if (f == JFUNC_MIN || f == JFUNC_MAX)
+      for (uint32_t i = threadIdx.x; i < cells; i += JHASH_THREADS) jsmem[at * cells + i] = f == JFUNC_MIN ? 0x7fffffffu : 0x80000000u;
+    at += f == JFUNC_SUM ? 2 : 1;
+  }
+  __syncthreads();
+  const uint64_t stride = (uint64_t)gridDim.x * JHASH_THREADS;
+  for (uint64_t base = (uint64_t)blockIdx.x * JHASH_THREADS + threadIdx.x; base < rows; base += stride * JHASH_UNROLL)
+  {
+    uint32_t key[JHASH_UNROLL];
+#pragma unroll
+    for (uint32_t u = 0; u < JHASH_UNROLL; u++) key[u] = base + u * stride < rows ? __ldcs(fact + base + u * stride) : 0u;
+    // each row's first entry, all loads in flight together; a row whose chain goes on walks it below
+    uint32_t cell[JHASH_UNROLL];
+    {
+      unsigned long long entry[JHASH_UNROLL];
+#pragma unroll
+      for (uint32_t u = 0; u < JHASH_UNROLL; u++)
+      {
+        uint32_t slot = (key[u] * 0x9E3779B1u) >> (32u - log2_size);
+        entry[u] = STAGED ? staged[slot] : __ldg(&global_table[slot]);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < JHASH_UNROLL; u++)
+      {
+        unsigned long long t = entry[u];
+        uint32_t slot = (key[u] * 0x9E3779B1u) >> (32u - log2_size);
+        for (uint32_t p = 0; t != JHASH_EMPTY && (uint32_t)t != key[u] && p <= mask; p++)
+        {
+          slot = (slot + 1u) & mask;
+          t = STAGED ? staged[slot] : __ldg(&global_table[slot]);
+        }
+        bool match = base + u * stride < rows && t != JHASH_EMPTY && (uint32_t)t == key[u];
+        uint32_t high = (uint32_t)(t >> 32), visit = high & visit_mask, g = 0;
+        if (match) g = PACKED ? high >> visit_bits : __ldg(&visit_group[visit]);
+        cell[u] = match ? (g << copies_log2) + copy : 0xffffffffu;
+        if (match && visit < s_first[g]) atomicMin(&s_first[g], visit);
+      }
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < JHASH_UNROLL; u++)
+      if (cell[u] != 0xffffffffu) atomicAdd(&jsmem[cell[u]], 1u);
+    uint32_t word = 1;
+#pragma unroll 1
+    for (uint32_t e = 0; e < exprs; e++)
+    {
+      uint32_t f = (funcs >> (4 * e)) & 0xfu;
+      if (f == JFUNC_COUNT) continue;
+      uint32_t ai = (arg_index >> (4 * e)) & 0x3u;
+      bool is_signed = ((arg_signed >> ai) & 1u) != 0;
+      const uint32_t* arg = (const uint32_t*)a.buf[1 + ai];
+      uint32_t w[JHASH_UNROLL];
+#pragma unroll
+      for (uint32_t u = 0; u < JHASH_UNROLL; u++) w[u] = cell[u] != 0xffffffffu ? __ldcs(arg + base + u * stride) : 0u;
+      uint32_t* lo = jsmem + word * cells;
+      uint32_t* hi = lo + cells;
+#pragma unroll
+      for (uint32_t u = 0; u < JHASH_UNROLL; u++)
+      {
+        if (cell[u] == 0xffffffffu) continue;
+        if (f == JFUNC_SUM)
+        {
+          uint32_t old = atomicAdd(&lo[cell[u]], w[u]);
+          uint32_t up = ((is_signed && (int)w[u] < 0) ? 0xffffffffu : 0u) + ((old + w[u] < old) ? 1u : 0u);
+          if (up) atomicAdd(&hi[cell[u]], up);
+        }
+        else if (f == JFUNC_MIN) atomicMin((int*)&lo[cell[u]], (int)w[u]);
+        else atomicMax((int*)&lo[cell[u]], (int)w[u]);
+      }
+      word += f == JFUNC_SUM ? 2 : 1;
+    }
+  }
+  __syncthreads();
+  unsigned long long* counts = (unsigned long long*)a.buf[6];
+  unsigned long long* sums = counts + G;
+  int* mins = (int*)(sums + (uint64_t)G * exprs);
+  int* maxs = mins + (uint64_t)G * exprs;
+  uint32_t* first = (uint32_t*)(maxs + (uint64_t)G * exprs);
+  for (uint32_t g = threadIdx.x; g < G; g += JHASH_THREADS)
+  {
+    uint32_t n = 0;
+    for (uint32_t c = 0; c < (1u << copies_log2); c++) n += jsmem[(g << copies_log2) + c];
+    if (n == 0) continue;
+    atomicAdd(&counts[g], (unsigned long long)n);
+    atomicMin(&first[g], s_first[g]);
+    uint32_t word = 1;
+    for (uint32_t e = 0; e < exprs; e++)
+    {
+      uint32_t f = (funcs >> (4 * e)) & 0xfu;
+      if (f == JFUNC_COUNT) continue;
+      const uint32_t* lo = jsmem + word * cells + (g << copies_log2);
+      uint64_t index = (uint64_t)g * exprs + e;
+      if (f == JFUNC_SUM)
+      {
+        unsigned long long s = 0;
+        for (uint32_t c = 0; c < (1u << copies_log2); c++) s += ((unsigned long long)lo[cells + c] << 32) + lo[c];
+        atomicAdd(&sums[index], s);
+      }
+      else
+      {
+        int x = (int)lo[0];
+        for (uint32_t c = 1; c < (1u << copies_log2); c++) x = f == JFUNC_MIN ? min(x, (int)lo[c]) : max(x, (int)lo[c]);
+        if (f == JFUNC_MIN) atomicMin(&mins[index], x);
+        else atomicMax(&maxs[index], x);
+      }
+      word += f == JFUNC_SUM ? 2 : 1;
+    }
+  }
+}
+
+static int launch_join_hash_probe(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t rows = a.push[0];
+  uint32_t exprs = cql_word(a, 2), funcs = cql_word(a, 4), arg_index = cql_word(a, 6), log2_size = cql_word(a, 8), G = cql_word(a, 10), cl = cql_word(a, 11);
+  if (rows == 0) return 0;
+  if (rows > 0xffffffffull || exprs == 0 || exprs > 8 || log2_size == 0 || log2_size > 28 || G == 0 || cl > 5 || a.bytes[0] < rows * 4 ||
+      a.bytes[5] < (8ull << log2_size) || a.bytes[6] < (uint64_t)G * (12 + 16ull * exprs))
+    return (int)cudaErrorInvalidValue;
+  uint64_t words = 1;
+  for (uint32_t e = 0; e < exprs; e++)
+  {
+    uint32_t f = (funcs >> (4 * e)) & 0xfu;
+    if (f == JFUNC_COUNT) continue;
+    if (!(f == JFUNC_SUM || f == JFUNC_MIN || f == JFUNC_MAX) || a.bytes[1 + ((arg_index >> (4 * e)) & 3u)] < rows * 4) return (int)cudaErrorInvalidValue;
+    words += f == JFUNC_SUM ? 2 : 1;
+  }
+  uint64_t smem = 4 * ((words << cl) + 1) * G;
+  if (smem > JHASH_SMEM) return (int)cudaErrorInvalidValue;
+  bool packed = cql_word(a, 9) < 32;
+  // staged beside the totals while two CTAs or more still share an SM
+  bool staged = packed && (1u << log2_size) <= JHASH_STAGED && smem + (8ull << log2_size) <= JHASH_SMEM;
+  if (staged) smem += 8ull << log2_size;
+  const void* fn = staged ? (const void*)k_join_hash_probe<true, true> : packed ? (const void*)k_join_hash_probe<true, false> : (const void*)k_join_hash_probe<false, false>;
+  if (smem > 40 * 1024)
+  {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)JHASH_SMEM);
+    if (e != cudaSuccess) return (int)e;
+  }
+  int per_sm = (int)std::min<uint64_t>(3, 220 * 1024 / (smem + 1024));
+  uint32_t grid = cql_stream_grid((rows + JHASH_THREADS * JHASH_UNROLL - 1) / (JHASH_THREADS * JHASH_UNROLL), per_sm);
+  if (staged) k_join_hash_probe<true, true><<<grid, JHASH_THREADS, smem, stream>>>(a, rows);
+  else if (packed) k_join_hash_probe<true, false><<<grid, JHASH_THREADS, smem, stream>>>(a, rows);
+  else k_join_hash_probe<false, false><<<grid, JHASH_THREADS, smem, stream>>>(a, rows);
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
+__global__ void __launch_bounds__(JOIN_THREADS) k_join_group_range(CqlLaunch a, uint64_t visits)
+{
+  __shared__ unsigned long long s_lo, s_hi;
+  __shared__ uint32_t s_bad;
+  if (threadIdx.x == 0)
+  {
+    s_lo = ~0ull;
+    s_hi = 0ull;
+    s_bad = 0;
+  }
+  __syncthreads();
+  const uint32_t* visit_rows = (const uint32_t*)a.buf[0];
+  const double* value = (const double*)a.buf[1];
+  bool listed = cql_word(a, 2) != 0;
+  uint64_t value_rows = a.bytes[1] / 8;
+  unsigned long long lo = ~0ull, hi = 0ull;
+  uint32_t bad = 0;
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < visits; v += (uint64_t)gridDim.x * blockDim.x)
+  {
+    uint64_t row = listed ? visit_rows[v] : v;
+    if (row >= value_rows)
+    {
+      bad = 1;
+      continue;
+    }
+    double x = value[row];
+    if (!(x >= -9.0e15 && x <= 9.0e15) || x != trunc(x) || __double_as_longlong(x) == (long long)0x8000000000000000ull)
+    {
+      bad = 1;
+      continue;
+    }
+    unsigned long long o = cql_f64_order_key(x);
+    lo = min(lo, o);
+    hi = max(hi, o);
+  }
+  if (lo != ~0ull) atomicMin(&s_lo, lo);
+  if (hi != 0ull) atomicMax(&s_hi, hi);
+  if (bad) s_bad = 1;
+  __syncthreads();
+  unsigned long long* out = (unsigned long long*)a.buf[2];
+  if (threadIdx.x == 0)
+  {
+    if (s_lo != ~0ull) atomicMin(&out[0], s_lo);
+    if (s_hi != 0ull) atomicMax(&out[1], s_hi);
+    if (s_bad) atomicMax(&out[2], 1ull);
+  }
+}
+
+static int launch_join_group_range(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t visits = a.push[0];
+  if (visits == 0) return 0;
+  if (a.bytes[2] < 24) return (int)cudaErrorInvalidValue;
+  k_join_group_range<<<cql_stream_grid((visits + JOIN_THREADS - 1) / JOIN_THREADS, 4), JOIN_THREADS, 0, stream>>>(a, visits);
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
 const CqlKernelDesc cql_kernels_join[] = {
   { "hash_join_build_count", launch_join_build_count },
   { "prefix_sum", launch_prefix_sum },
@@ -950,5 +1288,8 @@ const CqlKernelDesc cql_kernels_join[] = {
   { "cql_join_lut_map", launch_join_lut_map },
   { "cql_join_lut_first", launch_join_lut_first },
   { "cql_join_dim_fold", launch_join_dim_fold },
+  { "cql_join_hash_build", launch_join_hash_build },
+  { "cql_join_hash_probe", launch_join_hash_probe },
+  { "cql_join_group_range", launch_join_group_range },
   { nullptr, nullptr },
 };

@@ -972,6 +972,266 @@ static int slot_by_first(const void* a, const void* b)
   return x < y ? -1 : (x > y);
 }
 
+/* The groups of totals per slot read back to `host` (counts u64 at 0, sums i64, MIN and MAX i32, first visits u32 at
+   their offsets): the slots with a first visit, in its order, as the host pass meets them. */
+static int join_slots_finish(const CqlJoinAgg* q, uint32_t core_count, const uint32_t* core_of_expr, uint64_t slots, const unsigned char* host,
+                             uint64_t sums_at, uint64_t mins_at, uint64_t maxs_at, uint64_t first_at, uint64_t max_groups, uint64_t* out_groups,
+                             uint64_t* out_group_dim_row, double* out_results)
+{
+  const uint64_t* counts = (const uint64_t*)(host);
+  const int64_t* sums = (const int64_t*)(host + sums_at);
+  const int32_t* mins = (const int32_t*)(host + mins_at);
+  const int32_t* maxs = (const int32_t*)(host + maxs_at);
+  const uint32_t* first = (const uint32_t*)(host + first_at);
+  SlotFirst* order = (SlotFirst*)malloc(slots * sizeof(SlotFirst));
+  uint64_t groups = 0;
+  int ok = order != NULL;
+  for (uint64_t s2 = 0; ok && s2 < slots; s2++)
+    if (first[s2] != 0xffffffffu)
+    {
+      order[groups].first = first[s2];
+      order[groups].slot = (uint32_t)s2;
+      groups++;
+    }
+  if (ok && groups > max_groups) ok = refuse("more groups than the output arrays hold");
+  if (ok)
+  {
+    /* groups in the order of their first kept dim row, as the host pass meets them */
+    qsort(order, groups, sizeof(SlotFirst), slot_by_first);
+    for (uint64_t g = 0; g < groups; g++)
+    {
+      uint64_t s2 = order[g].slot;
+      out_group_dim_row[g] = q->dim_rows ? q->dim_rows[order[g].first] : order[g].first;
+      for (uint32_t e = 0; e < q->expr_count; e++)
+      {
+        uint64_t c = s2 * core_count + core_of_expr[e];
+        double r;
+        switch (q->funcs[e])
+        {
+          case CQLOPS_FUNC_COUNT: r = (double)counts[s2]; break;
+          case CQLOPS_FUNC_SUM: r = (double)sums[c]; break;
+          case CQLOPS_FUNC_AVG: r = counts[s2] ? (double)sums[c] / (double)counts[s2] : 0.0; break;
+          case CQLOPS_FUNC_MIN: r = (double)mins[c]; break;
+          default: r = (double)maxs[c]; break;
+        }
+        out_results[g * q->expr_count + e] = r;
+      }
+    }
+    *out_groups = groups;
+  }
+  free(order);
+  return ok;
+}
+
+/* ---- a hash table of the dim keys that carries each key's group (cql_join_hash_build, cql_join_hash_probe) ----
+   For fact keys over a wide range, with unique dim keys and one small whole-number GROUP BY value (or none): the table
+   is built on the device, each fact row's match is its group, and the totals are kept per group, so nothing is
+   kept per dim row. The group values' range comes from the resident column's zone or from the values themselves
+   (on the device past JHASH_HOST_VISITS of them: the host reads about a value a nanosecond, a launch and its wait cost
+   some 20 us). Gives way (-1) for duplicate keys, other group values, dim-side aggregates, narrow fact columns, and
+   more groups than a CTA's shared memory holds. */
+#define JHASH_SMEM_BYTES (96u * 1024u)
+#define JHASH_SMEM_WANTED (32u * 1024u)
+#define JHASH_HOST_VISITS 16384u
+
+static double order_key_value(uint64_t k)
+{
+  uint64_t b = (k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k;
+  double v;
+  memcpy(&v, &b, 8);
+  return v;
+}
+
+static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const uint32_t* core_funcs, const CqlColumn* const* core_cols,
+                               const uint32_t* core_of_expr, uint64_t max_groups, uint64_t* out_groups, uint64_t* out_group_dim_row,
+                               double* out_results)
+{
+  const CqlColumn* fk = q->fact_key;
+  uint64_t rows = fk->rows, D = q->dim_table_rows, visits = q->dim_rows ? q->dim_count : D;
+  if (!fk->buffer || fk->width != 0 || q->group_count > 1 || visits == 0 || D == 0 || D > PROBE_STREAM_MAX_DIM_ROWS || visits > PROBE_STREAM_MAX_DIM_ROWS)
+    return -1;
+  for (uint32_t e = 0; q->dim_args && e < q->expr_count; e++)
+    if (q->dim_args[e]) return -1;
+  const CqlColumn* args[4] = { 0 };
+  uint32_t arg_count = 0, funcs = 0, arg_index = 0, arg_signed = 0, words = 1, extrema = 0;
+  for (uint32_t c = 0; c < core_count; c++)
+  {
+    funcs |= (core_funcs[c] & 0xfu) << (4 * c);
+    if (core_funcs[c] == CQLOPS_FUNC_COUNT) continue;
+    const CqlColumn* a = core_cols[c];
+    if (!a || !(a->type == CQLOPS_TYPE_U32 || a->type == CQLOPS_TYPE_I32) || a->rows != rows || a->width != 0 || !a->buffer) return -1;
+    int extremum = core_funcs[c] == CQLOPS_FUNC_MIN || core_funcs[c] == CQLOPS_FUNC_MAX;
+    if (extremum && (!a->has_range || a->zone_min < -2147483648.0 || a->zone_max > 2147483647.0)) return -1;
+    uint32_t i = 0;
+    while (i < arg_count && args[i] != a) i++;
+    if (i == arg_count)
+    {
+      if (arg_count == 4) return -1;
+      args[arg_count++] = a;
+    }
+    arg_index |= i << (4 * c);
+    if (a->type == CQLOPS_TYPE_I32) arg_signed |= 1u << i;
+    words += extremum ? 1 : 2;
+    extrema |= (uint32_t)extremum;
+  }
+  const CqlColumn* dkc = q->dim_key_column;
+  const CqlColumn* dgc = q->group_count ? q->dim_group_column : NULL;
+  int dev_keys = dkc && dkc->buffer && dkc->width == 0 && dkc->rows == D && (dkc->type == CQLOPS_TYPE_U32 || dkc->type == CQLOPS_TYPE_I32);
+  int dev_groups = dev_keys && dgc && dgc->buffer && dgc->width == 0 && dgc->rows == D && dgc->has_range &&
+                   (dgc->type == CQLOPS_TYPE_U32 || dgc->type == CQLOPS_TYPE_I32);
+  const double* gv = q->group_count ? q->dim_group_values[0] : NULL;
+  uint32_t* visit_list = NULL;
+  if (q->dim_rows)
+  {
+    visit_list = (uint32_t*)malloc(visits * 4);
+    if (!visit_list) return refuse("out of host memory");
+    for (uint64_t v = 0; v < visits; v++)
+    {
+      if (q->dim_rows[v] >= D)
+      {
+        free(visit_list);
+        return -1;
+      }
+      visit_list[v] = (uint32_t)q->dim_rows[v];
+    }
+  }
+  CqlBuffer* vbuf = pooled("join_hash_visits", visit_list ? visits * 4 : 4, CQLCUDA_BUFFER_WRITE);
+  CqlBuffer* kbuf = dev_keys ? dkc->buffer : pooled("join_hash_dim_keys", D * 4, CQLCUDA_BUFFER_WRITE);
+  CqlBuffer* gbuf = dev_groups ? dgc->buffer : pooled("join_hash_group_values", gv ? D * 8 : 8, CQLCUDA_BUFFER_WRITE);
+  int ok = vbuf && kbuf && gbuf;
+  /* the groups: the values from the smallest on */
+  double vmin = 0.0, vmax = 0.0;
+  int fits = 1, uploaded = 0;
+  if (ok && gv && dev_groups)
+  {
+    vmin = dgc->zone_min;
+    vmax = dgc->zone_max;
+  }
+  else if (ok && gv && visits <= JHASH_HOST_VISITS)
+  {
+    vmin = HUGE_VAL;
+    vmax = -HUGE_VAL;
+    for (uint64_t v = 0; v < visits && fits; v++)
+    {
+      double x = gv[visit_list ? visit_list[v] : v];
+      if (!(x >= -9.0e15 && x <= 9.0e15) || x != (double)(int64_t)x || (x == 0.0 && signbit(x))) fits = 0;
+      if (x < vmin) vmin = x;
+      if (x > vmax) vmax = x;
+    }
+  }
+  else if (ok && gv)
+  {
+    CqlBuffer* rb = pooled("join_hash_range", 24, CQLCUDA_BUFFER_READ_WRITE);
+    CqlKernel* kr = kernel("cql_join_group_range");
+    uint64_t range[3] = { ~0ull, 0, 0 };
+    ok = rb && kr;
+    if (ok)
+    {
+      cqlcuda_kernel_set_arg_buffer(kr, 0, vbuf);
+      cqlcuda_kernel_set_arg_buffer(kr, 1, gbuf);
+      cqlcuda_kernel_set_arg_buffer(kr, 2, rb);
+      cqlcuda_kernel_set_arg_u64(kr, 0, visits);
+      cqlcuda_kernel_set_arg_u64(kr, 1, visit_list ? 1 : 0);
+      CqlBatch* b = cqlcuda_batch_begin(visits * 12, 24);
+      if (visit_list) cqlcuda_batch_buffer_write(b, vbuf, visit_list, visits * 4);
+      cqlcuda_batch_buffer_write(b, gbuf, gv, D * 8);
+      cqlcuda_batch_buffer_write(b, rb, range, 24);
+      cqlcuda_batch_kernel_execute(b, kr, (uint32_t)visits, QE_GPU_WORKGROUP_SIZE);
+      cqlcuda_batch_buffer_read(b, rb, range, 24);
+      ok = cqlcuda_batch_end(b);
+      uploaded = 1;
+      if (range[2] || range[0] > range[1]) fits = 0;
+      vmin = order_key_value(range[0]);
+      vmax = order_key_value(range[1]);
+    }
+  }
+  if (!ok || !fits || !(vmax - vmin <= 65535.0))
+  {
+    free(visit_list);
+    return ok ? -1 : 0;
+  }
+  uint64_t slots = gv ? (uint64_t)(vmax - vmin) + 1 : 1, E = core_count;
+  uint32_t copies_log2 = 5;
+  while (copies_log2 > 0 && 4ull * ((words << copies_log2) + 1) * slots > JHASH_SMEM_WANTED) copies_log2--;
+  if (4ull * ((words << copies_log2) + 1) * slots > JHASH_SMEM_BYTES)
+  {
+    free(visit_list);
+    return -1;
+  }
+  uint32_t log2_size = 4;
+  while ((1ull << log2_size) < visits * 2) log2_size++;
+  uint64_t sums_at = slots * 8, mins_at = sums_at + slots * E * 8, maxs_at = mins_at + slots * E * 4, first_at = maxs_at + slots * E * 4,
+           error_at = (first_at + slots * 4 + 15) & ~15ull, bytes = error_at + 16;
+  /* a group and a visit's number share a word of the entry where they fit 31 bits */
+  uint32_t visit_bits = 0;
+  while ((1ull << visit_bits) < visits) visit_bits++;
+  if ((slots << visit_bits) > (1ull << 31)) visit_bits = 32;
+  CqlBuffer* table = pooled("join_hash_table", 8ull << log2_size, CQLCUDA_BUFFER_READ_WRITE);
+  CqlBuffer* visit_group = pooled("join_hash_visit_groups", visit_bits == 32 ? visits * 4 : 4, CQLCUDA_BUFFER_READ_WRITE);
+  CqlBuffer* out = pooled("join_hash_slots", bytes, CQLCUDA_BUFFER_READ_WRITE);
+  CqlKernel* kb = kernel("cql_join_hash_build");
+  CqlKernel* kp = kernel("cql_join_hash_probe");
+  unsigned char* host = (unsigned char*)malloc(bytes);
+  if (!table || !visit_group || !out || !kb || !kp || !host)
+  {
+    free(visit_list);
+    free(host);
+    return 0;
+  }
+  uint64_t group_min_bits;
+  memcpy(&group_min_bits, &vmin, 8);
+  cqlcuda_kernel_set_arg_buffer(kb, 0, vbuf);
+  cqlcuda_kernel_set_arg_buffer(kb, 1, kbuf);
+  cqlcuda_kernel_set_arg_buffer(kb, 2, gbuf);
+  cqlcuda_kernel_set_arg_buffer(kb, 3, table);
+  cqlcuda_kernel_set_arg_buffer_range(kb, 4, out, error_at, 16);
+  cqlcuda_kernel_set_arg_u64(kb, 0, visits);
+  cqlcuda_kernel_set_arg_u64(kb, 1, visit_list ? 1 : 0);
+  cqlcuda_kernel_set_arg_u64(kb, 2, log2_size);
+  cqlcuda_kernel_set_arg_buffer(kb, 5, visit_group);
+  cqlcuda_kernel_set_arg_u64(kb, 3, visit_bits);
+  cqlcuda_kernel_set_arg_u64(kb, 4, group_min_bits);
+  cqlcuda_kernel_set_arg_u64(kb, 5, gv ? 1 : 0);
+  cqlcuda_kernel_set_arg_u64(kb, 6, dev_groups ? dgc->type : CQLOPS_TYPE_F64);
+  cqlcuda_kernel_set_arg_u64(kb, 7, slots);
+  cqlcuda_kernel_set_arg_buffer(kp, 0, fk->buffer);
+  for (uint32_t i = 0; i < 4; i++) cqlcuda_kernel_set_arg_buffer(kp, 1 + i, i < arg_count ? args[i]->buffer : fk->buffer);
+  cqlcuda_kernel_set_arg_buffer(kp, 5, table);
+  cqlcuda_kernel_set_arg_buffer(kp, 6, out);
+  cqlcuda_kernel_set_arg_u64(kp, 0, rows);
+  cqlcuda_kernel_set_arg_u64(kp, 1, E);
+  cqlcuda_kernel_set_arg_u64(kp, 2, funcs);
+  cqlcuda_kernel_set_arg_u64(kp, 3, (uint64_t)arg_index | ((uint64_t)arg_signed << 32));
+  cqlcuda_kernel_set_arg_buffer(kp, 7, visit_group);
+  cqlcuda_kernel_set_arg_u64(kp, 4, (uint64_t)log2_size | ((uint64_t)visit_bits << 32));
+  cqlcuda_kernel_set_arg_u64(kp, 5, slots | ((uint64_t)copies_log2 << 32));
+  CqlBatch* b = cqlcuda_batch_begin(visits * 4 + D * 12, bytes);
+  if (visit_list && !uploaded) cqlcuda_batch_buffer_write(b, vbuf, visit_list, visits * 4);
+  if (!dev_keys) cqlcuda_batch_buffer_write(b, kbuf, q->dim_keys, D * 4);
+  if (gv && !dev_groups && !uploaded) cqlcuda_batch_buffer_write(b, gbuf, gv, D * 8);
+  cqlcuda_batch_buffer_fill(b, table, 8ull << log2_size, 0xffffffffu);
+  cqlcuda_batch_buffer_zero(b, out, mins_at);
+  if (extrema)
+  {
+    cqlcuda_batch_fill_range(b, out, mins_at, slots * E * 4, 0x7fffffffu);
+    cqlcuda_batch_fill_range(b, out, maxs_at, slots * E * 4, 0x80000000u);
+  }
+  cqlcuda_batch_fill_range(b, out, first_at, slots * 4, 0xffffffffu);
+  cqlcuda_batch_fill_range(b, out, error_at, 16, 0);
+  cqlcuda_batch_kernel_execute(b, kb, (uint32_t)visits, QE_GPU_WORKGROUP_SIZE);
+  cqlcuda_batch_kernel_execute(b, kp, (uint32_t)rows, QE_GPU_WORKGROUP_SIZE);
+  cqlcuda_batch_buffer_read(b, out, host, bytes);
+  ok = cqlcuda_batch_end(b);
+  free(visit_list);
+  uint32_t error = 0;
+  memcpy(&error, host + error_at, 4);
+  int result = !ok ? 0 : error ? -1
+                  : join_slots_finish(q, core_count, core_of_expr, slots, host, sums_at, mins_at, maxs_at, first_at, max_groups, out_groups,
+                                      out_group_dim_row, out_results);
+  free(host);
+  return result;
+}
+
 /* -1 when the query does not take this path (the host pass then runs), else 0 / 1 */
 static int join_device_pass(const CqlJoinAgg* q, uint32_t core_count, const uint32_t* core_funcs, const CqlColumn* const* core_cols,
                             const uint32_t* core_of_expr, uint64_t max_groups, uint64_t* out_groups, uint64_t* out_group_dim_row,
@@ -1055,49 +1315,9 @@ static int join_device_pass(const CqlJoinAgg* q, uint32_t core_count, const uint
   if (t.batch) cqlcuda_batch_end(t.batch);   /* a refusal above: the dense pass's batch still ends */
   if (ok)
   {
-    const uint64_t* counts = (const uint64_t*)(host + counts_at);
-    const int64_t* sums = (const int64_t*)(host + sums_at);
-    const int32_t* mins = (const int32_t*)(host + mins_at);
-    const int32_t* maxs = (const int32_t*)(host + maxs_at);
-    const uint32_t* first = (const uint32_t*)(host + first_at);
-    SlotFirst* order = (SlotFirst*)malloc(slots * sizeof(SlotFirst));
-    uint64_t groups = 0;
-    ok = order != NULL;
-    for (uint64_t s2 = 0; ok && s2 < slots; s2++)
-      if (first[s2] != 0xffffffffu)
-      {
-        order[groups].first = first[s2];
-        order[groups].slot = (uint32_t)s2;
-        groups++;
-      }
-    if (ok && groups > max_groups) ok = refuse("more groups than the output arrays hold");
-    if (ok)
-    {
-      /* groups in the order of their first kept dim row, as the host pass meets them */
-      qsort(order, groups, sizeof(SlotFirst), slot_by_first);
-      for (uint64_t g = 0; g < groups; g++)
-      {
-        uint64_t s2 = order[g].slot;
-        out_group_dim_row[g] = q->dim_rows ? q->dim_rows[order[g].first] : order[g].first;
-        for (uint32_t e = 0; e < q->expr_count; e++)
-        {
-          uint64_t c = s2 * E + core_of_expr[e];
-          double r;
-          switch (q->funcs[e])
-          {
-            case CQLOPS_FUNC_COUNT: r = (double)counts[s2]; break;
-            case CQLOPS_FUNC_SUM: r = (double)sums[c]; break;
-            case CQLOPS_FUNC_AVG: r = counts[s2] ? (double)sums[c] / (double)counts[s2] : 0.0; break;
-            case CQLOPS_FUNC_MIN: r = (double)mins[c]; break;
-            default: r = (double)maxs[c]; break;
-          }
-          out_results[g * q->expr_count + e] = r;
-        }
-      }
-      *out_groups = groups;
-      if (out_strategy) *out_strategy = 1u;
-    }
-    free(order);
+    ok = join_slots_finish(q, core_count, core_of_expr, slots, host, sums_at, mins_at, maxs_at, first_at, max_groups, out_groups, out_group_dim_row,
+                           out_results);
+    if (ok && out_strategy) *out_strategy = 1u;
   }
   free(host);
   free(vl);
@@ -1179,6 +1399,17 @@ int cqlops_join_aggregate(const CqlJoinAgg* q, uint64_t max_groups, uint64_t* ou
     int r = join_device_pass(q, core_count, core_funcs, core_cols, core_of_expr, max_groups, out_groups, out_group_dim_row, out_results,
                              out_strategy);
     if (r >= 0) return r;
+  }
+  /* fact keys over a wide range: totals per group through a hash table of the dim keys */
+  if (q->strategy == 0 && !(fk->has_range && groups_cap <= 65536))
+  {
+    int r = hash_join_aggregate(q, core_count, core_funcs, core_cols, core_of_expr, max_groups, out_groups, out_group_dim_row, out_results);
+    if (r >= 0)
+    {
+      if (r == 1 && out_strategy) *out_strategy = 2u;
+      return r;
+    }
+    cqlops_note_error("");
   }
   JoinTotals totals;
   if (!join_totals(q, core_count, core_funcs, core_cols, &totals)) return 0;
