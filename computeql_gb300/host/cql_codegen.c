@@ -534,8 +534,12 @@ static void emit_fused_accumulate(Str* out, const CqlFusedAgg* f)
         break;
       default:
       {
+        /* only the addition is FP64 work, whose rate on GB300 is a small fraction of the integer rate: the extremes are
+           kept as integers of the doubles' order, NaN left out */
         char* d = dbl_of(s, (int)f->coltypes[c]);
-        sprintf_(out, "          { double x = %s; ds%u += x; dn%u = fmin(dn%u, x); dx%u = fmax(dx%u, x); }\n", d, c, c, c, c, c);
+        sprintf_(out, "          { double x = %s; ds%u += x; long long o = __double_as_longlong(x); bool num = (o & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll;\n"
+                      "            o ^= (o >> 63) & 0x7fffffffffffffffll; dn%u = num && o < dn%u ? o : dn%u; dx%u = num && o > dx%u ? o : dx%u; }\n",
+                 d, c, c, c, c, c, c, c);
         free(d);
       }
     }
@@ -634,7 +638,7 @@ int cqlops_program_source(const CqlProgram* prog, uint32_t kind, const CqlFusedA
         case CQLOPS_TYPE_U32: sprintf_(&s, "  u64 us%u = 0ull; u32 un%u = 0xffffffffu, ux%u = 0u;\n", c, c, c); break;
         case CQLOPS_TYPE_I32: sprintf_(&s, "  long long is%u = 0ll; int in%u = 0x7fffffff, ix%u = (int)0x80000000;\n", c, c, c); break;
         case CQLOPS_TYPE_F32: sprintf_(&s, "  double ds%u = 0.0; float fn%u = __int_as_float(0x7f7fffff), fx%u = -__int_as_float(0x7f7fffff);\n", c, c, c); break;
-        default: sprintf_(&s, "  double ds%u = 0.0, dn%u = 1.7976931348623157e308, dx%u = -1.7976931348623157e308;\n", c, c, c);
+        default: sprintf_(&s, "  double ds%u = 0.0; long long dn%u = 0x7fefffffffffffffll, dx%u = (long long)0x8010000000000000ull;   // +-DBL_MAX\n", c, c, c);
       }
     }
     sputs(&s,
@@ -648,7 +652,7 @@ int cqlops_program_source(const CqlProgram* prog, uint32_t kind, const CqlFusedA
     sputs(&s, "        }\n      }\n    }\n  }\n");
     /* block reduction and the partials */
     sputs(&s,
-          "  __shared__ double sh_d[8]; __shared__ unsigned long long sh_u[8]; __shared__ u32 sh_w[8]; __shared__ float sh_f[8];\n"
+          "  __shared__ double sh_d[8]; __shared__ unsigned long long sh_u[8], sh_v[8]; __shared__ u32 sh_w[8]; __shared__ float sh_f[8];\n"
           "  double* partials = (double*)a.buf[3]; const u64 pcap = a.bytes[3] / 8ull; const u32 wgs = cql_word(a, 12);\n");
     sprintf_(&s, "  const u32 width = %uu;\n", 1 + 3 * kc);
     sputs(&s,
@@ -694,18 +698,14 @@ int cqlops_program_source(const CqlProgram* prog, uint32_t kind, const CqlFusedA
                "    double X = (double)sh_f[0]; __syncthreads();\n"
                "    if (threadIdx.x == 0u && at + %u + 2 < pcap) { partials[at + %u] = S; partials[at + %u + 1] = block_count ? N : 1.7976931348623157e308; partials[at + %u + 2] = block_count ? X : -1.7976931348623157e308; } }\n";
       else
-        fold = "  { double s_ = ds%u, n_ = dn%u, x_ = dx%u;\n"
-               "    for (int o = 16; o > 0; o >>= 1) { s_ += __shfl_xor_sync(0xffffffffu, s_, o); n_ = fmin(n_, __shfl_xor_sync(0xffffffffu, n_, o)); x_ = fmax(x_, __shfl_xor_sync(0xffffffffu, x_, o)); }\n"
-               "    if (lane == 0u) sh_d[warp] = s_; __syncthreads();\n"
-               "    if (threadIdx.x == 0u) { for (int w = 1; w < 8; w++) s_ += sh_d[w]; sh_d[0] = s_; } __syncthreads();\n"
-               "    double S = sh_d[0]; __syncthreads();\n"
-               "    if (lane == 0u) sh_d[warp] = n_; __syncthreads();\n"
-               "    if (threadIdx.x == 0u) { for (int w = 1; w < 8; w++) n_ = fmin(n_, sh_d[w]); sh_d[0] = n_; } __syncthreads();\n"
-               "    double N = sh_d[0]; __syncthreads();\n"
-               "    if (lane == 0u) sh_d[warp] = x_; __syncthreads();\n"
-               "    if (threadIdx.x == 0u) { for (int w = 1; w < 8; w++) x_ = fmax(x_, sh_d[w]); sh_d[0] = x_; } __syncthreads();\n"
-               "    double X = sh_d[0]; __syncthreads();\n"
-               "    if (threadIdx.x == 0u && at + %u + 2 < pcap) { partials[at + %u] = S; partials[at + %u + 1] = N; partials[at + %u + 2] = X; } }\n";
+        fold = "  { double s_ = ds%u; long long n_ = dn%u, x_ = dx%u;\n"
+               "    for (int o = 16; o > 0; o >>= 1) { s_ += __shfl_xor_sync(0xffffffffu, s_, o); n_ = min(n_, __shfl_xor_sync(0xffffffffu, n_, o)); x_ = max(x_, __shfl_xor_sync(0xffffffffu, x_, o)); }\n"
+               "    if (lane == 0u) { sh_d[warp] = s_; sh_u[warp] = (unsigned long long)n_; sh_v[warp] = (unsigned long long)x_; } __syncthreads();\n"
+               "    if (threadIdx.x == 0u) {\n"
+               "      for (int w = 1; w < 8; w++) { s_ += sh_d[w]; n_ = min(n_, (long long)sh_u[w]); x_ = max(x_, (long long)sh_v[w]); }\n"
+               "      n_ ^= (n_ >> 63) & 0x7fffffffffffffffll; x_ ^= (x_ >> 63) & 0x7fffffffffffffffll;\n"
+               "      if (at + %u + 2 < pcap) { partials[at + %u] = s_; partials[at + %u + 1] = __longlong_as_double(n_); partials[at + %u + 2] = __longlong_as_double(x_); } }\n"
+               "    __syncthreads(); }\n";
       sprintf_(&s, fold, c, c, c, 1 + 3 * c, 1 + 3 * c, 1 + 3 * c, 1 + 3 * c);
     }
     /* workgroups of the reference's grid this launch did not cover: neutral partials */

@@ -14,6 +14,7 @@
 #include "cqlops.h"
 #include "cql_ops_internal.h"
 
+#include <math.h>
 #include <pthread.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -23,6 +24,8 @@
 #define QE_SCAN_MAX_STACK 8
 #define FAILED_CAP 64
 #define FUSE_GROUP_SHARED_WORDS 4096
+#define FUSE_ROWS_PER_GROUP 2048
+#define FUSE_GROUPS_PER_SM 6   /* the generated kernels' launch bound */
 
 const char* cqlops_last_error(void);
 uint32_t cqlops_program_simple_leaves(const CqlProgram* prog, CqlLeaf* out, uint32_t cap);
@@ -166,8 +169,8 @@ static uint64_t program_rows(const CqlProgram* prog, const CqlColumn* columns, u
   return prog->binding_count ? columns[prog->binding_column[0]].rows : columns[0].rows;
 }
 
-/* bytecode, constants and string pool of a program into pooled buffers, written in one batch */
-static int upload_program(const CqlProgram* prog, CqlBuffer** out_code, CqlBuffer** out_consts, CqlBuffer** out_strs)
+/* pooled buffers for a program's bytecode, constants and string pool */
+static int program_buffers(const CqlProgram* prog, CqlBuffer** out_code, CqlBuffer** out_consts, CqlBuffer** out_strs)
 {
   uint64_t code_bytes = (uint64_t)prog->word_count * 4;
   uint64_t const_bytes = (uint64_t)(prog->const_count ? prog->const_count : 1) * 8;
@@ -175,18 +178,23 @@ static int upload_program(const CqlProgram* prog, CqlBuffer** out_code, CqlBuffe
   *out_code = pooled("cqlops_scan_bytecode", code_bytes ? code_bytes : 4, CQLCUDA_BUFFER_WRITE);
   *out_consts = pooled("cqlops_scan_num_consts", const_bytes, CQLCUDA_BUFFER_WRITE);
   *out_strs = pooled("cqlops_scan_str_consts", str_bytes, CQLCUDA_BUFFER_WRITE);
-  if (!*out_code || !*out_consts || !*out_strs) return 0;
-  CqlBatch* batch = cqlcuda_batch_begin(code_bytes + const_bytes + str_bytes, 0);
-  if (code_bytes) cqlcuda_batch_buffer_write(batch, *out_code, prog->words, code_bytes);
-  if (prog->const_count) cqlcuda_batch_buffer_write(batch, *out_consts, prog->consts, (uint64_t)prog->const_count * 8);
+  return *out_code && *out_consts && *out_strs;
+}
+
+/* The program written into its buffers, in the batch of the kernel that reads it: a batch of its own cost a wait for the
+   device (13 us of a 1M-row query's 138) before the kernel was even launched. The generated kernels read no bytecode. */
+static void upload_program(CqlBatch* batch, const CqlProgram* prog, int bytecode, CqlBuffer* code, CqlBuffer* consts, CqlBuffer* strs)
+{
+  if (bytecode && prog->word_count) cqlcuda_batch_buffer_write(batch, code, prog->words, (uint64_t)prog->word_count * 4);
+  if (prog->const_count) cqlcuda_batch_buffer_write(batch, consts, prog->consts, (uint64_t)prog->const_count * 8);
   if (prog->str_pool_size)
   {
     uint8_t pad[CQLOPS_MAX_STR_POOL + 4];
-    memset(pad, 0, str_bytes);
+    uint64_t str_bytes = (prog->str_pool_size + 3u) & ~3u;
+    memset(pad + prog->str_pool_size, 0, str_bytes - prog->str_pool_size);
     memcpy(pad, prog->str_pool, prog->str_pool_size);
-    cqlcuda_batch_buffer_write(batch, *out_strs, pad, str_bytes);
+    cqlcuda_batch_buffer_write(batch, strs, pad, str_bytes);
   }
-  return cqlcuda_batch_end(batch);
 }
 
 /* scan_simple over the program's leaves, columns remapped to the leaf columns */
@@ -264,7 +272,7 @@ static int scan_filter_run(const CqlProgram* prog, const CqlColumn* columns, uin
     if (!k) return 0;
   }
   CqlBuffer *code, *consts, *strs;
-  if (!upload_program(prog, &code, &consts, &strs)) return 0;
+  if (!program_buffers(prog, &code, &consts, &strs)) return 0;
   CqlBuffer* counter = pooled("scan_filter_result_counter", 8, CQLCUDA_BUFFER_READ_WRITE);
   CqlBuffer* filler = pooled("cqlops_filler", 16, CQLCUDA_BUFFER_WRITE);
   if (!counter || !filler) return 0;
@@ -293,6 +301,7 @@ static int scan_filter_run(const CqlProgram* prog, const CqlColumn* columns, uin
     cqlcuda_kernel_set_arg_buffer(k, 3, bits);
     uint32_t c32[2] = { 0, 0 };
     CqlBatch* batch = cqlcuda_batch_begin(0, 8);
+    upload_program(batch, prog, ran == CQLOPS_SCAN_INTERPRETER, code, consts, strs);
     cqlcuda_batch_buffer_zero(batch, counter, 8);
     cqlcuda_batch_kernel_execute(batch, k, (uint32_t)(rows < 0xffffffffull ? rows : 0xffffffffull), QE_GPU_WORKGROUP_SIZE);
     cqlcuda_batch_buffer_read(batch, counter, c32, 8);
@@ -318,6 +327,7 @@ static int scan_filter_run(const CqlProgram* prog, const CqlColumn* columns, uin
     cqlcuda_kernel_set_arg_buffer(k, 3, output);
     uint32_t c32[2] = { 0, 0 };
     CqlBatch* batch = cqlcuda_batch_begin(0, 8);
+    if (attempt == 0) upload_program(batch, prog, ran == CQLOPS_SCAN_INTERPRETER, code, consts, strs);
     cqlcuda_batch_buffer_zero(batch, counter, 8);
     cqlcuda_batch_kernel_execute(batch, k, (uint32_t)(rows < 0xffffffffull ? rows : 0xffffffffull), QE_GPU_WORKGROUP_SIZE);
     cqlcuda_batch_buffer_read(batch, counter, c32, 8);
@@ -412,11 +422,14 @@ int cqlops_fused_filter_aggregate(const CqlProgram* prog_in, const CqlColumn* co
   }
   CqlKernel* k = ok ? generated_kernel(prog, CQLOPS_KERNEL_FUSED_AGG, &fuse) : NULL;
   CqlBuffer *code = NULL, *consts = NULL, *strs = NULL;
-  if (k) ok = upload_program(prog, &code, &consts, &strs);
+  if (k) ok = program_buffers(prog, &code, &consts, &strs);
   else ok = 0;
   uint64_t rows = ok ? program_rows(prog, columns, 0) : 0;
-  uint64_t groups = rows / 65536;
-  if (groups > 2048) groups = 2048;
+  /* A workgroup for each 2048 rows (8 a thread), up to what is resident: the reference's 65536 rows a workgroup gave a
+     1M-row table 15 of them, on 15 of 152 SMs (75 us of kernel, 488 workgroups 23), and tables past 2^26 rows the same grid. */
+  uint64_t groups = (rows + FUSE_ROWS_PER_GROUP - 1) / FUSE_ROWS_PER_GROUP;
+  uint64_t resident = (uint64_t)cqlcuda_sm_count() * FUSE_GROUPS_PER_SM;
+  if (groups > resident) groups = resident;
   if (groups < 1) groups = 1;
   uint64_t width = 1 + 3 * (uint64_t)agg_count;
   CqlBuffer* partials_buf = ok ? pooled("fused_agg_partials", groups * width * 8, CQLCUDA_BUFFER_READ_WRITE) : NULL;
@@ -439,15 +452,17 @@ int cqlops_fused_filter_aggregate(const CqlProgram* prog_in, const CqlColumn* co
     cqlcuda_kernel_set_arg_u64(k, 4, 0);
     cqlcuda_kernel_set_arg_u64(k, 6, groups);
     CqlBatch* batch = cqlcuda_batch_begin(0, groups * width * 8);
+    upload_program(batch, prog, 0, code, consts, strs);
     cqlcuda_batch_kernel_execute(batch, k, (uint32_t)(groups * QE_GPU_WORKGROUP_SIZE), QE_GPU_WORKGROUP_SIZE);
     cqlcuda_batch_buffer_read(batch, partials_buf, partials, groups * width * 8);
     ok = cqlcuda_batch_end(batch);
   }
   if (ok)
   {
-    /* combined in workgroup order (:10200-10219) */
+    /* combined in workgroup order (:10200-10219), what each addition rounds away kept beside the sum: the fold of many
+       workgroups is as exact as that of few */
     double matched = 0.0;
-    double sum[4] = { 0, 0, 0, 0 }, mn[4], mx[4];
+    double sum[4] = { 0, 0, 0, 0 }, rest[4] = { 0, 0, 0, 0 }, mn[4], mx[4];
     for (uint32_t c = 0; c < 4; c++)
     {
       mn[c] = 1.7976931348623157e308;
@@ -459,7 +474,9 @@ int cqlops_fused_filter_aggregate(const CqlProgram* prog_in, const CqlColumn* co
       matched += row[0];
       for (uint32_t c = 0; c < agg_count; c++)
       {
-        sum[c] += row[1 + 3 * c];
+        double x = row[1 + 3 * c], t = sum[c] + x;
+        rest[c] += fabs(sum[c]) >= fabs(x) ? (sum[c] - t) + x : (x - t) + sum[c];
+        sum[c] = t;
         mn[c] = row[2 + 3 * c] < mn[c] ? row[2 + 3 * c] : mn[c];
         mx[c] = row[3 + 3 * c] > mx[c] ? row[3 + 3 * c] : mx[c];
       }
@@ -467,7 +484,7 @@ int cqlops_fused_filter_aggregate(const CqlProgram* prog_in, const CqlColumn* co
     if (out_count) *out_count = matched;
     for (uint32_t c = 0; c < agg_count; c++)
     {
-      if (out_sum) out_sum[c] = sum[c];
+      if (out_sum) out_sum[c] = isfinite(sum[c]) ? sum[c] + rest[c] : sum[c];
       if (out_min) out_min[c] = mn[c];
       if (out_max) out_max[c] = mx[c];
     }
@@ -560,7 +577,7 @@ int cqlops_fused_filter_group(const CqlProgram* prog_in, const CqlColumn* column
   fuse.group_count = (uint32_t)total;
   CqlKernel* kern = ok ? generated_kernel(prog, CQLOPS_KERNEL_FUSED_GROUP, &fuse) : NULL;
   CqlBuffer *code = NULL, *consts = NULL, *strs = NULL;
-  ok = kern && upload_program(prog, &code, &consts, &strs);
+  ok = kern && program_buffers(prog, &code, &consts, &strs);
   uint64_t rows = ok ? program_rows(prog, columns, 0) : 0;
   uint64_t words = total * width;
   CqlBuffer* out_buf = ok ? pooled("fused_group_output", words * 4, CQLCUDA_BUFFER_READ_WRITE) : NULL;
@@ -577,8 +594,12 @@ int cqlops_fused_filter_group(const CqlProgram* prog_in, const CqlColumn* column
       init[g * width + 1] = 0xffffffffu;
       for (uint32_t c = 0; c < agg_count; c++) init[g * width + 4 + 4 * c] = 0xffffffffu;
     }
-    uint64_t wgs = rows / 131072;
-    if (wgs > 1024) wgs = 1024;
+    /* a workgroup for each 8192 to 131072 rows, by what its table costs to merge (a row read against a 64th of a
+       table word), up to what is resident */
+    uint64_t per = words / 64 < 4 ? 4 : words / 64 > 64 ? 64 : words / 64;
+    uint64_t wgs = (rows + per * FUSE_ROWS_PER_GROUP - 1) / (per * FUSE_ROWS_PER_GROUP);
+    uint64_t resident = (uint64_t)cqlcuda_sm_count() * FUSE_GROUPS_PER_SM;
+    if (wgs > resident) wgs = resident;
     if (wgs < 1) wgs = 1;
     cqlcuda_kernel_set_arg_buffer(kern, 0, filler);
     cqlcuda_kernel_set_arg_buffer(kern, 1, consts);
@@ -594,6 +615,7 @@ int cqlops_fused_filter_group(const CqlProgram* prog_in, const CqlColumn* column
     cqlcuda_kernel_set_arg_u64(kern, 6, wgs | ((uint64_t)(uint32_t)key_min[2] << 32));
     cqlcuda_kernel_set_arg_u64(kern, 7, (uint64_t)(uint32_t)key_min[0] | ((uint64_t)(uint32_t)key_min[1] << 32));
     CqlBatch* batch = cqlcuda_batch_begin(words * 4, words * 4);
+    upload_program(batch, prog, 0, code, consts, strs);
     cqlcuda_batch_buffer_write(batch, out_buf, init, words * 4);
     cqlcuda_batch_kernel_execute(batch, kern, (uint32_t)(wgs * QE_GPU_WORKGROUP_SIZE), QE_GPU_WORKGROUP_SIZE);
     cqlcuda_batch_buffer_read(batch, out_buf, result, words * 4);
