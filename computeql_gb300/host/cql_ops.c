@@ -323,47 +323,28 @@ static int simple_leaf_words(uint32_t* words, uint32_t slot, const CqlColumn* co
    size / 4 of them; the emit kernel stops there). */
 int cqlops_bitmap_rows_enqueue(CqlBatch* b, CqlBuffer* bitmap, uint64_t first_row, uint64_t rows, CqlBuffer* list)
 {
-  uint64_t words = (rows + 31) / 32, blocks = (words + 255) / 256, scan_blocks = (blocks + 255) / 256;
+  uint64_t words = (rows + 31) / 32;
   if (words == 0) return 1;
-  CqlBuffer* counts = pooled("bitmap_block_counts", blocks * 4, CQLCUDA_BUFFER_READ_WRITE);
-  CqlBuffer* offsets = pooled("bitmap_block_offsets", (blocks + 1) * 4, CQLCUDA_BUFFER_READ_WRITE);
-  CqlBuffer* cursor = pooled("bitmap_block_cursor", blocks * 4, CQLCUDA_BUFFER_READ_WRITE);
-  CqlBuffer* block_sums = pooled("bitmap_scan_sums", scan_blocks * 4, CQLCUDA_BUFFER_READ_WRITE);
+  CqlBuffer* counts = pooled("bitmap_run_counts", (uint64_t)cqlcuda_sm_count() * 64, CQLCUDA_BUFFER_READ_WRITE);
   CqlKernel* popc = kernel_named("cql_bitmap_popc");
-  CqlKernel* scan = kernel_named("prefix_sum");
   CqlKernel* emit = kernel_named("cql_bitmap_emit");
-  if (!counts || !offsets || !cursor || !block_sums || !popc || !scan || !emit) return 0;
+  if (!counts || !popc || !emit) return 0;
   cqlcuda_kernel_set_arg_buffer(popc, 0, bitmap);
   cqlcuda_kernel_set_arg_buffer(popc, 1, counts);
   cqlcuda_kernel_set_arg_u64(popc, 0, words);
-  cqlcuda_kernel_set_arg_buffer(scan, 0, counts);
-  cqlcuda_kernel_set_arg_buffer(scan, 1, offsets);
-  cqlcuda_kernel_set_arg_buffer(scan, 2, cursor);
-  cqlcuda_kernel_set_arg_buffer(scan, 3, block_sums);
-  cqlcuda_kernel_set_arg_u64(scan, 0, blocks);
   cqlcuda_kernel_set_arg_buffer(emit, 0, bitmap);
-  cqlcuda_kernel_set_arg_buffer(emit, 1, offsets);
+  cqlcuda_kernel_set_arg_buffer(emit, 1, counts);
   cqlcuda_kernel_set_arg_buffer(emit, 2, list);
   cqlcuda_kernel_set_arg_u64(emit, 0, words);
   cqlcuda_kernel_set_arg_u64(emit, 1, first_row);
-  if (blocks == 1) cqlcuda_batch_buffer_zero(b, offsets, 4);   /* one block: its rows start at 0 */
-  else
-  {
-    cqlcuda_batch_kernel_execute(b, popc, (uint32_t)(blocks * 256), QE_GPU_WORKGROUP_SIZE);
-    for (uint32_t mode = 0; mode < 3; mode++)
-    {
-      cqlcuda_kernel_set_arg_u64(scan, 1, mode);
-      cqlcuda_batch_kernel_execute(b, scan, mode == 1 ? 256u : (uint32_t)(scan_blocks * 256), 256);
-    }
-  }
-  cqlcuda_batch_kernel_execute(b, emit, (uint32_t)(blocks * 256), QE_GPU_WORKGROUP_SIZE);
+  cqlcuda_batch_kernel_execute(b, popc, (uint32_t)(words < 0xffffffffull ? words : 0xffffffffull), QE_GPU_WORKGROUP_SIZE);
+  cqlcuda_batch_kernel_execute(b, emit, (uint32_t)(words < 0xffffffffull ? words : 0xffffffffull), QE_GPU_WORKGROUP_SIZE);
   return 1;
 }
 
-/* The rows of a selection bitmap (one bit a row, as the scans write it in bitmap mode; its first bit is
-   table row first_row, a multiple of 32) in ascending order, on the device: each 256-word block's
-   population, an exclusive scan over the blocks, then every block's rows written from its offset. The
-   first min(count, cap) rows land in out_rows; count is the bitmap's population. */
+/* The rows of a selection bitmap (one bit a row, as the scans write it in bitmap mode; its first bit is table row
+   first_row, a multiple of 32) in ascending order, on the device. The first min(count, cap) rows land in out_rows;
+   count is the bitmap's population. */
 int cqlops_bitmap_rows(CqlBuffer* bitmap, uint64_t first_row, uint64_t rows, uint64_t count, uint32_t* out_rows, uint64_t cap)
 {
   if (!count || !cap || !out_rows) return 1;
