@@ -631,6 +631,576 @@ static int launch_radix_scatter(const CqlLaunch& a, uint32_t gws, uint32_t lws, 
   return 0;
 }
 
+// ---------------------------------------------------------------------------------------------
+// ORDER BY of more than 32 key bits by a 32-bit prefix (not in the reference, nor the sort above): most of a wide
+// key's bits only break ties, and few rows tie in the bits that matter. Each key's smallest and largest order word are
+// found first; the highest 32 bits of the keys' distances from their ends, in the keys' order, make a prefix; the rows
+// are sorted by it in four passes, and the short runs of rows that share a prefix are put in order in shared memory,
+// by the full keys.
+//
+//  cql_sort_range   binding 0..3 the key columns, 4 selection, 5 out: per key (smallest, largest) order word, u64 each
+//                   (all ones and 0 before); words as below
+//  cql_sort_sample  the same, 6 out: how many rows of the sample share another's prefix and differ in the rest (u32)
+//  cql_sort_prefix  the same with binding 5 the prefixes out (u32), 6 the histogram [256][tiles] of their low byte, 7 its
+//                   totals [256] (zero before), 8 the ranges as found
+//  cql_sort_runs    the same with binding 5 the sorted prefixes, 6 their positions, 7 rows out, 8 the ranges, 9 status
+//                   (bit 0: a run longer than the kernel takes is out of order)
+//  words: 0 n, 2 keys, 3 1 = the positions are the selection's rows, 4 CQL types (4 bits a key), 5 descending (bits), 6
+//  narrow widths (2 bits a key), slots 4 and 5 the narrow bases (32 bits a key)
+//
+// 64-bit integers order as themselves while they lie within 2^53 of zero, where the F64 values they are compared as are
+// all different; a column with others orders by those values. Distances, and not the words' own bits: doubles from 0.1
+// to 4000 differ from bit 62 down, but span 2^56, so the prefix holds 28 bits of their fractions and not 21 (20M
+// lognormal rows: most rows in runs, 407 us for the runs, against 125).
+//
+// 20M rows by (f64 DESC, u32): twelve passes over 12- and 8-byte pairs took 2.43 ms of kernels, this form 0.89: ranges 61 us, sample 17, prefixes 74, the four passes 612, runs 125.
+#define PREFIX_SAMPLE 2048u
+#define RUN_THREADS 256
+#define RUN_TILE 1024
+#define RUN_HALO 64
+#define WORD_SIGN 0x8000000000000000ull
+
+struct SortPlan
+{
+  uint32_t keys, bits;          // bits: of the prefix
+  uint32_t hi[4], take[4];      // key k gives the `take` bits below bit hi of its distance
+  uint32_t rest;                // the first key with bits below its part, `keys` when there is none
+  uint32_t desc, whole;         // per key: descending; 64-bit integers ordered as themselves
+  unsigned long long lo[4], top[4];
+};
+
+struct SortCols
+{
+  const void* col[4];
+  uint64_t rows[4];
+  const uint32_t* sel;
+  uint32_t keys, types, desc, widths;
+  uint64_t bases[2];
+};
+
+__device__ __forceinline__ bool sort_wide(uint32_t type) { return type == 2 || type == 4 || type == 8 || type == 10 || type == 11; }
+__device__ __forceinline__ bool sort_integer64(uint32_t type) { return sort_wide(type) && type != 4; }
+
+__device__ __forceinline__ SortCols sort_cols(const CqlLaunch& a)
+{
+  SortCols c;
+  c.types = cql_word(a, 4);
+  c.desc = cql_word(a, 5);
+  c.widths = cql_word(a, 6);
+  c.keys = cql_word(a, 2);
+  c.bases[0] = a.push[4];
+  c.bases[1] = a.push[5];
+#pragma unroll
+  for (uint32_t k = 0; k < 4; k++)
+  {
+    uint32_t t = (c.types >> (4 * k)) & 0xfu, w = (c.widths >> (2 * k)) & 3u;
+    c.col[k] = a.buf[k];
+    c.rows[k] = w == 3 ? ~0ull : a.bytes[k] / (w ? w : sort_wide(t) ? 8 : 4);
+  }
+  c.sel = cql_word(a, 3) ? (const uint32_t*)a.buf[4] : nullptr;
+  return c;
+}
+
+// one key of the columns, for a loop over rows
+struct SortKey
+{
+  const void* col;
+  uint64_t rows;
+  uint32_t type, width, base;
+  bool wide, whole;
+};
+
+__device__ __forceinline__ SortKey sort_key(const SortCols& c, uint32_t k, bool whole)
+{
+  SortKey s;
+  s.col = k == 0 ? c.col[0] : k == 1 ? c.col[1] : k == 2 ? c.col[2] : c.col[3];
+  s.rows = k == 0 ? c.rows[0] : k == 1 ? c.rows[1] : k == 2 ? c.rows[2] : c.rows[3];
+  s.type = (c.types >> (4 * k)) & 0xfu;
+  s.width = (c.widths >> (2 * k)) & 3u;
+  s.base = (uint32_t)((k < 2 ? c.bases[0] : c.bases[1]) >> (32 * (k & 1u)));
+  s.wide = sort_wide(s.type);
+  s.whole = whole && sort_integer64(s.type);
+  return s;
+}
+
+__device__ __forceinline__ unsigned long long sort_raw(const SortKey& s, uint32_t row)
+{
+  if (row >= s.rows) return 0;
+  if (s.wide) return ((const unsigned long long*)s.col)[row];
+  if (s.width == 0) return ((const uint32_t*)s.col)[row];
+  return s.width == 1 ? ((const uint8_t*)s.col)[row] : s.width == 2 ? ((const uint16_t*)s.col)[row] : row;
+}
+
+// the ascending order word; a row past the column orders first (the key pass's rule)
+__device__ __forceinline__ unsigned long long sort_word(const SortKey& s, uint32_t row, unsigned long long raw)
+{
+  if (row >= s.rows) return 0;
+  if (s.whole) return s.type == 2 ? raw : raw ^ WORD_SIGN;
+  if (s.wide) return order_bits(s.type, raw);
+  if (s.width == 0) return order_bits(s.type, (uint32_t)raw);
+  return ((uint32_t)raw + s.base) ^ ((s.type == 7 || s.type == 9) ? 0x80000000u : 0u);
+}
+
+// The forms a loop over a key's rows is compiled for: a full-width column that holds every row, by its type. The loops are
+// bound by issue (the general form's tests of type, width and row are 40 instructions a value), so a switch outside them
+// picks the form.
+enum SortForm { FORM_ANY = 0, FORM_U32, FORM_I32, FORM_F32, FORM_F64, FORM_I64, FORM_U64 };
+
+__device__ __forceinline__ int sort_form(const SortKey& s, bool selected, uint64_t n)
+{
+  if (selected || s.width != 0 || s.rows < n) return FORM_ANY;
+  switch (s.type)
+  {
+    case 1: case 12: return FORM_U32;
+    case 7: case 9: return FORM_I32;
+    case 3: return FORM_F32;
+    case 4: return FORM_F64;
+    case 2: return s.whole ? FORM_U64 : FORM_ANY;
+    default: return s.whole ? FORM_I64 : FORM_ANY;
+  }
+}
+
+template <int FORM>
+__device__ __forceinline__ unsigned long long form_raw(const SortKey& s, uint32_t row)
+{
+  if (FORM == FORM_ANY) return sort_raw(s, row);
+  if (FORM <= FORM_F32) return ((const uint32_t*)s.col)[row];
+  return ((const unsigned long long*)s.col)[row];
+}
+
+template <int FORM>
+__device__ __forceinline__ unsigned long long form_word(const SortKey& s, uint32_t row, unsigned long long raw)
+{
+  switch (FORM)
+  {
+    case FORM_U32: return (uint32_t)raw;
+    case FORM_I32: return (uint32_t)raw ^ 0x80000000u;
+    case FORM_F32: return order_bits(3, (uint32_t)raw);
+    case FORM_F64: return f64_order(raw);
+    case FORM_I64: return raw ^ WORD_SIGN;
+    case FORM_U64: return raw;
+    default: return sort_word(s, row, raw);
+  }
+}
+
+__device__ inline SortPlan sort_plan(const unsigned long long* range, const SortCols& c)
+{
+  SortPlan p;
+  p.keys = c.keys;
+  p.desc = c.desc;
+  p.bits = p.whole = 0;
+  p.rest = c.keys;
+  for (uint32_t k = 0; k < 4; k++)
+  {
+    p.hi[k] = p.take[k] = 0;
+    p.lo[k] = p.top[k] = 0;
+    if (k >= c.keys) continue;
+    uint32_t type = (c.types >> (4 * k)) & 0xfu;
+    unsigned long long lo = range[2 * k], top = range[2 * k + 1];
+    if (sort_integer64(type))
+    {
+      const unsigned long long near = 1ull << 53, zero = type == 2 ? 0ull : WORD_SIGN;
+      if (top <= zero + near && (type == 2 || lo >= zero - near)) p.whole |= 1u << k;
+      else
+      {
+        lo = order_bits(type, lo ^ zero);
+        top = order_bits(type, top ^ zero);
+      }
+    }
+    p.lo[k] = lo;
+    p.top[k] = top;
+    unsigned long long span = top - lo;
+    p.hi[k] = span ? 64u - (uint32_t)__clzll((long long)span) : 0u;
+    uint32_t room = 32 - p.bits;
+    p.take[k] = min(p.hi[k], room);
+    p.bits += p.take[k];
+    if (p.take[k] < p.hi[k] && p.rest == c.keys) p.rest = k;
+  }
+  return p;
+}
+
+// the key's distance from its first value in the order
+__device__ __forceinline__ unsigned long long sort_distance(const SortPlan& p, uint32_t k, unsigned long long word)
+{
+  return ((p.desc >> k) & 1u) ? p.top[k] - word : word - p.lo[k];
+}
+
+__device__ __forceinline__ uint32_t prefix_append(const SortPlan& p, uint32_t k, uint32_t v, unsigned long long distance)
+{
+  uint32_t take = p.take[k];
+  return (take == 32 ? 0u : v << take) | (uint32_t)((distance >> (p.hi[k] - take)) & ((1ull << take) - 1ull));
+}
+
+__device__ __forceinline__ unsigned long long sort_distance_of(const SortCols& c, const SortPlan& p, uint32_t k, uint32_t row)
+{
+  SortKey s = sort_key(c, k, (p.whole >> k) & 1u);
+  return sort_distance(p, k, sort_word(s, row, sort_raw(s, row)));
+}
+
+template <int FORM>
+__device__ __forceinline__ void range_of_key(const SortKey& s, const uint32_t* sel, uint64_t n, unsigned long long* out_lo, unsigned long long* out_top)
+{
+  unsigned long long lo = ~0ull, top = 0ull;
+  const uint32_t step = gridDim.x * SORT_THREADS, last = (uint32_t)(n - 1);
+  for (uint64_t i0 = (uint64_t)blockIdx.x * SORT_THREADS + threadIdx.x; i0 < n; i0 += (uint64_t)step * 8)
+  {
+    uint32_t row[8];
+    unsigned long long raw[8];
+#pragma unroll
+    for (uint32_t u = 0; u < 8; u++)
+    {
+      uint32_t i = (uint32_t)min(i0 + (uint64_t)u * step, (uint64_t)last);
+      row[u] = FORM == FORM_ANY && sel ? sel[i] : i;
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 8; u++) raw[u] = form_raw<FORM>(s, row[u]);
+#pragma unroll
+    for (uint32_t u = 0; u < 8; u++)
+    {
+      unsigned long long w = form_word<FORM>(s, row[u], raw[u]);
+      lo = min(lo, w);
+      top = max(top, w);
+    }
+  }
+  *out_lo = lo;
+  *out_top = top;
+}
+
+__global__ void __launch_bounds__(SORT_THREADS, 5) k_sort_range(CqlLaunch a, uint64_t n)
+{
+  const SortCols c = sort_cols(a);
+  unsigned long long* out = (unsigned long long*)a.buf[5];
+#pragma unroll 1
+  for (uint32_t k = 0; k < c.keys; k++)
+  {
+    const SortKey s = sort_key(c, k, true);
+    unsigned long long lo, top;
+    switch (sort_form(s, c.sel != nullptr, n))
+    {
+      case FORM_U32: range_of_key<FORM_U32>(s, c.sel, n, &lo, &top); break;
+      case FORM_I32: range_of_key<FORM_I32>(s, c.sel, n, &lo, &top); break;
+      case FORM_F32: range_of_key<FORM_F32>(s, c.sel, n, &lo, &top); break;
+      case FORM_F64: range_of_key<FORM_F64>(s, c.sel, n, &lo, &top); break;
+      case FORM_I64: range_of_key<FORM_I64>(s, c.sel, n, &lo, &top); break;
+      case FORM_U64: range_of_key<FORM_U64>(s, c.sel, n, &lo, &top); break;
+      default: range_of_key<FORM_ANY>(s, c.sel, n, &lo, &top); break;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+    {
+      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    if ((threadIdx.x & 31u) == 0)
+    {
+      if (lo < __ldcg(&out[2 * k])) atomicMin(&out[2 * k], lo);
+      if (top > __ldcg(&out[2 * k + 1])) atomicMax(&out[2 * k + 1], top);
+    }
+  }
+}
+
+// One CTA: the prefixes of a spread sample meet in a hash table, with a hash of the bits below them.
+__global__ void __launch_bounds__(1024) k_sort_sample(CqlLaunch a, uint64_t n)
+{
+  __shared__ unsigned long long table[2 * PREFIX_SAMPLE];
+  __shared__ uint32_t s_count;
+  const SortCols c = sort_cols(a);
+  const SortPlan p = sort_plan((const unsigned long long*)a.buf[5], c);
+  if (threadIdx.x == 0) s_count = 0;
+  for (uint32_t i = threadIdx.x; i < 2 * PREFIX_SAMPLE; i += 1024) table[i] = ~0ull;
+  __syncthreads();
+  uint32_t mine = 0;
+  for (uint32_t i = threadIdx.x; i < PREFIX_SAMPLE; i += 1024)
+  {
+    uint64_t at = (uint64_t)i * n / PREFIX_SAMPLE;
+    uint32_t row = c.sel ? c.sel[at] : (uint32_t)at, v = 0;
+    unsigned long long rest = 0;
+    for (uint32_t k = 0; k < p.keys; k++)
+    {
+      unsigned long long d = sort_distance_of(c, p, k, row);
+      if (p.take[k]) v = prefix_append(p, k, v, d);
+      if (k >= p.rest) rest = (rest ^ d) * 0x9E3779B97F4A7C15ull;
+    }
+    unsigned long long e = ((unsigned long long)v << 32) | (rest >> 33);   // never all ones
+    uint32_t slot = (v * 0x9E3779B1u) >> 20;                              // 4096 slots, half of them used at most
+    for (;;)
+    {
+      unsigned long long old = atomicCAS(&table[slot], ~0ull, e);
+      if (old == ~0ull) break;
+      if ((uint32_t)(old >> 32) == v)
+      {
+        mine += old != e;
+        break;
+      }
+      slot = (slot + 1u) & (2 * PREFIX_SAMPLE - 1u);
+    }
+  }
+  if (mine) atomicAdd(&s_count, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) *(uint32_t*)a.buf[6] = s_count;
+}
+
+template <int FORM>
+__device__ __forceinline__ void prefix_of_key(const SortKey& s, const SortPlan& p, uint32_t k, const uint32_t* row, uint32_t* v)
+{
+  unsigned long long raw[8];
+#pragma unroll
+  for (uint32_t j = 0; j < 8; j++) raw[j] = form_raw<FORM>(s, row[j]);
+  const bool desc = (p.desc >> k) & 1u;
+  const unsigned long long from = desc ? p.top[k] : p.lo[k], mask = (1ull << p.take[k]) - 1ull;
+  const uint32_t shift = p.hi[k] - p.take[k], take = p.take[k];
+#pragma unroll
+  for (uint32_t j = 0; j < 8; j++)
+  {
+    unsigned long long w = form_word<FORM>(s, row[j], raw[j]), d = desc ? from - w : w - from;
+    v[j] = (take == 32 ? 0u : v[j] << take) | (uint32_t)((d >> shift) & mask);
+  }
+}
+
+__global__ void __launch_bounds__(SORT_THREADS, 4) k_sort_prefix(CqlLaunch a, uint64_t n, uint32_t tiles)
+{
+  __shared__ uint32_t hist[SORT_WARPS][RADIX];
+  __shared__ SortPlan p;
+  const SortCols c = sort_cols(a);
+  uint32_t* out = (uint32_t*)a.buf[5];
+  uint32_t* hist_out = (uint32_t*)a.buf[6];
+  if (threadIdx.x == 0) p = sort_plan((const unsigned long long*)a.buf[8], c);
+  uint32_t warp = threadIdx.x >> 5, d = threadIdx.x, cta_total = 0;
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+  {
+    for (uint32_t i = threadIdx.x; i < SORT_WARPS * RADIX; i += SORT_THREADS) (&hist[0][0])[i] = 0;
+    __syncthreads();
+    uint64_t first = (uint64_t)tile * SORT_TILE;
+    DigitRun run;
+#pragma unroll 1
+    for (uint32_t j0 = 0; j0 < SORT_ROUNDS; j0 += 8)
+    {
+      uint32_t v[8], row[8];
+#pragma unroll
+      for (uint32_t j = 0; j < 8; j++)
+      {
+        uint64_t i = min(first + (j0 + j) * SORT_THREADS + threadIdx.x, n - 1);
+        row[j] = c.sel ? c.sel[i] : (uint32_t)i;
+        v[j] = 0;
+      }
+#pragma unroll 1
+      for (uint32_t k = 0; k < p.keys; k++)
+      {
+        if (p.take[k] == 0) continue;
+        const SortKey s = sort_key(c, k, (p.whole >> k) & 1u);
+        switch (sort_form(s, c.sel != nullptr, n))
+        {
+          case FORM_U32: prefix_of_key<FORM_U32>(s, p, k, row, v); break;
+          case FORM_I32: prefix_of_key<FORM_I32>(s, p, k, row, v); break;
+          case FORM_F32: prefix_of_key<FORM_F32>(s, p, k, row, v); break;
+          case FORM_F64: prefix_of_key<FORM_F64>(s, p, k, row, v); break;
+          case FORM_I64: prefix_of_key<FORM_I64>(s, p, k, row, v); break;
+          case FORM_U64: prefix_of_key<FORM_U64>(s, p, k, row, v); break;
+          default: prefix_of_key<FORM_ANY>(s, p, k, row, v); break;
+        }
+      }
+#pragma unroll
+      for (uint32_t j = 0; j < 8; j++)
+      {
+        uint64_t i = first + (j0 + j) * SORT_THREADS + threadIdx.x;
+        if (i >= n) continue;
+        out[i] = v[j];
+        run.add(hist[warp], v[j] & 0xffu);
+      }
+    }
+    run.flush(hist[warp]);
+    __syncthreads();
+    uint32_t total = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < SORT_WARPS; w++) total += hist[w][d];
+    hist_out[(uint64_t)d * tiles + tile] = total;
+    cta_total += total;
+    __syncthreads();
+  }
+  if (cta_total) atomicAdd(&((uint32_t*)a.buf[7])[d], cta_total);
+}
+
+// x before y among rows that share a prefix and the first unfinished key's word: by the keys after it
+__device__ __noinline__ int sort_compare_rest(const SortCols* c, const SortPlan* p, uint32_t x, uint32_t y)
+{
+  for (uint32_t k = p->rest + 1; k < c->keys; k++)
+  {
+    unsigned long long wx = sort_distance_of(*c, *p, k, x), wy = sort_distance_of(*c, *p, k, y);
+    if (wx != wy) return wx < wy ? -1 : 1;
+  }
+  return 0;
+}
+
+// A row of a run: where it belongs, by counting the rows of the run before it. Runs longer than RUN_HALO are only checked.
+__device__ __noinline__ int run_place(const SortCols* c, const SortPlan* p, const uint32_t* s_prefix, const uint32_t* s_row, const unsigned long long* s_word,
+                                      int j, int lo, int hi, bool* unsorted)
+{
+  uint32_t v = s_prefix[j];
+  bool more = p->rest + 1 < c->keys;
+  int left = j, right = j;
+  while (left > lo && j - left < RUN_HALO && s_prefix[left - 1] == v) left--;
+  while (right + 1 < hi && right - j < RUN_HALO && s_prefix[right + 1] == v) right++;
+  if (right - left + 1 > RUN_HALO)
+  {
+    // too long to rank (every row of the run finds so): fine when it is in order as it is
+    if (j + 1 < hi && s_prefix[j + 1] == v &&
+        (s_word[j] > s_word[j + 1] || (s_word[j] == s_word[j + 1] && more && sort_compare_rest(c, p, s_row[j], s_row[j + 1]) > 0)))
+      *unsorted = true;
+    return j;
+  }
+  unsigned long long w = s_word[j];
+  int at = left;
+  for (int m = left; m <= right; m++)
+  {
+    unsigned long long x = s_word[m];
+    bool before = x < w;
+    if (x == w && m != j)
+    {
+      int r = more ? sort_compare_rest(c, p, s_row[m], s_row[j]) : 0;
+      before = r < 0 || (r == 0 && m < j);
+    }
+    at += before ? 1 : 0;
+  }
+  return at;
+}
+
+__global__ void __launch_bounds__(RUN_THREADS) k_sort_runs(CqlLaunch a, uint64_t n)
+{
+  __shared__ uint32_t s_prefix[RUN_TILE + 2 * RUN_HALO], s_row[RUN_TILE + 2 * RUN_HALO];
+  __shared__ unsigned long long s_word[RUN_TILE + 2 * RUN_HALO];
+  __shared__ SortPlan p;
+  __shared__ SortCols c;
+  const uint32_t* prefix = (const uint32_t*)a.buf[5];
+  const uint32_t* pos = (const uint32_t*)a.buf[6];
+  const uint32_t* sel = cql_word(a, 3) ? (const uint32_t*)a.buf[4] : nullptr;
+  uint32_t* out = (uint32_t*)a.buf[7];
+  if (threadIdx.x == 0)
+  {
+    c = sort_cols(a);
+    p = sort_plan((const unsigned long long*)a.buf[8], c);
+  }
+  bool unsorted = false;
+  const int per = RUN_TILE / RUN_THREADS;
+  for (uint64_t tile = (uint64_t)blockIdx.x * RUN_TILE; tile < n; tile += (uint64_t)gridDim.x * RUN_TILE)
+  {
+    // place j of the shared arrays is position tile - RUN_HALO + j; lo and hi bound those that are there. A thread holds
+    // `per` rows of the tile and, of the first 2 x RUN_HALO threads, one of the halo.
+    int lo = tile < RUN_HALO ? RUN_HALO - (int)tile : 0, hi = (int)min((uint64_t)(RUN_TILE + 2 * RUN_HALO), n - tile + RUN_HALO);
+    int halo = (int)threadIdx.x < RUN_HALO ? (int)threadIdx.x : (int)threadIdx.x < 2 * RUN_HALO ? RUN_TILE + (int)threadIdx.x : -1;
+    if (halo < lo || halo >= hi) halo = -1;
+    uint32_t v[per + 1], row[per + 1];
+#pragma unroll
+    for (int u = 0; u <= per; u++)
+    {
+      int j = u < per ? RUN_HALO + u * RUN_THREADS + (int)threadIdx.x : halo;
+      bool there = j >= 0 && j < hi;
+      v[u] = there ? __ldcs(prefix + (tile + (uint64_t)j - RUN_HALO)) : 0u;
+      row[u] = there ? __ldcs(pos + (tile + (uint64_t)j - RUN_HALO)) : 0u;
+    }
+    if (sel)
+    {
+#pragma unroll
+      for (int u = 0; u <= per; u++)
+        if (u < per ? RUN_HALO + u * RUN_THREADS + (int)threadIdx.x < hi : halo >= 0) row[u] = sel[row[u]];
+    }
+    __syncthreads();   // the tile before is done with the arrays; the first time, the plan is there
+#pragma unroll
+    for (int u = 0; u <= per; u++)
+    {
+      int j = u < per ? RUN_HALO + u * RUN_THREADS + (int)threadIdx.x : halo;
+      if (j < 0 || j >= hi) continue;
+      s_prefix[j] = v[u];
+      s_row[j] = row[u];
+    }
+    __syncthreads();
+    uint32_t in_run = 0;
+#pragma unroll
+    for (int u = 0; u <= per; u++)
+    {
+      int j = u < per ? RUN_HALO + u * RUN_THREADS + (int)threadIdx.x : halo;
+      if (j < 0 || j >= hi) continue;
+      if ((j > lo && s_prefix[j - 1] == v[u]) || (j + 1 < hi && s_prefix[j + 1] == v[u])) in_run |= 1u << u;
+      else if (u < per) out[tile + (uint64_t)j - RUN_HALO] = row[u];
+    }
+    // most tiles have a few rows in runs: their words are read now, all rows' loads in flight together
+    if (!__syncthreads_or((int)in_run)) continue;
+    for (uint32_t left = in_run; left; left &= left - 1u)
+    {
+      int u = __ffs(left) - 1, j = u < per ? RUN_HALO + u * RUN_THREADS + (int)threadIdx.x : halo;
+      s_word[j] = sort_distance_of(c, p, p.rest, s_row[j]);
+    }
+    __syncthreads();
+    for (uint32_t left = in_run & ((1u << per) - 1u); left; left &= left - 1u)
+    {
+      int j = RUN_HALO + (__ffs(left) - 1) * RUN_THREADS + (int)threadIdx.x;
+      int at = run_place(&c, &p, s_prefix, s_row, s_word, j, lo, hi, &unsorted);
+      out[tile + (uint64_t)at - RUN_HALO] = s_row[j];
+    }
+  }
+  if (__syncthreads_or(unsorted) && threadIdx.x == 0) atomicOr((uint32_t*)a.buf[9], 1u);
+}
+
+static int sort_cols_check(const CqlLaunch& a, uint64_t n)
+{
+  uint32_t keys = cql_word(a, 2), types = cql_word(a, 4);
+  if (n == 0 || n > 0xffffffffull || keys == 0 || keys > 4 || (cql_word(a, 3) && a.bytes[4] < n * 4)) return 0;
+  for (uint32_t k = 0; k < keys; k++)
+    if (!sort_key_bytes((types >> (4 * k)) & 0xfu)) return 0;
+  return 1;
+}
+
+static int launch_sort_range(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t n = a.push[0];
+  if (n == 0) return 0;
+  if (!sort_cols_check(a, n) || a.bytes[5] < 64) return (int)cudaErrorInvalidValue;
+  k_sort_range<<<cql_stream_grid((n + SORT_THREADS * 8 - 1) / (SORT_THREADS * 8), 5), SORT_THREADS, 0, stream>>>(a, n);
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
+static int launch_sort_sample(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t n = a.push[0];
+  if (n == 0) return 0;
+  if (!sort_cols_check(a, n) || a.bytes[5] < 64 || a.bytes[6] < 4) return (int)cudaErrorInvalidValue;
+  k_sort_sample<<<1, 1024, 0, stream>>>(a, n);
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
+static int launch_sort_prefix(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t n = a.push[0];
+  if (n == 0) return 0;
+  uint32_t tiles = (uint32_t)((n + SORT_TILE - 1) / SORT_TILE);
+  if (!sort_cols_check(a, n) || a.bytes[5] < n * 4 || a.bytes[6] < (uint64_t)tiles * RADIX * 4 || a.bytes[7] < RADIX * 4 || a.bytes[8] < 64)
+    return (int)cudaErrorInvalidValue;
+  uint32_t grid = cql_stream_grid(tiles, resident_ctas((const void*)k_sort_prefix, 0));
+  k_sort_prefix<<<grid, SORT_THREADS, 0, stream>>>(a, n, tiles);
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
+static int launch_sort_runs(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t n = a.push[0];
+  if (n == 0) return 0;
+  if (!sort_cols_check(a, n) || a.bytes[5] < n * 4 || a.bytes[6] < n * 4 || a.bytes[7] < n * 4 || a.bytes[8] < 64 || a.bytes[9] < 4 || a.buf[6] == a.buf[7])
+    return (int)cudaErrorInvalidValue;
+  k_sort_runs<<<cql_stream_grid((n + RUN_TILE - 1) / RUN_TILE, resident_ctas((const void*)k_sort_runs, 0)), RUN_THREADS, 0, stream>>>(a, n);
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
 __global__ void k_pairs_unpack(CqlLaunch a, uint64_t n, uint32_t stride, uint32_t fa, uint32_t fb)
 {
   const uint32_t* rec = (const uint32_t*)a.buf[0];
@@ -689,5 +1259,9 @@ const CqlKernelDesc cql_kernels_sort[] = {
   { "cql_radix_count", launch_radix_count },
   { "cql_radix_offsets", launch_radix_offsets },
   { "cql_radix_scatter", launch_radix_scatter },
+  { "cql_sort_range", launch_sort_range },
+  { "cql_sort_sample", launch_sort_sample },
+  { "cql_sort_prefix", launch_sort_prefix },
+  { "cql_sort_runs", launch_sort_runs },
   { nullptr, nullptr },
 };
