@@ -10,7 +10,7 @@
 // build row lands in the same bucket. GB300 design: persistent grid-stride launches; the fused probe keeps
 // eight keys and their Bloom words in flight per thread and bounds every open-addressing walk by the
 // table size (the reference's walk assumes an empty slot exists).
-#include "cql_internal.cuh"
+#include "cql_bits.cuh"
 #include <algorithm>
 
 #define JOIN_THREADS 256
@@ -1277,6 +1277,283 @@ static int launch_join_group_range(const CqlLaunch& a, uint32_t gws, uint32_t lw
   return 0;
 }
 
+// ---------------------------------------------------------------------------------------------
+// The equi-join of a build side whose keys do not repeat (not a reference kernel: the reference's buckets, above, take
+// any build side, and their pairs come out in the order the warps meet them). Every probe row has at most one
+// match, so the pairs can be written in the order of the probe rows without a sort: the probe leaves each row's
+// match and each CTA's number of them, the emit ranks the rows of its CTA's run behind the runs before.
+//
+//  cql_join_unique_build  binding 0 build keys, 1 table (all ones before), 2 status; word 0 rows, 2 log2 of the table's
+//                         size, 4 the key form, 6 the column's CQL type
+//  cql_join_unique_probe  binding 0 probe keys, 1 table, 2 status, 3 the match of each row out (u32 build row, all ones
+//                         without one), 4 matches per CTA out; words as the build's, word 8 1 = write the matches
+//  cql_join_unique_emit   binding 0 the matches, 1 matches per CTA, 2 (probe, build) u32 pairs out, 3 the pairs' number
+//                         out, 4 status (nothing is written unless it is 0); word 0 rows, 2 1 = LEFT join (a row
+//                         without a match gives (row, all ones)), 4 1 = write the pairs
+//
+// Key forms: 0 both sides 32-bit words of one type, compared as they are, with 8-byte entries (key, row); 1 the bits
+// of the f64 values; 2 both sides I64 or both U64, compared as they are: as f64 values they are told apart up to 2^53.
+// Forms 1 and 2 have 16-byte entries. Status bit 0: a build key repeats, bit 1: a key that is NaN, -0.0 or past 2^53:
+// the caller then takes the buckets.
+//
+// 10M probe rows against 1M keys cost an L2 sector a row or two; the buckets read their bounds, their rows and the rows'
+// keys behind one another, after both key columns had been widened to f64, and sorted the pairs: 662 us of kernels,
+// this form 149 (table 28, probe 94, emit 27).
+#define JUNIQ_THREADS 512
+#define JUNIQ_UNROLL 4
+#define JUNIQ_CTAS_PER_SM 3
+#define JUNIQ_EMPTY 0xffffffffffffffffull
+
+template <int FORM>
+__device__ __forceinline__ unsigned long long juniq_key(const void* col, uint32_t type, uint64_t row, uint32_t* bad)
+{
+  if (FORM == 0) return (unsigned long long)__ldcs((const uint32_t*)col + row);
+  if (FORM == 2)
+  {
+    unsigned long long v = __ldcs((const unsigned long long*)col + row);
+    unsigned long long magnitude = (type == 8 && (long long)v < 0) ? 0ull - v : v;
+    if (magnitude > (1ull << 53)) *bad |= 2u;
+    return v ^ 0x8000000000000000ull;   // (all ones, the empty entry, is past 2^53)
+  }
+  unsigned long long b;
+  switch (type)
+  {
+    case 1: b = cql_int_bits((long long)__ldcs((const uint32_t*)col + row)); break;
+    case 7: b = cql_int_bits((long long)__ldcs((const int*)col + row)); break;
+    case 3: b = cql_f32_bits(__ldcs((const uint32_t*)col + row)); break;
+    case 2: b = (unsigned long long)__double_as_longlong((double)__ldcs((const unsigned long long*)col + row)); break;
+    case 8: b = (unsigned long long)__double_as_longlong((double)__ldcs((const long long*)col + row)); break;
+    default: b = __ldcs((const unsigned long long*)col + row); break;
+  }
+  if ((b & 0x7fffffffffffffffull) > 0x7ff0000000000000ull || b == 0x8000000000000000ull) *bad |= 2u;
+  return b;
+}
+
+template <int FORM>
+__device__ __forceinline__ uint32_t juniq_slot(unsigned long long key, uint32_t log2_size)
+{
+  if (FORM == 0) return ((uint32_t)key * 0x9E3779B1u) >> (32u - log2_size);
+  key ^= key >> 32;
+  return (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> 32) >> (32u - log2_size);
+}
+
+template <int FORM>
+__global__ void __launch_bounds__(JOIN_THREADS) k_join_unique_build(CqlLaunch a, uint64_t rows)
+{
+  unsigned long long* table = (unsigned long long*)a.buf[1];
+  uint32_t log2_size = cql_word(a, 2), mask = (1u << log2_size) - 1u, type = cql_word(a, 6), bad = 0;
+  for (uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += (uint64_t)gridDim.x * blockDim.x)
+  {
+    unsigned long long key = juniq_key<FORM>(a.buf[0], type, row, &bad);
+    if (FORM != 0 && key == JUNIQ_EMPTY) continue;   // flagged above
+    uint32_t slot = juniq_slot<FORM>(key, log2_size);
+    unsigned long long entry = FORM == 0 ? (row << 32) | key : key;
+    for (uint32_t p = 0; p <= mask; p++)   // at most half the slots are taken
+    {
+      unsigned long long old = atomicCAS(&table[FORM == 0 ? slot : 2ull * slot], JUNIQ_EMPTY, entry);
+      if (old == JUNIQ_EMPTY)
+      {
+        if (FORM != 0) table[2ull * slot + 1] = row;
+        break;
+      }
+      if (FORM == 0 ? (uint32_t)old == (uint32_t)key : old == key)
+      {
+        bad |= 1u;
+        break;
+      }
+      slot = (slot + 1u) & mask;
+    }
+  }
+  if (bad) atomicOr((uint32_t*)a.buf[2], bad);
+}
+
+// The rows of a CTA: an equal run each, in whole tiles of JUNIQ_THREADS x JUNIQ_UNROLL rows, the same for the probe and
+// the emit.
+struct JoinRuns
+{
+  uint32_t ctas;
+  uint64_t rows_per_cta;
+};
+
+static JoinRuns join_runs(uint64_t rows)
+{
+  const uint64_t tile = JUNIQ_THREADS * JUNIQ_UNROLL;
+  JoinRuns r;
+  uint64_t tiles = (rows + tile - 1) / tile, most = cql_stream_grid(tiles, JUNIQ_CTAS_PER_SM), per = (tiles + most - 1) / most;
+  r.rows_per_cta = per * tile;
+  r.ctas = (uint32_t)((tiles + per - 1) / per);
+  return r;
+}
+
+template <int FORM>
+__global__ void __launch_bounds__(JUNIQ_THREADS, JUNIQ_CTAS_PER_SM) k_join_unique_probe(CqlLaunch a, uint64_t rows, uint64_t rows_per_cta)
+{
+  __shared__ uint32_t s_count;
+  if (*(volatile const uint32_t*)a.buf[2] & 1u) return;   // a build key repeats
+  if (threadIdx.x == 0) s_count = 0;
+  __syncthreads();
+  const unsigned long long* table = (const unsigned long long*)a.buf[1];
+  uint32_t* match_out = (uint32_t*)a.buf[3];
+  uint32_t log2_size = cql_word(a, 2), mask = (1u << log2_size) - 1u, type = cql_word(a, 6), bad = 0, count = 0;
+  bool write = cql_word(a, 8) != 0;
+  uint64_t first = (uint64_t)blockIdx.x * rows_per_cta, end = min(first + rows_per_cta, rows);
+  for (uint64_t base = first + threadIdx.x; base < end; base += JUNIQ_THREADS * JUNIQ_UNROLL)
+  {
+    unsigned long long key[JUNIQ_UNROLL];
+#pragma unroll
+    for (uint32_t u = 0; u < JUNIQ_UNROLL; u++) key[u] = base + u * JUNIQ_THREADS < end ? juniq_key<FORM>(a.buf[0], type, base + u * JUNIQ_THREADS, &bad) : 0ull;
+    // every row's first entry in flight together; a row whose chain goes on walks it below
+    ulonglong2 entry[JUNIQ_UNROLL];
+#pragma unroll
+    for (uint32_t u = 0; u < JUNIQ_UNROLL; u++)
+    {
+      uint32_t slot = juniq_slot<FORM>(key[u], log2_size);
+      if (FORM == 0) entry[u].x = __ldg(&table[slot]);
+      else entry[u] = __ldg((const ulonglong2*)table + slot);
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < JUNIQ_UNROLL; u++)
+    {
+      uint64_t row = base + u * JUNIQ_THREADS;
+      if (row >= end) continue;
+      ulonglong2 t = entry[u];
+      uint32_t slot = juniq_slot<FORM>(key[u], log2_size), found = BUILD_NULL;
+      for (uint32_t p = 0; p <= mask && t.x != JUNIQ_EMPTY; p++)
+      {
+        if (FORM == 0 ? (uint32_t)t.x == (uint32_t)key[u] : t.x == key[u])
+        {
+          found = FORM == 0 ? (uint32_t)(t.x >> 32) : (uint32_t)t.y;
+          break;
+        }
+        slot = (slot + 1u) & mask;
+        if (FORM == 0) t.x = __ldg(&table[slot]);
+        else t = __ldg((const ulonglong2*)table + slot);
+      }
+      count += found != BUILD_NULL;
+      if (write) match_out[row] = found;
+    }
+  }
+  if (bad) atomicOr((uint32_t*)a.buf[2], bad);
+  if (count) atomicAdd(&s_count, count);
+  __syncthreads();
+  if (threadIdx.x == 0) ((uint32_t*)a.buf[4])[blockIdx.x] = s_count;
+}
+
+__global__ void __launch_bounds__(JUNIQ_THREADS, JUNIQ_CTAS_PER_SM) k_join_unique_emit(CqlLaunch a, uint64_t rows, uint64_t rows_per_cta)
+{
+  __shared__ uint32_t s_warp[JUNIQ_THREADS / 32], s_before;
+  const uint32_t* match = (const uint32_t*)a.buf[0];
+  const uint32_t* counts = (const uint32_t*)a.buf[1];
+  uint2* pairs = (uint2*)a.buf[2];
+  bool left = cql_word(a, 2) != 0, write = cql_word(a, 4) != 0;
+  uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, mine = 0;
+  if (*(const uint32_t*)a.buf[4]) return;
+  if (threadIdx.x == 0) s_before = 0;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += JUNIQ_THREADS) mine += counts[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if (lane == 0 && mine) atomicAdd(&s_before, mine);
+  __syncthreads();
+  uint64_t first = (uint64_t)blockIdx.x * rows_per_cta, end = min(first + rows_per_cta, rows);
+  uint64_t run = left ? first : s_before;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *(uint32_t*)a.buf[3] = left ? (uint32_t)rows : s_before + counts[blockIdx.x];
+  if (!write) return;
+  // a warp's rows of a tile are consecutive, 32 a round: ballots rank them, a sum over the warps before places the warp
+  for (uint64_t tile = first; tile < end; tile += JUNIQ_THREADS * JUNIQ_UNROLL)
+  {
+    uint64_t row0 = tile + warp * 32u * JUNIQ_UNROLL + lane;
+    uint32_t found[JUNIQ_UNROLL], kept[JUNIQ_UNROLL], total = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < JUNIQ_UNROLL; u++) found[u] = row0 + 32u * u < end ? __ldcs(match + row0 + 32u * u) : BUILD_NULL;
+#pragma unroll
+    for (uint32_t u = 0; u < JUNIQ_UNROLL; u++)
+    {
+      kept[u] = __ballot_sync(0xffffffffu, row0 + 32u * u < end && (left || found[u] != BUILD_NULL));
+      total += (uint32_t)__popc(kept[u]);
+    }
+    __syncthreads();
+    if (lane == 0) s_warp[warp] = total;
+    __syncthreads();
+    uint64_t at = run;
+    uint32_t all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < JUNIQ_THREADS / 32; w++)
+    {
+      uint32_t n = s_warp[w];
+      if (w < warp) at += n;
+      all += n;
+    }
+    run += all;
+#pragma unroll
+    for (uint32_t u = 0; u < JUNIQ_UNROLL; u++)
+    {
+      if ((kept[u] >> lane) & 1u) pairs[at + __popc(kept[u] & ((1u << lane) - 1u))] = make_uint2((uint32_t)(row0 + 32u * u), found[u]);
+      at += __popc(kept[u]);
+    }
+  }
+}
+
+static int join_unique_check(const CqlLaunch& a, uint64_t rows)
+{
+  uint32_t log2_size = cql_word(a, 2), form = cql_word(a, 4), type = cql_word(a, 6);
+  bool wide = type == 2 || type == 4 || type == 8;
+  return rows <= 0xffffffffull && log2_size >= 4 && log2_size <= 29 && form <= 2 && (wide || type == 1 || type == 3 || type == 7) &&
+         (form != 0 || !wide) && (form != 2 || type == 2 || type == 8) && a.bytes[0] >= rows * (wide ? 8 : 4) &&
+         a.bytes[1] >= ((form == 0 ? 8ull : 16ull) << log2_size) && a.bytes[2] >= 4;
+}
+
+static int launch_join_unique_build(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t rows = a.push[0];
+  if (rows == 0) return 0;
+  if (!join_unique_check(a, rows) || rows * 2 > (1ull << cql_word(a, 2))) return (int)cudaErrorInvalidValue;
+  uint32_t grid = cql_stream_grid((rows + JOIN_THREADS - 1) / JOIN_THREADS, 8);
+  switch (cql_word(a, 4))
+  {
+    case 0: k_join_unique_build<0><<<grid, JOIN_THREADS, 0, stream>>>(a, rows); break;
+    case 1: k_join_unique_build<1><<<grid, JOIN_THREADS, 0, stream>>>(a, rows); break;
+    default: k_join_unique_build<2><<<grid, JOIN_THREADS, 0, stream>>>(a, rows); break;
+  }
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
+static int launch_join_unique_probe(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t rows = a.push[0];
+  if (rows == 0) return 0;
+  JoinRuns r = join_runs(rows);
+  if (!join_unique_check(a, rows) || (cql_word(a, 8) && a.bytes[3] < rows * 4) || a.bytes[4] < r.ctas * 4ull) return (int)cudaErrorInvalidValue;
+  switch (cql_word(a, 4))
+  {
+    case 0: k_join_unique_probe<0><<<r.ctas, JUNIQ_THREADS, 0, stream>>>(a, rows, r.rows_per_cta); break;
+    case 1: k_join_unique_probe<1><<<r.ctas, JUNIQ_THREADS, 0, stream>>>(a, rows, r.rows_per_cta); break;
+    default: k_join_unique_probe<2><<<r.ctas, JUNIQ_THREADS, 0, stream>>>(a, rows, r.rows_per_cta); break;
+  }
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
+static int launch_join_unique_emit(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaStream_t stream)
+{
+  (void)gws;
+  (void)lws;
+  uint64_t rows = a.push[0];
+  if (rows == 0) return 0;
+  JoinRuns r = join_runs(rows);
+  bool write = cql_word(a, 4) != 0;
+  if (rows > 0xffffffffull || (write && (a.bytes[0] < rows * 4 || a.bytes[2] < rows * 8)) || a.bytes[1] < r.ctas * 4ull || a.bytes[3] < 4 || a.bytes[4] < 4)
+    return (int)cudaErrorInvalidValue;
+  k_join_unique_emit<<<r.ctas, JUNIQ_THREADS, 0, stream>>>(a, rows, r.rows_per_cta);
+  CQL_LAUNCH_CHECK();
+  return 0;
+}
+
 const CqlKernelDesc cql_kernels_join[] = {
   { "hash_join_build_count", launch_join_build_count },
   { "prefix_sum", launch_prefix_sum },
@@ -1291,5 +1568,8 @@ const CqlKernelDesc cql_kernels_join[] = {
   { "cql_join_hash_build", launch_join_hash_build },
   { "cql_join_hash_probe", launch_join_hash_probe },
   { "cql_join_group_range", launch_join_group_range },
+  { "cql_join_unique_build", launch_join_unique_build },
+  { "cql_join_unique_probe", launch_join_unique_probe },
+  { "cql_join_unique_emit", launch_join_unique_emit },
   { nullptr, nullptr },
 };

@@ -343,7 +343,7 @@ static int scan_filter_run(const CqlProgram* prog, const CqlColumn* columns, uin
     uint64_t m = result < out_capacity ? result : out_capacity;
     uint32_t* pairs = (uint32_t*)malloc(m * 8);
     if (!pairs) return 0;
-    if (!cqlops_sort_pairs(output, result, 2, 0, 1, 0, pairs, out_capacity))
+    if (!cqlops_sort_pairs(output, result, 2, 0, 1, 0, 32, 32, pairs, out_capacity))
     {
       free(pairs);
       return 0;

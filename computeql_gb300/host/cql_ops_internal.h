@@ -18,7 +18,7 @@ int cqlops_bitmap_rows_enqueue(CqlBatch* b, CqlBuffer* bitmap, uint64_t first_ro
 
 /* result pairs put in order on the device by the radix sort (cql_ops_sort.c) */
 int cqlops_sort_pairs(CqlBuffer* records, uint64_t n, uint32_t stride_words, uint32_t first_word, uint32_t second_word, int by_second,
-                      uint32_t* out, uint64_t out_capacity);
+                      uint32_t first_bits, uint32_t second_bits, uint32_t* out, uint64_t out_capacity);
 
 /* The dense group-by's totals left on the device for a caller's next operations: the counts (u64 per group,
    from 0), the sums (two u32 words per group and expression) at sum_at, MIN and MAX (i32 per group and

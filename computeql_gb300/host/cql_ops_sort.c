@@ -340,9 +340,10 @@ int cqlops_sort_rows(const CqlColumn* keys, uint32_t key_count, const uint32_t* 
 /* Result pairs put in order on the device (the join's pair output, the scan's rows with their scores): n
    records of stride_words u32 words in `records`; the pair (word first_word, word second_word) of each,
    sorted by the first word then the second (by_second) or by the first alone (ties by position) with the
-   radix sort above, and up to out_capacity sorted pairs (first, second) read into out. */
+   radix sort above, and up to out_capacity sorted pairs (first, second) read into out. first_bits and second_bits: below
+   which bit each word orders (32: all of it), so that row numbers are sorted by the bytes they have. */
 int cqlops_sort_pairs(CqlBuffer* records, uint64_t n, uint32_t stride_words, uint32_t first_word, uint32_t second_word, int by_second,
-                      uint32_t* out, uint64_t out_capacity)
+                      uint32_t first_bits, uint32_t second_bits, uint32_t* out, uint64_t out_capacity)
 {
   if (n == 0 || out_capacity == 0) return 1;
   if (!cqlops_rows_fit(n)) return 0;
@@ -371,7 +372,8 @@ int cqlops_sort_pairs(CqlBuffer* records, uint64_t n, uint32_t stride_words, uin
   cqlcuda_kernel_set_arg_u64(unpack, 3, second_word);
   cqlcuda_batch_kernel_execute(b, unpack, (uint32_t)n, QE_GPU_WORKGROUP_SIZE);
   CqlBuffer* sorted = NULL;
-  if (!sort_enqueue(b, keys, by_second ? 2u : 1u, NULL, NULL, n, NULL, &sorted))
+  uint32_t top_bits[4] = { first_bits, second_bits, 0, 0 };
+  if (!sort_enqueue(b, keys, by_second ? 2u : 1u, NULL, NULL, n, top_bits, &sorted))
   {
     cqlcuda_batch_end(b);
     return 0;
