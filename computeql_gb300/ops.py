@@ -174,7 +174,7 @@ def scan_simple(columns, leaves, want_rows=False, max_rows=None):
         out_ptr = N.ptr(rows)
     _check(N.load_ops().cqlops_scan_simple(arr, len(columns), lv, len(leaves), C.byref(count), out_ptr, cap), "cqlops_scan_simple")
     if want_rows:
-        rows = rows[: min(count.value, cap)]     # a view: the pages past the rows were never touched
+        rows = rows[: min(count.value, cap)].copy()
     return count.value, rows
 
 
@@ -339,7 +339,7 @@ def scan_filter(program, strategy=SCAN_AUTO, want_rows=False, max_rows=None):
     ok = N.load_ops().cqlops_scan_filter(C.byref(program.prog), program._cols, strategy, C.byref(count),
                                          N.ptr(rows_arr) if want_rows else None, cap, C.byref(ran))
     _check(ok, "cqlops_scan_filter")
-    rows = rows_arr[: min(count.value, cap)] if want_rows else None     # a view: the pages past the rows were never touched
+    rows = rows_arr[: min(count.value, cap)].copy() if want_rows else None
     return count.value, rows, ran.value
 
 
