@@ -752,13 +752,15 @@ static int launch_selection_gather(const CqlLaunch& a, uint32_t gws, uint32_t lw
 }
 
 // ---------------------------------------------------------------------------------------------
-// Row materialization: the values of the selected rows of many columns, the multi-column form of the
-// reference's per-column gathers (selection_gather.comp modes 0 and 1, qe_selection_gather_column
-// query_exec.c:4371-4410). One launch covers up to GATHER_COLUMNS columns, column j on blockIdx.y,
-// so the selected row numbers are read once per column from L2 and every store is coalesced.
+// Row materialization: the values of the selected rows of many columns, the multi-column form of the reference's
+// per-column gathers (selection_gather.comp modes 0 and 1, qe_selection_gather_column query_exec.c:4371-4410). One
+// launch takes every column, column j on blockIdx.y: a column's address is in its params, so their number is not bound
+// by the bindings (13 a launch before). A sparse selection's rows each cost a sector of every column, one DRAM latency
+// after the row number's; four rows a thread in flight, and CTAs for every row of a few columns at a time, hide it. With
+// one row in flight and 30 CTAs a column 100k rows of 28 columns took three launches of 24 us, this form one of 59 (20M rows at 5 %, near the sectors that hold them: 332 us).
 //
-//  cql_gather_columns  binding 0 selected rows (u32), 1 per-column params (u32 x 4: kind, base,
-//                      destination byte offset lo, hi), 2 destination, 3.. the columns' buffers;
+//  cql_gather_columns  binding 0 selected rows (u32), 1 per-column params (u32 x 8: kind, base, destination byte
+//                      offset, the column's address, its bytes: the last three u64), 2 destination;
 //                      word 0 count, word 2 1 = rows given (else rows 0..count-1), word 4 columns.
 //                      kind 0 4-byte values, 1 u8 codes (base + code), 2 u16 codes, 3 a sequence
 //                      (base + row, nothing read), 4 8-byte values, 5 1-byte values (BOOL)
@@ -769,35 +771,52 @@ static int launch_selection_gather(const CqlLaunch& a, uint32_t gws, uint32_t lw
 //                      rows given. A warp per selected row, its lanes over the row's bytes.
 // A row past a column's buffer reads as zero (the host checks the selection first).
 
-#define GATHER_COLUMNS 13
+#define GATHER_UNROLL 4
+
+template <typename SRC, typename DST>
+__device__ __forceinline__ void gather_column(const uint32_t* rows, const SRC* src, uint64_t src_rows, DST* dest, DST base, uint64_t count)
+{
+  const uint64_t step = (uint64_t)gridDim.x * HASH_THREADS;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * HASH_THREADS + threadIdx.x; i0 < count; i0 += step * GATHER_UNROLL)
+  {
+    uint64_t r[GATHER_UNROLL];
+    SRC v[GATHER_UNROLL];
+#pragma unroll
+    for (uint32_t u = 0; u < GATHER_UNROLL; u++)
+    {
+      uint64_t i = min(i0 + u * step, count - 1);
+      r[u] = rows ? rows[i] : i;
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < GATHER_UNROLL; u++) v[u] = r[u] < src_rows ? src[r[u]] : (SRC)0;
+#pragma unroll
+    for (uint32_t u = 0; u < GATHER_UNROLL; u++)
+      if (i0 + u * step < count) dest[i0 + u * step] = base + (DST)v[u];
+  }
+}
 
 __global__ void __launch_bounds__(HASH_THREADS) k_gather_columns(CqlLaunch a, uint64_t count)
 {
-  const uint32_t* rows = (const uint32_t*)a.buf[0];
-  const uint32_t* params = (const uint32_t*)a.buf[1];
-  unsigned char* dest = (unsigned char*)a.buf[2];
-  bool given = cql_word(a, 2) != 0;
-  uint32_t j = blockIdx.y;
-  const uint32_t* pj = params + j * 4;
+  const uint32_t* pj = (const uint32_t*)a.buf[1] + blockIdx.y * 8;
+  const uint32_t* rows = cql_word(a, 2) ? (const uint32_t*)a.buf[0] : nullptr;
   uint32_t kind = pj[0], base = pj[1];
-  uint64_t off = (uint64_t)pj[2] | ((uint64_t)pj[3] << 32);
-  const void* src = a.buf[3 + j];
-  uint64_t src_bytes = a.bytes[3 + j];
+  uint64_t off = ((const uint64_t*)pj)[1], bytes = ((const uint64_t*)pj)[3];
+  const void* src = (const void*)((const uint64_t*)pj)[2];
   // the column's section must lie inside the destination
   uint64_t size = kind == 4 ? 8 : kind == 5 ? 1 : 4;
   if (off % size != 0 || off > a.bytes[2] || count > (a.bytes[2] - off) / size) return;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x)
+  void* dest = (char*)a.buf[2] + off;
+  switch (kind)
   {
-    uint64_t r = given ? rows[i] : i;
-    switch (kind)
-    {
-      case 0: ((uint32_t*)(dest + off))[i] = (r + 1) * 4 <= src_bytes ? ((const uint32_t*)src)[r] : 0u; break;
-      case 1: ((uint32_t*)(dest + off))[i] = base + (r < src_bytes ? (uint32_t)((const uint8_t*)src)[r] : 0u); break;
-      case 2: ((uint32_t*)(dest + off))[i] = base + ((r + 1) * 2 <= src_bytes ? (uint32_t)((const uint16_t*)src)[r] : 0u); break;
-      case 3: ((uint32_t*)(dest + off))[i] = base + (uint32_t)r; break;
-      case 4: ((unsigned long long*)(dest + off))[i] = (r + 1) * 8 <= src_bytes ? ((const unsigned long long*)src)[r] : 0ull; break;
-      default: (dest + off)[i] = r < src_bytes ? ((const uint8_t*)src)[r] : (uint8_t)0; break;
-    }
+    case 0: gather_column(rows, (const uint32_t*)src, bytes / 4, (uint32_t*)dest, 0u, count); break;
+    case 1: gather_column(rows, (const uint8_t*)src, bytes, (uint32_t*)dest, base, count); break;
+    case 2: gather_column(rows, (const uint16_t*)src, bytes / 2, (uint32_t*)dest, base, count); break;
+    case 3:
+      for (uint64_t i = (uint64_t)blockIdx.x * HASH_THREADS + threadIdx.x; i < count; i += (uint64_t)gridDim.x * HASH_THREADS)
+        ((uint32_t*)dest)[i] = base + (rows ? rows[i] : (uint32_t)i);
+      break;
+    case 4: gather_column(rows, (const unsigned long long*)src, bytes / 8, (unsigned long long*)dest, 0ull, count); break;
+    default: gather_column(rows, (const uint8_t*)src, bytes, (uint8_t*)dest, (uint8_t)0, count); break;
   }
 }
 
@@ -843,10 +862,10 @@ static int launch_gather_columns(const CqlLaunch& a, uint32_t gws, uint32_t lws,
   uint64_t count = cql_word(a, 0);
   uint32_t cols = cql_word(a, 4);
   if (count == 0 || cols == 0) return 0;
-  if (cols > GATHER_COLUMNS || a.bytes[1] < cols * 16ull || (cql_word(a, 2) && a.bytes[0] < count * 4)) return (int)cudaErrorInvalidValue;
-  uint32_t blocks = cql_stream_grid((count + HASH_THREADS - 1) / HASH_THREADS, 8);
-  uint32_t x = (blocks + cols - 1) / cols;
-  k_gather_columns<<<dim3(x ? x : 1, cols), HASH_THREADS, 0, stream>>>(a, count);
+  if (cols > 65535 || a.bytes[1] < cols * 32ull || (cql_word(a, 2) && a.bytes[0] < count * 4)) return (int)cudaErrorInvalidValue;
+  // a quarter of the resident CTAs a column at most: the columns past the first few follow as those finish
+  uint32_t x = cql_stream_grid((count + HASH_THREADS * GATHER_UNROLL - 1) / (HASH_THREADS * GATHER_UNROLL), 2);
+  k_gather_columns<<<dim3(x, cols), HASH_THREADS, 0, stream>>>(a, count);
   CQL_LAUNCH_CHECK();
   return 0;
 }

@@ -15,7 +15,6 @@
 #include <stdlib.h>
 #include <string.h>
 
-#define GATHER_COLUMNS 13
 #define QE_GPU_WORKGROUP_SIZE 256
 
 static int refuse(const char* why)
@@ -103,7 +102,8 @@ int cqlops_gather_rows(const CqlColumn* columns, uint32_t column_count, const ui
   if (column_count == 0 || count == 0) return 1;
   if (!columns || !out_values) return refuse("columns and outputs are required");
   if (!cqlops_rows_fit(count)) return 0;
-  uint32_t* params = (uint32_t*)calloc((size_t)column_count * 4, sizeof(uint32_t));
+  if (column_count > 65535) return refuse("at most 65535 columns");
+  uint32_t* params = (uint32_t*)calloc((size_t)column_count * 8, sizeof(uint32_t));
   uint64_t* section = (uint64_t*)malloc((size_t)column_count * sizeof(uint64_t));
   uint32_t* sizes = (uint32_t*)malloc((size_t)column_count * sizeof(uint32_t));
   if (!params || !section || !sizes)
@@ -126,41 +126,37 @@ int cqlops_gather_rows(const CqlColumn* columns, uint32_t column_count, const ui
     if (columns[c].rows < min_rows) min_rows = columns[c].rows;
     section[c] = total;
     sizes[c] = size;
-    params[c * 4 + 0] = kind;
-    params[c * 4 + 1] = columns[c].base;
-    params[c * 4 + 2] = (uint32_t)total;
-    params[c * 4 + 3] = (uint32_t)(total >> 32);
+    uint64_t place[3] = { total, 0, 0 };   /* in the destination; the column's address and bytes */
+    if (columns[c].buffer)
+    {
+      place[1] = (uint64_t)(uintptr_t)cqlcuda_buffer_device_pointer(columns[c].buffer);
+      place[2] = cqlcuda_buffer_size(columns[c].buffer);
+    }
+    params[c * 8 + 0] = kind;
+    params[c * 8 + 1] = columns[c].base;
+    memcpy(&params[c * 8 + 2], place, sizeof(place));
     total += (count * size + 15) & ~15ull;
   }
   CqlBuffer* dest = ok ? pooled("gather_dest", total, CQLCUDA_BUFFER_READ_WRITE) : NULL;
-  CqlBuffer* pbuf = ok ? pooled("gather_params", (uint64_t)column_count * 16, CQLCUDA_BUFFER_WRITE) : NULL;
+  CqlBuffer* pbuf = ok ? pooled("gather_params", (uint64_t)column_count * 32, CQLCUDA_BUFFER_WRITE) : NULL;
   CqlKernel* k = ok ? cqlcuda_kernel_alloc("cql_gather_columns", strlen("cql_gather_columns")) : NULL;
   ok = ok && dest && pbuf && k;
   if (ok)
   {
-    CqlBatch* b = cqlcuda_batch_begin(count * 4 + (uint64_t)column_count * 16, total);
+    CqlBatch* b = cqlcuda_batch_begin(count * 4 + (uint64_t)column_count * 32, total);
     CqlBuffer* sel = NULL;
     uint32_t given = 0;
     ok = selection_source(b, rows, selection, count, min_rows, &sel, &given);
     if (ok)
     {
-      cqlcuda_batch_buffer_write(b, pbuf, params, (uint64_t)column_count * 16);
-      for (uint32_t first = 0; first < column_count; first += GATHER_COLUMNS)
-      {
-        uint32_t n = column_count - first < GATHER_COLUMNS ? column_count - first : GATHER_COLUMNS;
-        cqlcuda_kernel_set_arg_buffer(k, 0, sel ? sel : pbuf);
-        cqlcuda_kernel_set_arg_buffer_range(k, 1, pbuf, (uint64_t)first * 16, (uint64_t)n * 16);
-        cqlcuda_kernel_set_arg_buffer(k, 2, dest);
-        for (uint32_t j = 0; j < GATHER_COLUMNS; j++)
-        {
-          CqlBuffer* src = j < n ? columns[first + j].buffer : NULL;
-          cqlcuda_kernel_set_arg_buffer(k, 3 + j, src ? src : pbuf);
-        }
-        cqlcuda_kernel_set_arg_u64(k, 0, count);
-        cqlcuda_kernel_set_arg_u64(k, 1, given);
-        cqlcuda_kernel_set_arg_u64(k, 2, n);
-        cqlcuda_batch_kernel_execute(b, k, (uint32_t)count, QE_GPU_WORKGROUP_SIZE);
-      }
+      cqlcuda_batch_buffer_write(b, pbuf, params, (uint64_t)column_count * 32);
+      cqlcuda_kernel_set_arg_buffer(k, 0, sel ? sel : pbuf);
+      cqlcuda_kernel_set_arg_buffer(k, 1, pbuf);
+      cqlcuda_kernel_set_arg_buffer(k, 2, dest);
+      cqlcuda_kernel_set_arg_u64(k, 0, count);
+      cqlcuda_kernel_set_arg_u64(k, 1, given);
+      cqlcuda_kernel_set_arg_u64(k, 2, column_count);
+      cqlcuda_batch_kernel_execute(b, k, (uint32_t)count, QE_GPU_WORKGROUP_SIZE);
       /* outputs laid out as the device sections are (one host block, each column at its section's offset):
          one read of the whole block; else a read a column */
       int contiguous = 1;
