@@ -54,13 +54,15 @@ enum
   OP_STR_EQ = 11, OP_STR_CONTAINS = 12, OP_TRIGRAM_SIM = 15, OP_EDIT_DISTANCE = 16, OP_STR_NE = 17, OP_STR_GE = 21,
 };
 
-/* a threshold, 32 bytes: a/b the interval (low, span), c = invert (or the op of a float test), d = strict */
+/* a threshold, 32 bytes: a/b the interval (low, span), c = invert (or the op of a float test), d = strict;
+   site: the column it tests plus one (0 = no comparison), THR_F32 with a float test (the host's own use) */
 typedef struct
 {
   uint64_t a, b;
   uint32_t c, d;
-  uint64_t pad;
+  uint64_t site;
 } Thr;
+#define THR_F32 0x100u
 
 /* ---- thresholds, worked out on the host ---- */
 
@@ -822,6 +824,387 @@ static char* batch_source_tiled(char** shape_exprs, const uint32_t* shape_sites,
   return b.p;
 }
 
+/* ---- the rank form ---- */
+
+/* A batch's comparisons of one column with literals split the column's values into few ranges: with the
+   literals' cut points sorted, a value's rank (how many cuts are at or below it) decides every one of them.
+   A CTA turns a tile of rows into ranks once - a byte a row and column, four rows a word - and the summed
+   columns into byte planes of their fixed-point summands; each comparison is then two subtractions and one
+   logical operation for four rows (bit 7 of each byte), and each plane's sum one __dp4a of the match bytes
+   with the plane. A warp takes one query over the tile, its lanes 16 rows a step, and adds the query's
+   totals to the CTA's accumulators once per tile.
+
+   What bounds it is the integer pipe: the register form spends about 31 warp instructions per query and 32
+   rows (64-bit interval compares, mask assembly, predicated 64-bit adds, five reductions every 8 rows),
+   this one about 6, plus about 200 a row for the ranks and planes, whatever the number of queries.
+
+   Ranks are at most RANK_CUTS (the cuts of a launch on one column), so a rank with bit 7 set minus a bound
+   in [0, 128] keeps bit 7 exactly when it is at or above the bound, with no borrow between the bytes. */
+#define RANK_CUTS 127u
+#define RANK_TABLE (RANK_CUTS + 1u)                                     /* a column's cuts, padded to a power of two */
+#define RANK_CUT_BYTES (CQLOPS_MAX_BINDINGS * RANK_TABLE * 8u + 64u)    /* a launch's cuts, then each column's search steps */
+#define RANK_QUERIES 192u       /* a launch's queries: its accumulators leave room for three CTAs an SM */
+#define RANK_MIN_LAUNCH 48u     /* launches are halved down to this many while their cuts do not fit */
+#define RANK_MIN_QUERIES 2u
+#define FORM_REGISTERS (1u << 24)   /* with a form: not as ranks */
+#define RANK_BAD (1ull << 44)   /* added to the first query's count by a CTA that met a summand outside its planes */
+
+/* a launch's per-query thresholds: four copies of each bound, and the inversion in bit 7 */
+typedef struct
+{
+  uint32_t lo, hi, inv, pad;
+} RankThr;
+
+typedef struct
+{
+  uint32_t tile, per_sm, smem, planes;
+} RankLayout;
+
+/* whether a shape's predicate is comparisons of columns with literals joined by & and | alone */
+static int rank_expr(const char* e)
+{
+  while (*e)
+  {
+    unsigned slot, site;
+    int n = 0;
+    if (*e == '(' || *e == ')' || *e == ' ' || *e == '&' || *e == '|')
+    {
+      e++;
+      continue;
+    }
+    if ((sscanf(e, "cql_bi(&T%u, r%u[k] ^ 0x80000000u)%n", &site, &slot, &n) == 2 && n) || (sscanf(e, "cql_bi(&T%u, r%u[k])%n", &site, &slot, &n) == 2 && n) ||
+        (sscanf(e, "cql_bf(&T%u, __uint_as_float(r%u[k]))%n", &site, &slot, &n) == 2 && n) ||
+        (sscanf(e, "cql_bk(&T%u, kd%u[k])%n", &site, &slot, &n) == 2 && n))
+    {
+      e += n;
+      continue;
+    }
+    return 0;
+  }
+  return 1;
+}
+
+/* the layout: byte planes of the summands (|summand| <= 2^(62 - bits of an accumulator's rows), so 6 bytes
+   from 2^15 rows on, else 7) and 2048 rows a tile where three CTAs then fit an SM, else 1024 */
+static RankLayout rank_layout(const int* slot_type, uint32_t sum_col_count, int warp_row_bits)
+{
+  RankLayout l;
+  uint32_t slots = 0, cuts = 0;
+  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
+    if (slot_type[s])
+    {
+      slots++;
+      cuts += RANK_TABLE * (slot_type[s] == CQLOPS_TYPE_F64 ? 8u : 4u);
+    }
+  l.planes = warp_row_bits >= 16 ? 6u : 7u;
+  const uint32_t fixed = RANK_QUERIES * 13u + cuts;   /* sums, counts and shapes per query */
+  const uint32_t row = slots + 1u + sum_col_count * l.planes;
+  l.tile = row * 2048u + fixed <= 75u * 1024u ? 2048u : 1024u;
+  l.smem = (row * l.tile + fixed + 15u) & ~15u;
+  uint32_t per_sm = (227u * 1024u) / (l.smem + 1024u);
+  l.per_sm = per_sm > 5 ? 5 : (per_sm < 1 ? 1 : per_sm);
+  return l;
+}
+
+static const char* RANK_PRELUDE =
+  "struct RankThr { u32 lo, hi, inv, pad; };\n"
+  "struct Rk { u32 v; };\n"
+  "struct Mk { u32 m; };\n"
+  "__device__ __forceinline__ Rk operator^(Rk a, u32) { return a; }\n"
+  "__device__ __forceinline__ Mk operator&(Mk a, Mk b) { Mk r; r.m = a.m & b.m; return r; }\n"
+  "__device__ __forceinline__ Mk operator|(Mk a, Mk b) { Mk r; r.m = a.m | b.m; return r; }\n"
+  "__device__ __forceinline__ Mk cql_rk(const RankThr* t, Rk r) { Mk m; m.m = ((r.v - t->lo) & ~(r.v - t->hi)) ^ t->inv; return m; }\n"
+  /* four rows' 64-bit words to byte planes: plane p holds byte p of each row */
+  "__device__ __forceinline__ void cql_planes(u32 a, u32 b, u32 c, u32 d, u32& p0, u32& p1, u32& p2, u32& p3)\n"
+  "{\n"
+  "  const u32 x = __byte_perm(a, b, 0x5140), y = __byte_perm(c, d, 0x5140), z = __byte_perm(a, b, 0x7362), w = __byte_perm(c, d, 0x7362);\n"
+  "  p0 = __byte_perm(x, y, 0x5410); p1 = __byte_perm(x, y, 0x7632); p2 = __byte_perm(z, w, 0x5410); p3 = __byte_perm(z, w, 0x7632);\n"
+  "}\n";
+
+static char* batch_source_ranks(char** shape_exprs, const uint32_t* shape_sites, uint32_t shapes, const int* slot_type, const int* sum_cols,
+                                uint32_t sum_col_count, int warp_row_bits)
+{
+  const RankLayout L = rank_layout(slot_type, sum_col_count, warp_row_bits);
+  const uint32_t words = L.tile / 4u, quads = words / QE_GPU_WORKGROUP_SIZE;
+  Buf b;
+  memset(&b, 0, sizeof(b));
+  bput(&b, "// cql: block=%u smem=%u per_sm=%u\n", QE_GPU_WORKGROUP_SIZE, L.smem, L.per_sm);
+  bput(&b, "%s%s", BATCH_PRELUDE, RANK_PRELUDE);
+  for (uint32_t s = 0; s < shapes; s++) bput(&b, "#define CQL_SHAPE_%u(k) (%s)\n", s, shape_exprs[s]);
+  /* the summand n of a row as the low bytes of 1.5 * 2^52 (+ 2^47 with 6 planes) + n, the double nearest to
+     value * 2^k plus that number: one fused multiply-add rounds as cql_fx64 does. The high bits tell a value
+     outside its column's stated range (or a NaN), which the planes cannot hold. */
+  const char* magic = L.planes == 6u ? "0x4338800000000000ull" : "0x4338000000000000ull";
+  const char* bias = L.planes == 6u ? "0x0000800000000000ull" : "0x0038000000000000ull";
+  bput(&b,
+       "extern \"C\" __global__ void __launch_bounds__(%u, %u) cql_main(CqlLaunch a)\n{\n"
+       "  const u32 TILE = %uu, WORDS = %uu, QUADS = %uu;\n"
+       "  const u64 rows = cql_word(a, 0); const u32 nq = cql_word(a, 2); const u32 q0 = cql_word(a, 4);\n"
+       "  const u32 need = cql_word(a, 6), need_sum = cql_word(a, 7);   /* the columns this launch reads and sums */\n"
+       "  const double* col_scale = (const double*)a.buf[0];   /* 2^k per summed column, then k at [16 + column] */\n"
+       "  const long long* col_shift = (const long long*)a.buf[0] + 16;\n"
+       "  const RankThr* thr = (const RankThr*)a.buf[1];\n"
+       "  const u64* cuts = (const u64*)a.buf[2];\n"
+       "  const u32* steps = (const u32*)(cuts + %uu);\n"
+       "  const u32* qsum = (const u32*)a.buf[3];\n"
+       "  const u32* shape_begin = (const u32*)a.buf[4];\n"
+       "  u64* partials = (u64*)a.buf[5]; const u64 pcap = a.bytes[5] / 24ull;\n"
+       "  (void)col_scale; (void)col_shift; (void)need_sum; (void)need;\n"
+       "  extern __shared__ uint4 s_mem[];\n"
+       "  u32* s_words = (u32*)s_mem;\n",
+       QE_GPU_WORKGROUP_SIZE, L.per_sm, L.tile, words, quads, CQLOPS_MAX_BINDINGS * RANK_TABLE);
+  /* shared memory: the words of every column's ranks, the ones, the planes, then sums, cuts, counts and shapes */
+  uint32_t at = 0;
+  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
+    if (slot_type[s]) bput(&b, "  u32* const s_rk%d = s_words + %uu;\n", s, at++ * words);
+  bput(&b, "  u32* const s_one = s_words + %uu;\n", at++ * words);
+  for (uint32_t i = 0; i < sum_col_count; i++, at += L.planes) bput(&b, "  u32* const s_pl%d = s_words + %uu;\n", sum_cols[i], at * words);
+  bput(&b, "  u64* const s_sum = (u64*)(s_words + %uu);\n", at * words);
+  uint32_t off = 0;
+  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
+    if (slot_type[s] == CQLOPS_TYPE_F64) bput(&b, "  u64* const s_cut%d = s_sum + %uu;\n", s, RANK_QUERIES + off++ * RANK_TABLE);
+  bput(&b, "  u32* const s_cnt = (u32*)(s_sum + %uu);\n", RANK_QUERIES + off * RANK_TABLE);
+  off = 0;
+  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
+    if (slot_type[s] && slot_type[s] != CQLOPS_TYPE_F64) bput(&b, "  u32* const s_cut%d = s_cnt + %uu;\n", s, RANK_QUERIES + off++ * RANK_TABLE);
+  bput(&b,
+       "  unsigned char* const s_shape = (unsigned char*)(s_cnt + %uu);\n"
+       "  const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;\n"
+       "  for (u32 q = threadIdx.x; q < nq; q += %uu) { s_sum[q] = 0ull; s_cnt[q] = 0u; u32 s = 0u; while (s + 1u < %uu && q >= shape_begin[s + 1u]) s++; s_shape[q] = (unsigned char)s; }\n",
+       RANK_QUERIES + off * RANK_TABLE, QE_GPU_WORKGROUP_SIZE, shapes);
+  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
+    if (slot_type[s])
+      bput(&b, "  for (u32 i = threadIdx.x; i < %uu; i += %uu) s_cut%d[i] = (%s)cuts[%u + i];\n", RANK_TABLE, QE_GPU_WORKGROUP_SIZE, s,
+           slot_type[s] == CQLOPS_TYPE_F64 ? "u64" : "u32", (uint32_t)s * RANK_TABLE);
+  bput(&b,
+       "  u32 bad = 0u;   /* bits that differ from the magic number's above the summand's field */\n"
+       "  /* a query is also split over the tile's rows where there are too few queries to go round the warps */\n"
+       "  const u32 parts = nq >= 32u ? 1u : (nq >= 16u ? 2u : (WORDS / 128u < 4u ? 2u : 4u));\n"
+       "  const u32 items = nq * parts, span = WORDS / 128u / parts;\n"
+       "  const u64 tiles = (rows + TILE - 1ull) / TILE;\n"
+       "  for (u64 t = blockIdx.x; t < tiles; t += gridDim.x)\n  {\n"
+       "    const u64 base = t * TILE;\n"
+       "    const u32 n = (u32)min((u64)TILE, rows - base);\n"
+       "    __syncthreads();\n"
+       "    for (u32 j = 0; j < QUADS; j++) { const u32 w = threadIdx.x + j * %uu, i0 = 4u * w; const u32 v = i0 < n ? min(4u, n - i0) : 0u;\n"
+       "      s_one[w] = v == 4u ? 0x01010101u : (0x01010101u & ((1u << (8u * v)) - 1u)); }\n",
+       QE_GPU_WORKGROUP_SIZE);
+  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
+  {
+    const int t = slot_type[s];
+    if (!t) continue;
+    const int w = type_bytes(t);
+    int summed = 0;
+    for (uint32_t i = 0; i < sum_col_count; i++)
+      if (sum_cols[i] == s) summed = 1;
+    bput(&b, "    if ((need >> %d) & 1u)\n    {\n      %s x[QUADS * 4u];\n", s, w == 8 ? "u64" : "u32");
+    bput(&b, "#pragma unroll\n      for (u32 j = 0; j < QUADS; j++)\n      {\n        const u32 i0 = 4u * (threadIdx.x + j * %uu);\n", QE_GPU_WORKGROUP_SIZE);
+    if (w == 8)
+      bput(&b,
+           "        if (n == TILE) { const uint4 f = cql_ld4((const u64*)a.buf[%d] + base + i0), g = cql_ld4((const u64*)a.buf[%d] + base + i0 + 2u);\n"
+           "          x[4 * j] = ((u64)f.y << 32) | f.x; x[4 * j + 1] = ((u64)f.w << 32) | f.z; x[4 * j + 2] = ((u64)g.y << 32) | g.x; x[4 * j + 3] = ((u64)g.w << 32) | g.z; }\n"
+           "        else { for (u32 e = 0; e < 4u; e++) x[4 * j + e] = i0 + e < n ? ((const u64*)a.buf[%d])[base + i0 + e] : 0ull; }\n",
+           6 + s, 6 + s, 6 + s);
+    else if (w == 4)
+      bput(&b,
+           "        if (n == TILE) { const uint4 f = cql_ld4((const u32*)a.buf[%d] + base + i0); x[4 * j] = f.x; x[4 * j + 1] = f.y; x[4 * j + 2] = f.z; x[4 * j + 3] = f.w; }\n"
+           "        else { for (u32 e = 0; e < 4u; e++) x[4 * j + e] = i0 + e < n ? ((const u32*)a.buf[%d])[base + i0 + e] : 0u; }\n",
+           6 + s, 6 + s);
+    else
+      bput(&b, "        for (u32 e = 0; e < 4u; e++) x[4 * j + e] = i0 + e < n ? (u32)((const unsigned char*)a.buf[%d])[base + i0 + e] : 0u;\n", 6 + s);
+    bput(&b, "      }\n");
+    if (summed)
+    {
+      char expr[200];
+      if (t == CQLOPS_TYPE_F64) snprintf(expr, sizeof(expr), "(u64)__double_as_longlong(__fma_rn(__longlong_as_double((long long)x[i]), sc, __longlong_as_double((long long)%s)))", magic);
+      else if (t == CQLOPS_TYPE_F32) snprintf(expr, sizeof(expr), "(u64)__double_as_longlong(__fma_rn((double)__uint_as_float(x[i]), sc, __longlong_as_double((long long)%s)))", magic);
+      else if (t == CQLOPS_TYPE_I32)
+        snprintf(expr, sizeof(expr), "%s + (u64)(sh >= 0 ? (long long)(int)x[i] * (1ll << sh) : __double2ll_rn((double)(int)x[i] * sc))", magic);
+      else if (t == CQLOPS_TYPE_U64) snprintf(expr, sizeof(expr), "%s + (u64)__double2ll_rn((double)x[i] * sc)", magic);
+      else if (t == CQLOPS_TYPE_I64) snprintf(expr, sizeof(expr), "%s + (u64)__double2ll_rn(cql_i64d(x[i]) * sc)", magic);
+      else snprintf(expr, sizeof(expr), "%s + (u64)(sh >= 0 ? (long long)((u64)x[i] << sh) : __double2ll_rn((double)x[i] * sc))", magic);
+      bput(&b,
+           "      if ((need_sum >> %d) & 1u)\n      {\n        const double sc = col_scale[%d]; const int sh = (int)col_shift[%d]; (void)sc; (void)sh;\n"
+           "#pragma unroll\n        for (u32 j = 0; j < QUADS; j++)\n        {\n"
+           "          const u32 w = threadIdx.x + j * %uu; u32 lo[4], hi[4], p0, p1, p2, p3;\n"
+           "          for (u32 e = 0; e < 4u; e++) { const u32 i = 4 * j + e; const u64 f = %s; lo[e] = (u32)f; hi[e] = (u32)(f >> 32); bad |= hi[e] ^ (u32)(%s >> 32); }\n"
+           "          if (n != TILE) { for (u32 e = 0; e < 4u; e++) if (4u * w + e >= n) { lo[e] = 0u; hi[e] = 0u; } }\n"
+           "          cql_planes(lo[0], lo[1], lo[2], lo[3], p0, p1, p2, p3);\n"
+           "          s_pl%d[w] = p0; s_pl%d[WORDS + w] = p1; s_pl%d[2u * WORDS + w] = p2; s_pl%d[3u * WORDS + w] = p3;\n"
+           "          cql_planes(hi[0], hi[1], hi[2], hi[3], p0, p1, p2, p3);\n"
+           "          s_pl%d[4u * WORDS + w] = p0; s_pl%d[5u * WORDS + w] = p1;%s",
+           s, s, s, QE_GPU_WORKGROUP_SIZE, expr, magic, s, s, s, s, s, s, L.planes == 7u ? "" : "\n");
+      if (L.planes == 7u) bput(&b, " s_pl%d[6u * WORDS + w] = p2;\n", s);
+      bput(&b, "        }\n      }\n");
+    }
+    /* 64-bit integers have no comparisons in a batch, only sums */
+    if (t == CQLOPS_TYPE_U64 || t == CQLOPS_TYPE_I64)
+    {
+      bput(&b, "    }\n");
+      continue;
+    }
+    const char* key = "x[i]";
+    if (t == CQLOPS_TYPE_F64) key = "cql_key(x[i])";
+    else if (t == CQLOPS_TYPE_F32) key = "((x[i] >> 31) ? ~x[i] : (x[i] | 0x80000000u))";
+    else if (t == CQLOPS_TYPE_I32 || t == 9) key = "(x[i] ^ 0x80000000u)";
+    bput(&b,
+         "      u32 p[QUADS * 4u];\n"
+         "#pragma unroll\n      for (u32 i = 0; i < QUADS * 4u; i++) { x[i] = %s; p[i] = 0u; }\n"
+         "      for (u32 h = 1u << steps[%d]; h > 1u; )\n      {\n        h >>= 1;\n"
+         "#pragma unroll\n        for (u32 i = 0; i < QUADS * 4u; i++) if (x[i] >= s_cut%d[p[i] + h - 1u]) p[i] += h;\n      }\n"
+         "#pragma unroll\n      for (u32 j = 0; j < QUADS; j++)\n"
+         "        s_rk%d[threadIdx.x + j * %uu] = (p[4 * j] | (p[4 * j + 1] << 8) | (p[4 * j + 2] << 16) | (p[4 * j + 3] << 24)) | 0x80808080u;\n"
+         "    }\n",
+         key, s, s, s, QE_GPU_WORKGROUP_SIZE);
+  }
+  bput(&b,
+       "    __syncthreads();\n"
+       "#define __uint_as_float(x) (x)\n#define cql_bi cql_rk\n#define cql_bf cql_rk\n#define cql_bk cql_rk\n"
+       "    for (u32 it = warp; it < items; it += %uu)\n    {\n"
+       "      const u32 q = it / parts, st0 = (it - q * parts) * span;\n"
+       "      const RankThr* TH = thr + (u64)(q0 + q) * %uu;\n"
+       "      (void)TH;\n"
+       "      const u32 sc = qsum[q0 + q];\n"
+       "      const u32* pl = ",
+       QE_GPU_WORKGROUP_SIZE / 32u, BATCH_MAX_SITES);
+  for (uint32_t i = 0; i < sum_col_count; i++) bput(&b, "sc == %du ? s_pl%d : ", sum_cols[i], sum_cols[i]);
+  bput(&b, "(const u32*)0;\n      u32 cnt = 0u");
+  for (uint32_t p = 0; p < L.planes; p++) bput(&b, ", a%u = 0u", p);
+  bput(&b, ";\n      switch (s_shape[q])\n      {\n");
+  for (uint32_t s = 0; s < shapes; s++)
+  {
+    bput(&b, "      case %uu:\n      {\n", s);
+    for (uint32_t i = 0; i < shape_sites[s] && i < BATCH_MAX_SITES; i++) bput(&b, "        const RankThr T%u = TH[%u];\n", i, i);
+    bput(&b, "        for (u32 st = st0; st < st0 + span; st++)\n        {\n          const u32 o = st * 128u + lane * 4u;\n");
+    for (int c = 0; c < CQLOPS_MAX_BINDINGS; c++)
+    {
+      char name[16];
+      snprintf(name, sizeof(name), slot_type[c] == CQLOPS_TYPE_F64 ? "kd%d[k]" : "r%d[k]", c);
+      if (!slot_type[c] || !strstr(shape_exprs[s], name)) continue;
+      snprintf(name, sizeof(name), slot_type[c] == CQLOPS_TYPE_F64 ? "kd%d" : "r%d", c);
+      bput(&b, "          const uint4 R%d = *(const uint4*)(s_rk%d + o); const Rk %s[4] = { { R%d.x }, { R%d.y }, { R%d.z }, { R%d.w } };\n", c, c, name, c, c, c,
+           c);
+    }
+    bput(&b,
+         "          const uint4 one = *(const uint4*)(s_one + o);\n"
+         "          const u32 m0 = (CQL_SHAPE_%u(0)).m & 0x80808080u, m1 = (CQL_SHAPE_%u(1)).m & 0x80808080u, m2 = (CQL_SHAPE_%u(2)).m & 0x80808080u, m3 = (CQL_SHAPE_%u(3)).m & 0x80808080u;\n"
+         "          cnt = __dp4a(m0, one.x, cnt); cnt = __dp4a(m1, one.y, cnt); cnt = __dp4a(m2, one.z, cnt); cnt = __dp4a(m3, one.w, cnt);\n"
+         "          if (pl)\n          {\n",
+         s, s, s, s);
+    for (uint32_t p = 0; p < L.planes; p++)
+      bput(&b,
+           "            { const uint4 v = *(const uint4*)(pl + %uu * WORDS + o); a%u = __dp4a(m0, v.x, a%u); a%u = __dp4a(m1, v.y, a%u); a%u = __dp4a(m2, v.z, a%u); a%u = __dp4a(m3, v.w, a%u); }\n",
+           p, p, p, p, p, p, p, p, p);
+    bput(&b, "          }\n        }\n        break;\n      }\n");
+  }
+  /* a match byte is 128, so every total carries a factor of 2^7 */
+  bput(&b, "      default: break;\n      }\n      cnt = __reduce_add_sync(0xffffffffu, cnt >> 7);\n      u64 v = 0ull;\n      if (pl)\n      {\n        v = (u64)(a0 >> 7)");
+  for (uint32_t p = 1; p < L.planes; p++) bput(&b, " + ((u64)a%u << %u)", p, 8u * p - 7u);
+  bput(&b,
+       ";\n        v = (u64)cql_wsum64((long long)v) - (u64)cnt * %s;\n      }\n"
+       "      if (lane == 0u && cnt) { atomicAdd(&s_cnt[q], cnt); if (v) atomicAdd(&s_sum[q], v); }\n"
+       "    }\n"
+       "  }\n"
+       "  const u32 any_bad = __syncthreads_or((bad >> %u) != 0u);\n"
+       "  for (u32 q = threadIdx.x; q < nq; q += %uu)\n  {\n"
+       "    const long long v = (long long)s_sum[q];\n"
+       "    const u64 at = (u64)blockIdx.x * nq + q;\n"
+       "    if (at < pcap) { partials[at * 3] = (u64)s_cnt[q] + (q == 0u && any_bad ? %lluull : 0ull); partials[at * 3 + 1] = (u64)v; partials[at * 3 + 2] = v < 0 ? ~0ull : 0ull; }\n"
+       "  }\n}\n",
+       bias, L.planes == 6u ? 16u : 20u, QE_GPU_WORKGROUP_SIZE, (unsigned long long)RANK_BAD);
+  if (b.failed)
+  {
+    free(b.p);
+    return NULL;
+  }
+  return b.p;
+}
+
+/* a threshold's interval [lo, hi] of its column's order keys; returns the inversion */
+static int rank_interval(const Thr* t, uint64_t* lo, uint64_t* hi)
+{
+  if (!(t->site & THR_F32))
+  {
+    *lo = t->a;
+    *hi = t->a + t->b;
+    return t->c != 0;
+  }
+  const uint32_t bits = (uint32_t)t->a, key = (bits >> 31) ? ~bits : (bits | 0x80000000u);
+  const uint64_t ninf = 0x007fffffull, pinf = 0xff800000ull;
+  const int zero = (bits << 1) == 0, nan = (bits << 1) > 0xff000000u;
+  const uint64_t first = zero ? 0x7fffffffull : key, last = zero ? 0x80000000ull : key;   /* the keys equal to the bound */
+  const uint32_t op = t->c;
+  int none = nan;
+  *lo = op == OP_CMP_LT || op == OP_CMP_LE ? ninf : (op == OP_CMP_GT && t->d ? last + 1 : first);
+  *hi = op == OP_CMP_GT || op == OP_CMP_GE ? pinf : (op == OP_CMP_LT && t->d ? first - 1 : last);
+  if (*lo > *hi) none = 1;
+  if (none)
+  {
+    /* nothing matches (or, with !=, everything): the full range, inverted */
+    *lo = 0;
+    *hi = 0xffffffffull;
+    return op != OP_CMP_NE;
+  }
+  return op == OP_CMP_NE;
+}
+
+static int cut_order(const void* x, const void* y)
+{
+  const uint64_t a = *(const uint64_t*)x, b = *(const uint64_t*)y;
+  return a < b ? -1 : a > b;
+}
+
+/* The cuts of a launch's thresholds and the thresholds as bounds of ranks; 0 when a column has more than
+   RANK_CUTS. A key is in [lo, hi] when its rank is at least lo's and below hi + 1's. */
+static int rank_thresholds(const Thr* thr, uint32_t queries, const int* slot_type, RankThr* out, unsigned char* cut_bytes)
+{
+  const uint64_t n = (uint64_t)queries * BATCH_MAX_SITES;
+  uint64_t* cuts = (uint64_t*)malloc((2 * n + 1) * sizeof(uint64_t));
+  uint64_t* table = (uint64_t*)cut_bytes;
+  uint32_t* steps = (uint32_t*)(cut_bytes + (uint64_t)CQLOPS_MAX_BINDINGS * RANK_TABLE * 8u);
+  int ok = cuts != NULL;
+  memset(out, 0, n * sizeof(RankThr));
+  memset(cut_bytes, 0, RANK_CUT_BYTES);
+  for (int c = 0; ok && c < CQLOPS_MAX_BINDINGS; c++)
+  {
+    if (!slot_type[c]) continue;
+    const uint64_t top = slot_type[c] == CQLOPS_TYPE_F64 ? ~0ull : 0xffffffffull;
+    uint64_t k = 0, lo, hi;
+    for (uint64_t i = 0; i < n; i++)
+    {
+      if ((thr[i].site & 0xffu) != (uint64_t)c + 1u) continue;
+      rank_interval(&thr[i], &lo, &hi);
+      if (lo > 0) cuts[k++] = lo;
+      if (hi < top) cuts[k++] = hi + 1;
+    }
+    qsort(cuts, k, sizeof(uint64_t), cut_order);
+    uint32_t u = 0;
+    for (uint64_t i = 0; i < k; i++)
+      if (u == 0 || cuts[u - 1] != cuts[i]) cuts[u++] = cuts[i];
+    if (u > RANK_CUTS)
+    {
+      ok = 0;
+      break;
+    }
+    while ((1u << steps[c]) <= u) steps[c]++;
+    for (uint32_t i = 0; i < RANK_TABLE; i++) table[(uint32_t)c * RANK_TABLE + i] = i < u ? cuts[i] : top;
+    for (uint64_t i = 0; i < n; i++)
+    {
+      if ((thr[i].site & 0xffu) != (uint64_t)c + 1u) continue;
+      const int inv = rank_interval(&thr[i], &lo, &hi);
+      uint32_t rl = 0, rh = 0;
+      while (rl < u && cuts[rl] <= lo) rl++;
+      if (hi < top) while (rh < u && cuts[rh] <= hi + 1) rh++;
+      else rh = 128;
+      out[i].lo = rl * 0x01010101u;
+      out[i].hi = rh == 128 ? 0x80808080u : rh * 0x01010101u;
+      out[i].inv = inv ? 0x80808080u : 0u;
+    }
+  }
+  free(cuts);
+  return ok;
+}
+
 /* ---- the cube form: group once, answer many ---- */
 
 /* Queries whose WHERE reads only whole-number columns of small range are answered from a dense table of
@@ -1277,6 +1660,14 @@ static char* launch_source(char** shape_exprs, const uint32_t* shape_sites, uint
   return batch_source(shape_exprs, shape_sites, shapes, slot_type, sum_cols, sum_col_count, rows_per_thread, block, persistent);
 }
 
+/* a launch's kernel found or compiled */
+static int kernel_ready(const char* src)
+{
+  char name[64];
+  snprintf(name, sizeof(name), "qk_batch_%016llx", (unsigned long long)fnv_str(src));
+  return cqlcuda_kernel_alloc(name, strlen(name)) || cqlcuda_kernel_alloc_from_image(name, strlen(name), src, strlen(src));
+}
+
 /* ---- the shape catalog ---- */
 
 struct CqlBatchCatalog
@@ -1460,6 +1851,8 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   /* the form: rows per thread in the low byte, the register form's block size / 256 in the next (1 or 2) */
   uint32_t block = ((rows_per_thread >> 8) & 0xffu) == 2u ? 512u : 256u;
   int persistent_source = mode == BATCH_SOURCE && ((rows_per_thread >> 16) & 1u);   /* the persistent form's source */
+  /* the default form, 8 rows a thread in CTAs of 256: its batches run as ranks where their predicates allow */
+  int ranks = (rows_per_thread & 0xffu) == 8u && block == 256u && !persistent_source && !(rows_per_thread & FORM_REGISTERS);
   rows_per_thread &= 0xffu;
   if (rows_per_thread != 0 && rows_per_thread != 4 && rows_per_thread != 8 && rows_per_thread != 16) rows_per_thread = 8;
   uint64_t rows = columns[0].rows;
@@ -1579,6 +1972,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
       if (t == CQLOPS_TYPE_F32) thr_f32(c, (int)sites[i].op, th);
       else if (t == CQLOPS_TYPE_F64) thr_f64(c, (int)sites[i].op, th);
       else thr_int(c, (int)sites[i].op, t == CQLOPS_TYPE_I32 || t == 9, th);
+      th->site = (sites[i].col_slot + 1u) | (t == CQLOPS_TYPE_F32 ? THR_F32 : 0u);
     }
     for (uint32_t i = 0; i < p->const_count; i++) qconst[(uint64_t)q * BATCH_MAX_CONSTS + i] = const_value(p, i);
     int32_t sc = sum_columns ? sum_columns[q] : -1;
@@ -1596,6 +1990,21 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   double col_scale[CQLOPS_MAX_BINDINGS] = { 0 };
   int64_t col_shift[CQLOPS_MAX_BINDINGS] = { 0 };
   uint32_t sum_mask = 0;
+  /* the rows one accumulator takes, the most any form takes: in the register form a warp's passes over
+     the grid (32 lanes x rows per thread each), in the tile and rank forms a CTA's tiles (at most one SM's
+     share of the rows and 2048, whatever the CTAs per SM). One bound for every form gives every form the
+     same scale, so a query's sum is the same integer whichever form (or the autotuner's choice) runs
+     it - and the cube form, which adds the same summands to 128-bit cell totals. */
+  const uint64_t per_pass = (uint64_t)(sm_count ? sm_count : 152) * BATCH_CTAS_PER_SM * QE_GPU_WORKGROUP_SIZE;
+  uint64_t warp_rows = rows / (sm_count ? sm_count : 152) + 2048;
+  for (uint32_t rpt = 4; rpt <= 16; rpt *= 2)
+  {
+    uint64_t groups = (rows + rpt - 1) / rpt;
+    uint64_t w = ((groups + per_pass - 1) / per_pass) * 32 * rpt;
+    if (w > warp_rows) warp_rows = w;
+  }
+  int wr = 0;
+  frexp((double)warp_rows, &wr);   /* warp_rows < 2^wr */
   for (uint32_t q = 0; ok && q < query_count; q++)
   {
     if (qsum[q] == 0xffffffffu) continue;
@@ -1612,21 +2021,6 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     double m = fabs(col->zone_min) > fabs(col->zone_max) ? fabs(col->zone_min) : fabs(col->zone_max);
     int e = 0;
     if (m > 0.0) frexp(m, &e);   /* m < 2^e */
-    /* the rows one accumulator takes, the most any form takes: in the register form a warp's passes over
-       the grid (32 lanes x rows per thread each), in the tile form a CTA's tiles (at most one SM's share
-       of the rows and two tiles, whatever the CTAs per SM). One bound for every form gives every form the
-       same scale, so a query's sum is the same integer whichever form (or the autotuner's choice) runs
-       it - and the cube form, which adds the same summands to 128-bit cell totals. */
-    uint64_t per_pass = (uint64_t)(sm_count ? sm_count : 152) * BATCH_CTAS_PER_SM * QE_GPU_WORKGROUP_SIZE;
-    uint64_t warp_rows = rows / (sm_count ? sm_count : 152) + 2048;
-    for (uint32_t rpt = 4; rpt <= 16; rpt *= 2)
-    {
-      uint64_t groups = (rows + rpt - 1) / rpt;
-      uint64_t w = ((groups + per_pass - 1) / per_pass) * 32 * rpt;
-      if (w > warp_rows) warp_rows = w;
-    }
-    int wr = 0;
-    frexp((double)warp_rows, &wr);   /* warp_rows < 2^wr */
     col_scale[c] = ldexp(1.0, 62 - e - wr);
     col_shift[c] = 62 - e - wr;
     sum_mask |= 1u << c;
@@ -1749,8 +2143,33 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     }
   uint64_t* folded = ok && mode == BATCH_RUN ? (uint64_t*)malloc((size_t)nalloc * 24) : NULL;
   ok = ok && (folded || mode != BATCH_RUN);
-  /* one launch per slice of at most CQL_BATCH_LAUNCH_QUERIES queries: its shapes (all of the catalog's,
-     with a catalog) and where each starts */
+  /* the rank form, where every predicate is comparisons with literals and the launches' cuts fit, in
+     launches of fewer queries if need be */
+  uint32_t launch_cap = CQL_BATCH_LAUNCH_QUERIES;
+  RankThr* rank_thr = NULL;
+  unsigned char* rank_cuts = NULL;
+  ranks = ranks && ok && scan_n >= RANK_MIN_QUERIES && (mode == BATCH_RUN || mode == BATCH_PREPARE || mode == BATCH_SOURCE);
+  for (uint32_t sh = 0; ranks && sh < launch_shapes; sh++) ranks = rank_expr(launch_exprs[sh]);
+  for (uint32_t c = 0; ranks && mode == BATCH_RUN && c < column_count; c++)
+    ranks = !(((uint64_t)(uintptr_t)cqlcuda_buffer_device_pointer(columns[c].buffer)) & 15u);
+  if (ranks)
+  {
+    rank_thr = (RankThr*)malloc((size_t)scan_n * BATCH_MAX_SITES * sizeof(RankThr));
+    rank_cuts = (unsigned char*)malloc((size_t)(scan_n / RANK_MIN_LAUNCH + 1) * RANK_CUT_BYTES);
+    int fits = 0;
+    launch_cap = RANK_QUERIES;
+    for (; rank_thr && rank_cuts && !fits && launch_cap >= RANK_MIN_LAUNCH; launch_cap /= fits ? 1 : 2)
+    {
+      fits = 1;
+      for (uint32_t first = 0; fits && first < scan_n; first += launch_cap)
+        fits = rank_thresholds(thr_o + (uint64_t)first * BATCH_MAX_SITES, scan_n - first < launch_cap ? scan_n - first : launch_cap, launch_types,
+                               rank_thr + (uint64_t)first * BATCH_MAX_SITES, rank_cuts + (uint64_t)(first / launch_cap) * RANK_CUT_BYTES);
+    }
+    ranks = fits;
+    if (!fits) launch_cap = CQL_BATCH_LAUNCH_QUERIES;
+  }
+  /* one launch per slice of at most launch_cap queries: its shapes (all of the catalog's, with a catalog)
+     and where each starts */
   uint32_t begin[BATCH_MAX_SHAPES + 1];
   char* slice_exprs[BATCH_MAX_SHAPES];
   uint32_t slice_sites[BATCH_MAX_SHAPES];
@@ -1839,10 +2258,11 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   }
   if (ok && (mode == BATCH_SOURCE || mode == BATCH_PREPARE) && (scan_n || view))
   {
-    uint32_t nq = scan_n < CQL_BATCH_LAUNCH_QUERIES ? scan_n : CQL_BATCH_LAUNCH_QUERIES;
+    uint32_t nq = scan_n < launch_cap ? scan_n : launch_cap;
     uint32_t ns;
     SLICE_SHAPES(0, nq, ns);
-    char* src = launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, persistent_source);
+    char* src = ranks ? batch_source_ranks(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, wr)
+                      : launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, persistent_source);
     ok = src != NULL;
     if (ok && mode == BATCH_SOURCE)
     {
@@ -1851,14 +2271,15 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
       if (src_out && src_cap) snprintf(src_out, src_cap, "%s", src);
       if (src_out && n + 1 > src_cap) ok = 0;
     }
-    else if (ok)
-    {
-      char name[64];
-      snprintf(name, sizeof(name), "qk_batch_%016llx", (unsigned long long)fnv_str(src));
-      size_t nlen = strlen(name);
-      ok = cqlcuda_kernel_alloc(name, nlen) || cqlcuda_kernel_alloc_from_image(name, nlen, src, strlen(src));
-    }
+    else if (ok) ok = kernel_ready(src);
     free(src);
+    if (ok && mode == BATCH_PREPARE && ranks && view)
+    {
+      /* a batch of the catalog's shapes whose cuts do not fit takes the register form */
+      src = launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, 0);
+      ok = src && kernel_ready(src);
+      free(src);
+    }
   }
   if (ok && (mode == BATCH_SOURCE || mode == BATCH_PREPARE) && out_shapes) *out_shapes = shapes;
   if (mode == BATCH_PERSIST)
@@ -1879,15 +2300,16 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   int launch = ok && mode == BATCH_RUN;
   /* one upload of every launch parameter: the scales (doubles at 0..), then their exponents (64-bit
      integers at 16..), the scan's thresholds, literals and summed columns in shape order, each slice's shape
-     starts, then the cube queries' thresholds, literals and (shape, cube, summed column); each part on a
+     starts, the rank form's cuts per slice, then the cube queries' thresholds, literals and (shape, cube, summed column); each part on a
      16-byte boundary */
-  uint32_t slices = (scan_n + CQL_BATCH_LAUNCH_QUERIES - 1) / CQL_BATCH_LAUNCH_QUERIES;
+  uint32_t slices = (scan_n + launch_cap - 1) / launch_cap;
   const uint64_t off_thr = 256;
   const uint64_t off_qc = off_thr + (uint64_t)scan_n * BATCH_MAX_SITES * sizeof(Thr);
   const uint64_t off_qs = off_qc + (uint64_t)scan_n * BATCH_MAX_CONSTS * 8;
   const uint64_t off_begin = off_qs + (((uint64_t)scan_n * 4 + 15) & ~15ull);
   const uint64_t begin_stride = ((BATCH_MAX_SHAPES + 1) * 4 + 15) & ~15ull;
-  const uint64_t off_cthr = off_begin + (uint64_t)slices * begin_stride;
+  const uint64_t off_cuts = off_begin + (uint64_t)slices * begin_stride;
+  const uint64_t off_cthr = off_cuts + (ranks ? (uint64_t)slices * RANK_CUT_BYTES : 0);
   const uint64_t off_cqc = off_cthr + (uint64_t)cube_n * BATCH_MAX_SITES * sizeof(Thr);
   const uint64_t off_cmeta = off_cqc + (uint64_t)cube_n * BATCH_MAX_CONSTS * 8;
   const uint64_t param_bytes = off_cmeta + (((uint64_t)cube_n * 4 + 15) & ~15ull) + 16;
@@ -1897,7 +2319,13 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   {
     memcpy(params, col_scale, sizeof(col_scale));
     memcpy(params + 128, col_shift, sizeof(col_shift));
-    memcpy(params + off_thr, thr_o, (size_t)scan_n * BATCH_MAX_SITES * sizeof(Thr));
+    if (ranks)
+    {
+      memcpy(params + off_thr, rank_thr, (size_t)scan_n * BATCH_MAX_SITES * sizeof(RankThr));
+      memcpy(params + off_cuts, rank_cuts, (size_t)slices * RANK_CUT_BYTES);
+    }
+    else
+      memcpy(params + off_thr, thr_o, (size_t)scan_n * BATCH_MAX_SITES * sizeof(Thr));
     memcpy(params + off_qc, qc_o, (size_t)scan_n * BATCH_MAX_CONSTS * 8);
     memcpy(params + off_qs, qs_o, (size_t)scan_n * 4);
     for (uint32_t i = 0; i < cube_n; i++)
@@ -1912,9 +2340,10 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
       memcpy(params + off_cmeta + (uint64_t)i * 4, &meta, 4);
     }
   }
-  uint32_t per_sm = rows_per_thread ? register_ctas_per_sm(block) : tiled_layout(launch_types, sum_col_count).per_sm;
+  uint32_t per_sm = ranks ? rank_layout(launch_types, sum_col_count, wr).per_sm
+                          : (rows_per_thread ? register_ctas_per_sm(block) : tiled_layout(launch_types, sum_col_count).per_sm);
   uint64_t ctas = (uint64_t)(sm_count ? sm_count : 152) * per_sm;
-  uint32_t widest = scan_n < CQL_BATCH_LAUNCH_QUERIES ? scan_n : CQL_BATCH_LAUNCH_QUERIES;
+  uint32_t widest = scan_n < launch_cap ? scan_n : launch_cap;
   const uint64_t cube_out_bytes = 16 + (uint64_t)cube_n * 24;   /* the error word, then (count, lo, hi) per cube query */
   uint64_t* cube_out = launch && cube_n ? (uint64_t*)malloc(cube_out_bytes) : NULL;
   if (launch && cube_n && !cube_out) ok = 0;
@@ -1934,8 +2363,8 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   CqlKernel* shared_k = NULL;
   for (uint32_t sl = 0; launch && ok && sl < slices; sl++)
   {
-    uint32_t first = sl * CQL_BATCH_LAUNCH_QUERIES;
-    uint32_t nq = scan_n - first < CQL_BATCH_LAUNCH_QUERIES ? scan_n - first : CQL_BATCH_LAUNCH_QUERIES;
+    uint32_t first = sl * launch_cap;
+    uint32_t nq = scan_n - first < launch_cap ? scan_n - first : launch_cap;
     uint32_t ns;
     SLICE_SHAPES(first, nq, ns);
     memcpy(params + off_begin + sl * begin_stride, begin, (ns + 1) * 4);
@@ -1943,7 +2372,8 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     CqlKernel* k = shared_k;
     if (!k)
     {
-      char* src = launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, 0);
+      char* src = ranks ? batch_source_ranks(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, wr)
+                        : launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, 0);
       if (!src)
       {
         ok = 0;
@@ -2003,12 +2433,13 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     }
     for (uint32_t sl = 0; sl < slices; sl++)
     {
-      uint32_t first = sl * CQL_BATCH_LAUNCH_QUERIES;
-      uint32_t nq = scan_n - first < CQL_BATCH_LAUNCH_QUERIES ? scan_n - first : CQL_BATCH_LAUNCH_QUERIES;
+      uint32_t first = sl * launch_cap;
+      uint32_t nq = scan_n - first < launch_cap ? scan_n - first : launch_cap;
       CqlKernel* k = kernels[sl];
       cqlcuda_kernel_set_arg_buffer_range(k, 0, param_buf, 0, 256);
       cqlcuda_kernel_set_arg_buffer_range(k, 1, param_buf, off_thr, off_qc - off_thr);
-      cqlcuda_kernel_set_arg_buffer_range(k, 2, param_buf, off_qc, off_qs - off_qc);
+      if (ranks) cqlcuda_kernel_set_arg_buffer_range(k, 2, param_buf, off_cuts + (uint64_t)sl * RANK_CUT_BYTES, RANK_CUT_BYTES);
+      else cqlcuda_kernel_set_arg_buffer_range(k, 2, param_buf, off_qc, off_qs - off_qc);
       cqlcuda_kernel_set_arg_buffer_range(k, 3, param_buf, off_qs, (uint64_t)scan_n * 4);
       cqlcuda_kernel_set_arg_buffer_range(k, 4, param_buf, off_begin + sl * begin_stride, (slice_ns[sl] + 1) * 4);
       cqlcuda_kernel_set_arg_buffer_range(k, 5, parts, 0, ctas * nq * 24);
@@ -2033,7 +2464,14 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   free(params);
   free(kernels);
   free(slice_ns);
-  if (launch && ok)
+  /* a summand outside the rank form's planes (a value outside its column's stated range): the batch runs
+     again in the register form */
+  int again = 0;
+  for (uint32_t first = 0; ranks && launch && ok && first < scan_n; first += launch_cap) again |= folded[first * 3] >= RANK_BAD;
+  if (again)
+    ok = batch_run(catalog, programs, query_count, columns, column_count, sum_columns, rows_per_thread | FORM_REGISTERS, out_counts, out_sums,
+                   out_shapes, BATCH_RUN, NULL, 0, NULL, allow_cubes);
+  else if (launch && ok)
   {
     for (uint32_t i = 0; i < scan_n + cube_n; i++)
     {
@@ -2117,6 +2555,8 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   free(thr_o);
   free(qc_o);
   free(qs_o);
+  free(rank_thr);
+  free(rank_cuts);
   free(folded);
   return ok;
 }

@@ -199,7 +199,7 @@ static char* column_vs_const(Gen* g, const Val* col, const Val* k, int op)
     bs->const_index = (uint32_t)k->const_index;
     bs->op = (uint32_t)op;
     bs->col_type = (uint32_t)t;
-    bs->pad = 0;
+    bs->col_slot = (uint32_t)col->col_slot;
     if (t == CQLOPS_TYPE_U32 || t == 12 || t == CQLOPS_TYPE_BOOL) return dupf("cql_bi(&T%d, r%d[k])", site, col->col_slot);
     if (t == CQLOPS_TYPE_I32 || t == 9) return dupf("cql_bi(&T%d, r%d[k] ^ 0x80000000u)", site, col->col_slot);
     if (t == CQLOPS_TYPE_F32) return dupf("cql_bf(&T%d, __uint_as_float(r%d[k]))", site, col->col_slot);

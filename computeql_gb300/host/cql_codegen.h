@@ -13,7 +13,7 @@
    constant pool, the comparison opcode and the column type; the thresholds are worked out per query */
 typedef struct
 {
-  uint32_t const_index, op, col_type, pad;
+  uint32_t const_index, op, col_type, col_slot;
 } CqlBatchSite;
 
 /* The program as one boolean expression over raw row k of the column registers r<slot>[k], its
