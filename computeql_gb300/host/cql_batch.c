@@ -843,7 +843,7 @@ static char* batch_source_tiled(char** shape_exprs, const uint32_t* shape_sites,
 #define RANK_CUTS 127u
 #define RANK_TABLE (RANK_CUTS + 1u)                                     /* a column's cuts, padded to a power of two */
 #define RANK_CUT_BYTES (CQLOPS_MAX_BINDINGS * RANK_TABLE * 8u + 64u)    /* a launch's cuts, then each column's search steps */
-#define RANK_QUERIES 192u       /* a launch's queries: its accumulators leave room for three CTAs an SM */
+#define RANK_QUERIES 160u       /* a launch's queries: its accumulators leave room for three CTAs an SM */
 #define RANK_MIN_LAUNCH 48u     /* launches are halved down to this many while their cuts do not fit */
 #define RANK_MIN_QUERIES 2u
 #define FORM_REGISTERS (1u << 24)   /* with a form: not as ranks */
@@ -897,7 +897,7 @@ static RankLayout rank_layout(const int* slot_type, uint32_t sum_col_count, int 
       cuts += RANK_TABLE * (slot_type[s] == CQLOPS_TYPE_F64 ? 8u : 4u);
     }
   l.planes = warp_row_bits >= 16 ? 6u : 7u;
-  const uint32_t fixed = RANK_QUERIES * 13u + cuts;   /* sums, counts and shapes per query */
+  const uint32_t fixed = RANK_QUERIES * 14u + cuts;   /* sums, counts, shapes and summed planes per query */
   const uint32_t row = slots + 1u + sum_col_count * l.planes;
   l.tile = row * 2048u + fixed <= 75u * 1024u ? 2048u : 1024u;
   l.smem = (row * l.tile + fixed + 15u) & ~15u;
@@ -908,6 +908,7 @@ static RankLayout rank_layout(const int* slot_type, uint32_t sum_col_count, int 
 
 static const char* RANK_PRELUDE =
   "struct RankThr { u32 lo, hi, inv, pad; };\n"
+  "__device__ __forceinline__ float cql_float(u32 bits) { return __uint_as_float(bits); }\n"
   "struct Rk { u32 v; };\n"
   "struct Mk { u32 m; };\n"
   "__device__ __forceinline__ Rk operator^(Rk a, u32) { return a; }\n"
@@ -919,7 +920,21 @@ static const char* RANK_PRELUDE =
   "{\n"
   "  const u32 x = __byte_perm(a, b, 0x5140), y = __byte_perm(c, d, 0x5140), z = __byte_perm(a, b, 0x7362), w = __byte_perm(c, d, 0x7362);\n"
   "  p0 = __byte_perm(x, y, 0x5410); p1 = __byte_perm(x, y, 0x7632); p2 = __byte_perm(z, w, 0x5410); p3 = __byte_perm(z, w, 0x7632);\n"
-  "}\n";
+  "}\n"
+  /* four consecutive rows from row i0 of a tile of n at base (whole tiles with 16-byte loads) */
+  "__device__ __forceinline__ void cql_rows(u64* x, const u64* c, u32 i0, u32 n, bool whole)\n"
+  "{\n"
+  "  if (whole) { const uint4 f = cql_ld4(c + i0), g = cql_ld4(c + i0 + 2u);\n"
+  "    x[0] = ((u64)f.y << 32) | f.x; x[1] = ((u64)f.w << 32) | f.z; x[2] = ((u64)g.y << 32) | g.x; x[3] = ((u64)g.w << 32) | g.z; }\n"
+  "  else { for (u32 e = 0; e < 4u; e++) x[e] = i0 + e < n ? c[i0 + e] : 0ull; }\n"
+  "}\n"
+  "__device__ __forceinline__ void cql_rows(u32* x, const u32* c, u32 i0, u32 n, bool whole)\n"
+  "{\n"
+  "  if (whole) { const uint4 f = cql_ld4(c + i0); x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w; }\n"
+  "  else { for (u32 e = 0; e < 4u; e++) x[e] = i0 + e < n ? c[i0 + e] : 0u; }\n"
+  "}\n"
+  "__device__ __forceinline__ void cql_rows(u32* x, const unsigned char* c, u32 i0, u32 n, bool)\n"
+  "{ for (u32 e = 0; e < 4u; e++) x[e] = i0 + e < n ? (u32)c[i0 + e] : 0u; }\n";
 
 static char* batch_source_ranks(char** shape_exprs, const uint32_t* shape_sites, uint32_t shapes, const int* slot_type, const int* sum_cols,
                                 uint32_t sum_col_count, int warp_row_bits)
@@ -954,128 +969,160 @@ static char* batch_source_ranks(char** shape_exprs, const uint32_t* shape_sites,
        "  u32* s_words = (u32*)s_mem;\n",
        QE_GPU_WORKGROUP_SIZE, L.per_sm, L.tile, words, quads, CQLOPS_MAX_BINDINGS * RANK_TABLE);
   /* shared memory: the words of every column's ranks, the ones, the planes, then sums, cuts, counts and shapes */
-  uint32_t at = 0;
+  uint32_t at = 0, place[CQLOPS_MAX_BINDINGS], cut_of[CQLOPS_MAX_BINDINGS], cuts64 = 0, cuts32 = 0;
   for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
-    if (slot_type[s]) bput(&b, "  u32* const s_rk%d = s_words + %uu;\n", s, at++ * words);
+    if (slot_type[s])
+    {
+      cut_of[s] = slot_type[s] == CQLOPS_TYPE_F64 ? cuts64++ : cuts32++;
+      place[s] = at;
+      bput(&b, "  u32* const s_rk%d = s_words + %uu;\n", s, at++ * words);
+    }
   bput(&b, "  u32* const s_one = s_words + %uu;\n", at++ * words);
-  for (uint32_t i = 0; i < sum_col_count; i++, at += L.planes) bput(&b, "  u32* const s_pl%d = s_words + %uu;\n", sum_cols[i], at * words);
-  bput(&b, "  u64* const s_sum = (u64*)(s_words + %uu);\n", at * words);
-  uint32_t off = 0;
-  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
-    if (slot_type[s] == CQLOPS_TYPE_F64) bput(&b, "  u64* const s_cut%d = s_sum + %uu;\n", s, RANK_QUERIES + off++ * RANK_TABLE);
-  bput(&b, "  u32* const s_cnt = (u32*)(s_sum + %uu);\n", RANK_QUERIES + off * RANK_TABLE);
-  off = 0;
-  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
-    if (slot_type[s] && slot_type[s] != CQLOPS_TYPE_F64) bput(&b, "  u32* const s_cut%d = s_cnt + %uu;\n", s, RANK_QUERIES + off++ * RANK_TABLE);
+  const uint32_t plane_words = at * words;
+  at += sum_col_count * L.planes;
+  bput(&b, "  u64* const s_sum = (u64*)(s_words + %uu); u64* const s_cut64 = s_sum + %uu;\n", at * words, RANK_QUERIES);
+  bput(&b, "  u32* const s_cnt = (u32*)(s_cut64 + %uu); u32* const s_cut32 = s_cnt + %uu;\n", cuts64 * RANK_TABLE, RANK_QUERIES);
   bput(&b,
        "  unsigned char* const s_shape = (unsigned char*)(s_cnt + %uu);\n"
        "  const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;\n"
-       "  for (u32 q = threadIdx.x; q < nq; q += %uu) { s_sum[q] = 0ull; s_cnt[q] = 0u; u32 s = 0u; while (s + 1u < %uu && q >= shape_begin[s + 1u]) s++; s_shape[q] = (unsigned char)s; }\n",
-       RANK_QUERIES + off * RANK_TABLE, QE_GPU_WORKGROUP_SIZE, shapes);
+       "  unsigned char* const s_plane = s_shape + %uu;   /* its summed column's place among the planes, 255: none */\n"
+       "  for (u32 q = threadIdx.x; q < nq; q += %uu)\n  {\n"
+       "    s_sum[q] = 0ull; s_cnt[q] = 0u; u32 s = 0u; while (s + 1u < %uu && q >= shape_begin[s + 1u]) s++; s_shape[q] = (unsigned char)s;\n"
+       "    const u32 sc = qsum[q0 + q]; (void)sc; s_plane[q] = ",
+       RANK_QUERIES + cuts32 * RANK_TABLE, RANK_QUERIES, QE_GPU_WORKGROUP_SIZE, shapes);
+  for (uint32_t i = 0; i < sum_col_count; i++) bput(&b, "sc == %du ? %u : ", sum_cols[i], i);
+  bput(&b, "255;\n  }\n");
   for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
     if (slot_type[s])
-      bput(&b, "  for (u32 i = threadIdx.x; i < %uu; i += %uu) s_cut%d[i] = (%s)cuts[%u + i];\n", RANK_TABLE, QE_GPU_WORKGROUP_SIZE, s,
-           slot_type[s] == CQLOPS_TYPE_F64 ? "u64" : "u32", (uint32_t)s * RANK_TABLE);
+      bput(&b, "  for (u32 i = threadIdx.x; i < %uu; i += %uu) s_cut%s[%uu + i] = (%s)cuts[%u + i];\n", RANK_TABLE, QE_GPU_WORKGROUP_SIZE,
+           slot_type[s] == CQLOPS_TYPE_F64 ? "64" : "32", cut_of[s] * RANK_TABLE, slot_type[s] == CQLOPS_TYPE_F64 ? "u64" : "u32", (uint32_t)s * RANK_TABLE);
   bput(&b,
        "  u32 bad = 0u;   /* bits that differ from the magic number's above the summand's field */\n"
        "  /* a query is also split over the tile's rows where there are too few queries to go round the warps */\n"
-       "  const u32 parts = nq >= 32u ? 1u : (nq >= 16u ? 2u : (WORDS / 128u < 4u ? 2u : 4u));\n"
-       "  const u32 items = nq * parts, span = WORDS / 128u / parts;\n"
+       "  const u32 split = nq >= 32u ? 0u : (nq >= 16u || WORDS / 128u < 4u ? 1u : 2u);\n"
+       "  const u32 items = nq << split, span = WORDS / 128u >> split;\n"
        "  const u64 tiles = (rows + TILE - 1ull) / TILE;\n"
        "  for (u64 t = blockIdx.x; t < tiles; t += gridDim.x)\n  {\n"
        "    const u64 base = t * TILE;\n"
        "    const u32 n = (u32)min((u64)TILE, rows - base);\n"
        "    __syncthreads();\n"
-       "    for (u32 j = 0; j < QUADS; j++) { const u32 w = threadIdx.x + j * %uu, i0 = 4u * w; const u32 v = i0 < n ? min(4u, n - i0) : 0u;\n"
-       "      s_one[w] = v == 4u ? 0x01010101u : (0x01010101u & ((1u << (8u * v)) - 1u)); }\n",
+       "    const bool whole = n == TILE;\n"
+       "    if (!whole) { for (u32 j = 0; j < QUADS; j++) { const u32 w = threadIdx.x + j * %uu, i0 = 4u * w; const u32 v = i0 < n ? min(4u, n - i0) : 0u;\n"
+       "      s_one[w] = v == 4u ? 0x80808080u : (0x80808080u & ((1u << (8u * v)) - 1u)); } }\n",
        QE_GPU_WORKGROUP_SIZE);
-  for (int s = 0; s < CQLOPS_MAX_BINDINGS; s++)
+  /* the columns of each type in a loop - the code of every column side by side would not stay in the
+     instruction cache with the queries' - with the next column's rows on their way while this one's are ranked */
+  int done[CQLOPS_MAX_BINDINGS] = { 0 };
+  for (int s0 = 0; s0 < CQLOPS_MAX_BINDINGS; s0++)
   {
-    const int t = slot_type[s];
-    if (!t) continue;
+    const int t = slot_type[s0];
+    if (!t || done[s0]) continue;
     const int w = type_bytes(t);
+    unsigned long long slot_list = 0, rank_list = 0, plane_list = 0, cut_list = 0;
+    uint32_t count = 0;
     int summed = 0;
-    for (uint32_t i = 0; i < sum_col_count; i++)
-      if (sum_cols[i] == s) summed = 1;
-    bput(&b, "    if ((need >> %d) & 1u)\n    {\n      %s x[QUADS * 4u];\n", s, w == 8 ? "u64" : "u32");
-    bput(&b, "#pragma unroll\n      for (u32 j = 0; j < QUADS; j++)\n      {\n        const u32 i0 = 4u * (threadIdx.x + j * %uu);\n", QE_GPU_WORKGROUP_SIZE);
-    if (w == 8)
+    for (int s = s0; s < CQLOPS_MAX_BINDINGS; s++)
+      if (slot_type[s] == t)
+      {
+        unsigned long long plane = 15;
+        for (uint32_t i = 0; i < sum_col_count; i++)
+          if (sum_cols[i] == s) plane = i;
+        summed |= plane != 15;
+        slot_list |= (unsigned long long)s << 4 * count;
+        rank_list |= (unsigned long long)place[s] << 4 * count;
+        cut_list |= (unsigned long long)cut_of[s] << 4 * count;
+        plane_list |= plane << 4 * count;
+        done[s] = 1;
+        count++;
+      }
+    const char* word = w == 8 ? "u64" : "u32";
+    const char* stored = w == 8 ? "u64" : (w == 1 ? "unsigned char" : "u32");
+    bput(&b, "    {\n      %s y[QUADS * 4u];\n", word);
+    for (int ahead = 0; ahead < 2; ahead++)
+    {
+      if (ahead)
+        bput(&b,
+             "#pragma unroll 1\n      for (u32 c = 0; c < %uu; c++)\n      {\n"
+             "        const u32 slot = (u32)(0x%llxull >> (4u * c)) & 15u;\n"
+             "        %s x[QUADS * 4u];\n#pragma unroll\n        for (u32 i = 0; i < QUADS * 4u; i++) x[i] = y[i];\n"
+             "        if (c + 1u < %uu)\n        ",
+             count, slot_list, word, count);
       bput(&b,
-           "        if (n == TILE) { const uint4 f = cql_ld4((const u64*)a.buf[%d] + base + i0), g = cql_ld4((const u64*)a.buf[%d] + base + i0 + 2u);\n"
-           "          x[4 * j] = ((u64)f.y << 32) | f.x; x[4 * j + 1] = ((u64)f.w << 32) | f.z; x[4 * j + 2] = ((u64)g.y << 32) | g.x; x[4 * j + 3] = ((u64)g.w << 32) | g.z; }\n"
-           "        else { for (u32 e = 0; e < 4u; e++) x[4 * j + e] = i0 + e < n ? ((const u64*)a.buf[%d])[base + i0 + e] : 0ull; }\n",
-           6 + s, 6 + s, 6 + s);
-    else if (w == 4)
-      bput(&b,
-           "        if (n == TILE) { const uint4 f = cql_ld4((const u32*)a.buf[%d] + base + i0); x[4 * j] = f.x; x[4 * j + 1] = f.y; x[4 * j + 2] = f.z; x[4 * j + 3] = f.w; }\n"
-           "        else { for (u32 e = 0; e < 4u; e++) x[4 * j + e] = i0 + e < n ? ((const u32*)a.buf[%d])[base + i0 + e] : 0u; }\n",
-           6 + s, 6 + s);
-    else
-      bput(&b, "        for (u32 e = 0; e < 4u; e++) x[4 * j + e] = i0 + e < n ? (u32)((const unsigned char*)a.buf[%d])[base + i0 + e] : 0u;\n", 6 + s);
-    bput(&b, "      }\n");
+           "      { const u32 to = (u32)(0x%llxull >> (4u * %s)) & 15u; const %s* const col = (const %s*)a.buf[6u + to] + base;\n"
+           "#pragma unroll\n        for (u32 j = 0; j < QUADS; j++) { if ((need >> to) & 1u) cql_rows(y + 4u * j, col, 4u * (threadIdx.x + j * %uu), n, whole); else { y[4u * j] = 0; y[4u * j + 1u] = 0; y[4u * j + 2u] = 0; y[4u * j + 3u] = 0; } } }\n",
+           slot_list, ahead ? "(c + 1u)" : "0u", stored, stored, QE_GPU_WORKGROUP_SIZE);
+    }
+    bput(&b, "        if (!((need >> slot) & 1u)) continue;\n");
     if (summed)
     {
       char expr[200];
       if (t == CQLOPS_TYPE_F64) snprintf(expr, sizeof(expr), "(u64)__double_as_longlong(__fma_rn(__longlong_as_double((long long)x[i]), sc, __longlong_as_double((long long)%s)))", magic);
-      else if (t == CQLOPS_TYPE_F32) snprintf(expr, sizeof(expr), "(u64)__double_as_longlong(__fma_rn((double)__uint_as_float(x[i]), sc, __longlong_as_double((long long)%s)))", magic);
+      else if (t == CQLOPS_TYPE_F32) snprintf(expr, sizeof(expr), "(u64)__double_as_longlong(__fma_rn((double)cql_float(x[i]), sc, __longlong_as_double((long long)%s)))", magic);
       else if (t == CQLOPS_TYPE_I32)
         snprintf(expr, sizeof(expr), "%s + (u64)(sh >= 0 ? (long long)(int)x[i] * (1ll << sh) : __double2ll_rn((double)(int)x[i] * sc))", magic);
       else if (t == CQLOPS_TYPE_U64) snprintf(expr, sizeof(expr), "%s + (u64)__double2ll_rn((double)x[i] * sc)", magic);
       else if (t == CQLOPS_TYPE_I64) snprintf(expr, sizeof(expr), "%s + (u64)__double2ll_rn(cql_i64d(x[i]) * sc)", magic);
       else snprintf(expr, sizeof(expr), "%s + (u64)(sh >= 0 ? (long long)((u64)x[i] << sh) : __double2ll_rn((double)x[i] * sc))", magic);
       bput(&b,
-           "      if ((need_sum >> %d) & 1u)\n      {\n        const double sc = col_scale[%d]; const int sh = (int)col_shift[%d]; (void)sc; (void)sh;\n"
-           "#pragma unroll\n        for (u32 j = 0; j < QUADS; j++)\n        {\n"
-           "          const u32 w = threadIdx.x + j * %uu; u32 lo[4], hi[4], p0, p1, p2, p3;\n"
-           "          for (u32 e = 0; e < 4u; e++) { const u32 i = 4 * j + e; const u64 f = %s; lo[e] = (u32)f; hi[e] = (u32)(f >> 32); bad |= hi[e] ^ (u32)(%s >> 32); }\n"
-           "          if (n != TILE) { for (u32 e = 0; e < 4u; e++) if (4u * w + e >= n) { lo[e] = 0u; hi[e] = 0u; } }\n"
-           "          cql_planes(lo[0], lo[1], lo[2], lo[3], p0, p1, p2, p3);\n"
-           "          s_pl%d[w] = p0; s_pl%d[WORDS + w] = p1; s_pl%d[2u * WORDS + w] = p2; s_pl%d[3u * WORDS + w] = p3;\n"
-           "          cql_planes(hi[0], hi[1], hi[2], hi[3], p0, p1, p2, p3);\n"
-           "          s_pl%d[4u * WORDS + w] = p0; s_pl%d[5u * WORDS + w] = p1;%s",
-           s, s, s, QE_GPU_WORKGROUP_SIZE, expr, magic, s, s, s, s, s, s, L.planes == 7u ? "" : "\n");
-      if (L.planes == 7u) bput(&b, " s_pl%d[6u * WORDS + w] = p2;\n", s);
-      bput(&b, "        }\n      }\n");
+           "        const u32 plane = (u32)(0x%llxull >> (4u * c)) & 15u;\n"
+           "        if (plane != 15u && ((need_sum >> slot) & 1u))\n        {\n"
+           "          const double sc = col_scale[slot]; const int sh = (int)col_shift[slot]; (void)sc; (void)sh;\n"
+           "          u32* const pl = s_words + %uu + plane * %uu + threadIdx.x;\n"
+           "#pragma unroll\n          for (u32 j = 0; j < QUADS; j++)\n          {\n"
+           "            u32 lo[4], hi[4], p0, p1, p2, p3; u32* const at = pl + j * %uu;\n"
+           "            for (u32 e = 0; e < 4u; e++) { const u32 i = 4 * j + e; const u64 f = %s; lo[e] = (u32)f; hi[e] = (u32)(f >> 32); bad |= hi[e] ^ (u32)(%s >> 32); }\n"
+           "            cql_planes(lo[0], lo[1], lo[2], lo[3], p0, p1, p2, p3);\n"
+           "            at[0] = p0; at[WORDS] = p1; at[2u * WORDS] = p2; at[3u * WORDS] = p3;\n"
+           "            cql_planes(hi[0], hi[1], hi[2], hi[3], p0, p1, p2, p3);\n"
+           "            at[4u * WORDS] = p0; at[5u * WORDS] = p1;%s\n          }\n        }\n",
+           plane_list, plane_words, L.planes * words, QE_GPU_WORKGROUP_SIZE, expr, magic, L.planes == 7u ? " at[6u * WORDS] = p2;" : "");
     }
     /* 64-bit integers have no comparisons in a batch, only sums */
-    if (t == CQLOPS_TYPE_U64 || t == CQLOPS_TYPE_I64)
+    if (t != CQLOPS_TYPE_U64 && t != CQLOPS_TYPE_I64)
     {
-      bput(&b, "    }\n");
-      continue;
+      const char* key = "x[i]";
+      if (t == CQLOPS_TYPE_F64) key = "cql_key(x[i])";
+      else if (t == CQLOPS_TYPE_F32) key = "((x[i] >> 31) ? ~x[i] : (x[i] | 0x80000000u))";
+      else if (t == CQLOPS_TYPE_I32 || t == 9) key = "(x[i] ^ 0x80000000u)";
+      bput(&b,
+           "        u32 p[QUADS * 4u];\n"
+           "        const char* const cut = (const char*)(s_cut%s + ((u32)(0x%llxull >> (4u * c)) & 15u) * %uu);\n"
+           "#pragma unroll\n        for (u32 i = 0; i < QUADS * 4u; i++) { x[i] = %s; p[i] = 0u; }\n"
+           "        const u32 depth = steps[slot];\n",
+           w == 8 ? "64" : "32", cut_list, RANK_TABLE, key);
+      /* a step's halves are compile-time offsets of byte positions: a load, a compare and an add a row */
+      for (uint32_t h = RANK_TABLE / 2u, d = 7; h; h >>= 1, d--)
+        bput(&b,
+             "        if (depth >= %uu)\n        {\n"
+             "#pragma unroll\n          for (u32 i = 0; i < QUADS * 4u; i++) if (x[i] >= *(const %s*)(cut + p[i] + %uu)) p[i] += %uu;\n        }\n",
+             d, word, (h - 1u) * (w == 8 ? 8u : 4u), h * (w == 8 ? 8u : 4u));
+      const uint32_t sh = w == 8 ? 3u : 2u;
+      bput(&b,
+           "        u32* const rk = s_words + ((u32)(0x%llxull >> (4u * c)) & 15u) * WORDS + threadIdx.x;\n"
+           "#pragma unroll\n        for (u32 j = 0; j < QUADS; j++)\n"
+           "          rk[j * %uu] = ((p[4 * j] >> %u) | (p[4 * j + 1] << %u) | (p[4 * j + 2] << %u) | (p[4 * j + 3] << %u)) | 0x80808080u;\n",
+           rank_list, QE_GPU_WORKGROUP_SIZE, sh, 8u - sh, 16u - sh, 24u - sh);
     }
-    const char* key = "x[i]";
-    if (t == CQLOPS_TYPE_F64) key = "cql_key(x[i])";
-    else if (t == CQLOPS_TYPE_F32) key = "((x[i] >> 31) ? ~x[i] : (x[i] | 0x80000000u))";
-    else if (t == CQLOPS_TYPE_I32 || t == 9) key = "(x[i] ^ 0x80000000u)";
-    bput(&b,
-         "      u32 p[QUADS * 4u];\n"
-         "#pragma unroll\n      for (u32 i = 0; i < QUADS * 4u; i++) { x[i] = %s; p[i] = 0u; }\n"
-         "      for (u32 h = 1u << steps[%d]; h > 1u; )\n      {\n        h >>= 1;\n"
-         "#pragma unroll\n        for (u32 i = 0; i < QUADS * 4u; i++) if (x[i] >= s_cut%d[p[i] + h - 1u]) p[i] += h;\n      }\n"
-         "#pragma unroll\n      for (u32 j = 0; j < QUADS; j++)\n"
-         "        s_rk%d[threadIdx.x + j * %uu] = (p[4 * j] | (p[4 * j + 1] << 8) | (p[4 * j + 2] << 16) | (p[4 * j + 3] << 24)) | 0x80808080u;\n"
-         "    }\n",
-         key, s, s, s, QE_GPU_WORKGROUP_SIZE);
+    bput(&b, "      }\n    }\n");
   }
   bput(&b,
        "    __syncthreads();\n"
        "#define __uint_as_float(x) (x)\n#define cql_bi cql_rk\n#define cql_bf cql_rk\n#define cql_bk cql_rk\n"
        "    for (u32 it = warp; it < items; it += %uu)\n    {\n"
-       "      const u32 q = it / parts, st0 = (it - q * parts) * span;\n"
+       "      const u32 q = it >> split, st0 = (it - (q << split)) * span;\n"
        "      const RankThr* TH = thr + (u64)(q0 + q) * %uu;\n"
        "      (void)TH;\n"
-       "      const u32 sc = qsum[q0 + q];\n"
-       "      const u32* pl = ",
-       QE_GPU_WORKGROUP_SIZE / 32u, BATCH_MAX_SITES);
-  for (uint32_t i = 0; i < sum_col_count; i++) bput(&b, "sc == %du ? s_pl%d : ", sum_cols[i], sum_cols[i]);
-  bput(&b, "(const u32*)0;\n      u32 cnt = 0u");
+       "      const u32 place = s_plane[q];\n"
+       "      const u32* const pl = place == 255u ? (const u32*)0 : s_words + %uu + place * %uu;\n"
+       "      u32 cnt = 0u",
+       QE_GPU_WORKGROUP_SIZE / 32u, BATCH_MAX_SITES, plane_words, L.planes * words);
   for (uint32_t p = 0; p < L.planes; p++) bput(&b, ", a%u = 0u", p);
   bput(&b, ";\n      switch (s_shape[q])\n      {\n");
   for (uint32_t s = 0; s < shapes; s++)
   {
     bput(&b, "      case %uu:\n      {\n", s);
     for (uint32_t i = 0; i < shape_sites[s] && i < BATCH_MAX_SITES; i++) bput(&b, "        const RankThr T%u = TH[%u];\n", i, i);
-    bput(&b, "        for (u32 st = st0; st < st0 + span; st++)\n        {\n          const u32 o = st * 128u + lane * 4u;\n");
+    bput(&b, "#pragma unroll 1\n        for (u32 st = st0; st < st0 + span; st++)\n        {\n          const u32 o = st * 128u + lane * 4u;\n");
     for (int c = 0; c < CQLOPS_MAX_BINDINGS; c++)
     {
       char name[16];
@@ -1086,9 +1133,9 @@ static char* batch_source_ranks(char** shape_exprs, const uint32_t* shape_sites,
            c);
     }
     bput(&b,
-         "          const uint4 one = *(const uint4*)(s_one + o);\n"
-         "          const u32 m0 = (CQL_SHAPE_%u(0)).m & 0x80808080u, m1 = (CQL_SHAPE_%u(1)).m & 0x80808080u, m2 = (CQL_SHAPE_%u(2)).m & 0x80808080u, m3 = (CQL_SHAPE_%u(3)).m & 0x80808080u;\n"
-         "          cnt = __dp4a(m0, one.x, cnt); cnt = __dp4a(m1, one.y, cnt); cnt = __dp4a(m2, one.z, cnt); cnt = __dp4a(m3, one.w, cnt);\n"
+         "          u32 m0 = (CQL_SHAPE_%u(0)).m & 0x80808080u, m1 = (CQL_SHAPE_%u(1)).m & 0x80808080u, m2 = (CQL_SHAPE_%u(2)).m & 0x80808080u, m3 = (CQL_SHAPE_%u(3)).m & 0x80808080u;\n"
+         "          if (!whole) { const uint4 one = *(const uint4*)(s_one + o); m0 &= one.x; m1 &= one.y; m2 &= one.z; m3 &= one.w; }\n"
+         "          cnt = __dp4a(m0, 0x01010101u, cnt); cnt = __dp4a(m1, 0x01010101u, cnt); cnt = __dp4a(m2, 0x01010101u, cnt); cnt = __dp4a(m3, 0x01010101u, cnt);\n"
          "          if (pl)\n          {\n",
          s, s, s, s);
     for (uint32_t p = 0; p < L.planes; p++)
@@ -1097,12 +1144,18 @@ static char* batch_source_ranks(char** shape_exprs, const uint32_t* shape_sites,
            p, p, p, p, p, p, p, p, p);
     bput(&b, "          }\n        }\n        break;\n      }\n");
   }
-  /* a match byte is 128, so every total carries a factor of 2^7 */
-  bput(&b, "      default: break;\n      }\n      cnt = __reduce_add_sync(0xffffffffu, cnt >> 7);\n      u64 v = 0ull;\n      if (pl)\n      {\n        v = (u64)(a0 >> 7)");
+  /* a match byte is 128, so every total carries a factor of 2^7. A lane's sum of up to 64 fields has 54 bits
+     (62 with 7 planes): the warp adds it in slices of 27 bits */
+  bput(&b, "      default: break;\n      }\n      cnt = __reduce_add_sync(0xffffffffu, cnt >> 7);\n      u64 v = 0ull;\n      if (pl)\n      {\n        const u64 l = (u64)(a0 >> 7)");
   for (uint32_t p = 1; p < L.planes; p++) bput(&b, " + ((u64)a%u << %u)", p, 8u * p - 7u);
   bput(&b,
-       ";\n        v = (u64)cql_wsum64((long long)v) - (u64)cnt * %s;\n      }\n"
-       "      if (lane == 0u && cnt) { atomicAdd(&s_cnt[q], cnt); if (v) atomicAdd(&s_sum[q], v); }\n"
+       ";\n"
+       "        v = (u64)__reduce_add_sync(0xffffffffu, (u32)l & 0x7ffffffu) + ((u64)__reduce_add_sync(0xffffffffu, (u32)(l >> 27) & 0x7ffffffu) << 27)%s - (u64)cnt * %s;\n"
+       "      }\n"
+       "      if (lane == 0u)\n      {\n"
+       "        if (split) { atomicAdd(&s_cnt[q], cnt); if (v) atomicAdd(&s_sum[q], v); }\n"
+       "        else { s_cnt[q] += cnt; s_sum[q] += v; }   /* one warp has the query in this tile */\n"
+       "      }\n"
        "    }\n"
        "  }\n"
        "  const u32 any_bad = __syncthreads_or((bad >> %u) != 0u);\n"
@@ -1111,7 +1164,7 @@ static char* batch_source_ranks(char** shape_exprs, const uint32_t* shape_sites,
        "    const u64 at = (u64)blockIdx.x * nq + q;\n"
        "    if (at < pcap) { partials[at * 3] = (u64)s_cnt[q] + (q == 0u && any_bad ? %lluull : 0ull); partials[at * 3 + 1] = (u64)v; partials[at * 3 + 2] = v < 0 ? ~0ull : 0ull; }\n"
        "  }\n}\n",
-       bias, L.planes == 6u ? 16u : 20u, QE_GPU_WORKGROUP_SIZE, (unsigned long long)RANK_BAD);
+       L.planes == 6u ? "" : " + ((u64)__reduce_add_sync(0xffffffffu, (u32)(l >> 54)) << 54)", bias, L.planes == 6u ? 16u : 20u, QE_GPU_WORKGROUP_SIZE, (unsigned long long)RANK_BAD);
   if (b.failed)
   {
     free(b.p);
