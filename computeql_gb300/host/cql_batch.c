@@ -834,9 +834,13 @@ static char* batch_source_tiled(char** shape_exprs, const uint32_t* shape_sites,
    with the plane. A warp takes one query over the tile, its lanes 16 rows a step, and adds the query's
    totals to the CTA's accumulators once per tile.
 
-   What bounds it is the integer pipe: the register form spends about 31 warp instructions per query and 32
-   rows (64-bit interval compares, mask assembly, predicated 64-bit adds, five reductions every 8 rows),
-   this one about 6, plus about 200 a row for the ranks and planes, whatever the number of queries.
+   The register form is bound by the integer pipe: about 31 warp instructions per query and 32 rows (64-bit
+   interval compares, mask assembly, predicated 64-bit adds, five reductions every 8 rows). This one spends
+   about 8, plus about 290 per 32 rows of 8 columns for the ranks and planes, and is bound by the shared
+   memory the queries read (80 % of its wavefronts). Over 50M rows of 4 u32 and 4 f64 columns: 64 queries
+   6.1 -> 1.76 ms, 8 queries 2.0 -> 0.86; over 300 thousand rows 166 -> 107 us and 92 -> 61. Two queries of one
+   column sharing a warp's reads were slower (1.9 to 3.2 ms): the registers they take, or their code in the
+   instruction cache, cost more than the reads.
 
    Ranks are at most RANK_CUTS (the cuts of a launch on one column), so a rank with bit 7 set minus a bound
    in [0, 128] keeps bit 7 exactly when it is at or above the bound, with no borrow between the bytes. */
@@ -845,7 +849,7 @@ static char* batch_source_tiled(char** shape_exprs, const uint32_t* shape_sites,
 #define RANK_CUT_BYTES (CQLOPS_MAX_BINDINGS * RANK_TABLE * 8u + 64u)    /* a launch's cuts, then each column's search steps */
 #define RANK_QUERIES 160u       /* a launch's queries: its accumulators leave room for three CTAs an SM */
 #define RANK_MIN_LAUNCH 48u     /* launches are halved down to this many while their cuts do not fit */
-#define RANK_MIN_QUERIES 2u
+#define RANK_MIN_QUERIES 2u     /* two queries: 54 -> 47 us over 300 thousand rows, 454 -> 346 over 50M; one: equal */
 #define FORM_REGISTERS (1u << 24)   /* with a form: not as ranks */
 #define RANK_BAD (1ull << 44)   /* added to the first query's count by a CTA that met a summand outside its planes */
 
@@ -860,32 +864,43 @@ typedef struct
   uint32_t tile, per_sm, smem, planes;
 } RankLayout;
 
+static const char* skip_text(const char* e, const char* text)
+{
+  const size_t n = strlen(text);
+  return e && !strncmp(e, text, n) ? e + n : NULL;
+}
+
+static const char* skip_number(const char* e)
+{
+  if (!e || *e < '0' || *e > '9') return NULL;
+  while (*e >= '0' && *e <= '9') e++;
+  return e;
+}
+
 /* whether a shape's predicate is comparisons of columns with literals joined by & and | alone */
 static int rank_expr(const char* e)
 {
+  static const char* const site[3][2] = { { "cql_bi(&T", ", r" }, { "cql_bf(&T", ", __uint_as_float(r" }, { "cql_bk(&T", ", kd" } };
   while (*e)
   {
-    unsigned slot, site;
-    int n = 0;
     if (*e == '(' || *e == ')' || *e == ' ' || *e == '&' || *e == '|')
     {
       e++;
       continue;
     }
-    if ((sscanf(e, "cql_bi(&T%u, r%u[k] ^ 0x80000000u)%n", &site, &slot, &n) == 2 && n) || (sscanf(e, "cql_bi(&T%u, r%u[k])%n", &site, &slot, &n) == 2 && n) ||
-        (sscanf(e, "cql_bf(&T%u, __uint_as_float(r%u[k]))%n", &site, &slot, &n) == 2 && n) ||
-        (sscanf(e, "cql_bk(&T%u, kd%u[k])%n", &site, &slot, &n) == 2 && n))
-    {
-      e += n;
-      continue;
-    }
-    return 0;
+    const char* next = NULL;
+    for (int k = 0; k < 3 && !next; k++)
+      next = skip_text(skip_number(skip_text(skip_number(skip_text(e, site[k][0])), site[k][1])), "[k]");
+    if (!next) return 0;
+    const char* biased = skip_text(next, " ^ 0x80000000u");   /* a signed column's code */
+    e = biased ? biased : next;
   }
   return 1;
 }
 
 /* the layout: byte planes of the summands (|summand| <= 2^(62 - bits of an accumulator's rows), so 6 bytes
-   from 2^15 rows on, else 7) and 2048 rows a tile where three CTAs then fit an SM, else 1024 */
+   from 2^15 rows on, else 7) and 2048 rows a tile where three CTAs then fit an SM, else 1024 (a query's totals cost a tile
+   the same: 1.85 ms with tiles of 1024 in four CTAs, 1.66 with 2048 in three) */
 static RankLayout rank_layout(const int* slot_type, uint32_t sum_col_count, int warp_row_bits)
 {
   RankLayout l;
@@ -902,7 +917,7 @@ static RankLayout rank_layout(const int* slot_type, uint32_t sum_col_count, int 
   l.tile = row * 2048u + fixed <= 75u * 1024u ? 2048u : 1024u;
   l.smem = (row * l.tile + fixed + 15u) & ~15u;
   uint32_t per_sm = (227u * 1024u) / (l.smem + 1024u);
-  l.per_sm = per_sm > 5 ? 5 : (per_sm < 1 ? 1 : per_sm);
+  l.per_sm = per_sm > 4 ? 4 : (per_sm < 1 ? 1 : per_sm);
   return l;
 }
 
@@ -937,9 +952,8 @@ static const char* RANK_PRELUDE =
   "{ for (u32 e = 0; e < 4u; e++) x[e] = i0 + e < n ? (u32)c[i0 + e] : 0u; }\n";
 
 static char* batch_source_ranks(char** shape_exprs, const uint32_t* shape_sites, uint32_t shapes, const int* slot_type, const int* sum_cols,
-                                uint32_t sum_col_count, int warp_row_bits)
+                                uint32_t sum_col_count, const RankLayout L)
 {
-  const RankLayout L = rank_layout(slot_type, sum_col_count, warp_row_bits);
   const uint32_t words = L.tile / 4u, quads = words / QE_GPU_WORKGROUP_SIZE;
   Buf b;
   memset(&b, 0, sizeof(b));
@@ -1201,6 +1215,19 @@ static int rank_interval(const Thr* t, uint64_t* lo, uint64_t* hi)
   return op == OP_CMP_NE;
 }
 
+/* the cuts at or below a key */
+static uint32_t cut_rank(const uint64_t* cuts, uint32_t n, uint64_t key)
+{
+  uint32_t lo = 0, hi = n;
+  while (lo < hi)
+  {
+    const uint32_t mid = (lo + hi) / 2;
+    if (cuts[mid] <= key) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
 static int cut_order(const void* x, const void* y)
 {
   const uint64_t a = *(const uint64_t*)x, b = *(const uint64_t*)y;
@@ -1213,20 +1240,26 @@ static int rank_thresholds(const Thr* thr, uint32_t queries, const int* slot_typ
 {
   const uint64_t n = (uint64_t)queries * BATCH_MAX_SITES;
   uint64_t* cuts = (uint64_t*)malloc((2 * n + 1) * sizeof(uint64_t));
+  uint32_t* list = (uint32_t*)malloc((n + 1) * sizeof(uint32_t));
   uint64_t* table = (uint64_t*)cut_bytes;
   uint32_t* steps = (uint32_t*)(cut_bytes + (uint64_t)CQLOPS_MAX_BINDINGS * RANK_TABLE * 8u);
-  int ok = cuts != NULL;
+  int ok = cuts && list;
   memset(out, 0, n * sizeof(RankThr));
   memset(cut_bytes, 0, RANK_CUT_BYTES);
+  /* the comparisons of all queries (a query's come first among its places) */
+  uint32_t sites = 0;
+  for (uint32_t q = 0; ok && q < queries; q++)
+    for (uint32_t i = q * BATCH_MAX_SITES; i < (q + 1) * BATCH_MAX_SITES && thr[i].site; i++) list[sites++] = i;
   for (int c = 0; ok && c < CQLOPS_MAX_BINDINGS; c++)
   {
     if (!slot_type[c]) continue;
     const uint64_t top = slot_type[c] == CQLOPS_TYPE_F64 ? ~0ull : 0xffffffffull;
     uint64_t k = 0, lo, hi;
-    for (uint64_t i = 0; i < n; i++)
+    for (uint32_t i = 0; i < sites; i++)
     {
-      if ((thr[i].site & 0xffu) != (uint64_t)c + 1u) continue;
-      rank_interval(&thr[i], &lo, &hi);
+      const Thr* t = &thr[list[i]];
+      if ((t->site & 0xffu) != (uint64_t)c + 1u) continue;
+      rank_interval(t, &lo, &hi);
       if (lo > 0) cuts[k++] = lo;
       if (hi < top) cuts[k++] = hi + 1;
     }
@@ -1241,21 +1274,47 @@ static int rank_thresholds(const Thr* thr, uint32_t queries, const int* slot_typ
     }
     while ((1u << steps[c]) <= u) steps[c]++;
     for (uint32_t i = 0; i < RANK_TABLE; i++) table[(uint32_t)c * RANK_TABLE + i] = i < u ? cuts[i] : top;
-    for (uint64_t i = 0; i < n; i++)
+    for (uint32_t i = 0; i < sites; i++)
     {
-      if ((thr[i].site & 0xffu) != (uint64_t)c + 1u) continue;
-      const int inv = rank_interval(&thr[i], &lo, &hi);
-      uint32_t rl = 0, rh = 0;
-      while (rl < u && cuts[rl] <= lo) rl++;
-      if (hi < top) while (rh < u && cuts[rh] <= hi + 1) rh++;
-      else rh = 128;
-      out[i].lo = rl * 0x01010101u;
-      out[i].hi = rh == 128 ? 0x80808080u : rh * 0x01010101u;
-      out[i].inv = inv ? 0x80808080u : 0u;
+      const Thr* t = &thr[list[i]];
+      if ((t->site & 0xffu) != (uint64_t)c + 1u) continue;
+      const int inv = rank_interval(t, &lo, &hi);
+      const uint32_t rl = lo > 0 ? cut_rank(cuts, u, lo) : 0u, rh = hi < top ? cut_rank(cuts, u, hi + 1) : 128u;
+      out[list[i]].lo = rl * 0x01010101u;
+      out[list[i]].hi = rh * 0x01010101u;
+      out[list[i]].inv = inv ? 0x80808080u : 0u;
     }
   }
   free(cuts);
+  free(list);
   return ok;
+}
+
+/* a rank form's kernel, found by what its source is made from - the source itself, some 40 KB, is written
+   only when the kernel has to be compiled */
+static CqlKernel* rank_kernel(char** shape_exprs, const uint32_t* shape_sites, uint32_t shapes, const int* slot_type, const int* sum_cols,
+                              uint32_t sum_col_count, const RankLayout L)
+{
+  uint64_t h = 1469598103934665603ull, g = 0;
+  uint32_t words[4 + 2 * CQLOPS_MAX_BINDINGS] = { L.tile, L.planes, L.per_sm, sum_col_count };
+  for (int c = 0; c < CQLOPS_MAX_BINDINGS; c++) words[4 + c] = (uint32_t)slot_type[c];
+  for (uint32_t i = 0; i < sum_col_count; i++) words[4 + CQLOPS_MAX_BINDINGS + i] = (uint32_t)sum_cols[i] + 1u;
+  for (uint32_t i = 0; i < sizeof(words) / 4; i++) h = (h ^ words[i]) * 1099511628211ull, g = g * 0x9e3779b97f4a7c15ull + words[i] + 1;
+  for (uint32_t s = 0; s < shapes; s++)
+  {
+    for (const char* e = shape_exprs[s]; *e; e++) h = (h ^ (unsigned char)*e) * 1099511628211ull, g = g * 0x9e3779b97f4a7c15ull + (unsigned char)*e;
+    h = (h ^ (0x100u + shape_sites[s])) * 1099511628211ull;
+    g = g * 0x9e3779b97f4a7c15ull + 0x100u + shape_sites[s];
+  }
+  char name[64];
+  snprintf(name, sizeof(name), "qk_batch_rank_%016llx%016llx", (unsigned long long)h, (unsigned long long)g);
+  const size_t n = strlen(name);
+  CqlKernel* k = cqlcuda_kernel_alloc(name, n);
+  if (k) return k;
+  char* src = batch_source_ranks(shape_exprs, shape_sites, shapes, slot_type, sum_cols, sum_col_count, L);
+  k = src ? cqlcuda_kernel_alloc_from_image(name, n, src, strlen(src)) : NULL;
+  free(src);
+  return k;
 }
 
 /* ---- the cube form: group once, answer many ---- */
@@ -1714,11 +1773,12 @@ static char* launch_source(char** shape_exprs, const uint32_t* shape_sites, uint
 }
 
 /* a launch's kernel found or compiled */
-static int kernel_ready(const char* src)
+static CqlKernel* kernel_ready(const char* src)
 {
   char name[64];
   snprintf(name, sizeof(name), "qk_batch_%016llx", (unsigned long long)fnv_str(src));
-  return cqlcuda_kernel_alloc(name, strlen(name)) || cqlcuda_kernel_alloc_from_image(name, strlen(name), src, strlen(src));
+  CqlKernel* k = cqlcuda_kernel_alloc(name, strlen(name));
+  return k ? k : cqlcuda_kernel_alloc_from_image(name, strlen(name), src, strlen(src));
 }
 
 /* ---- the shape catalog ---- */
@@ -2199,6 +2259,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   /* the rank form, where every predicate is comparisons with literals and the launches' cuts fit, in
      launches of fewer queries if need be */
   uint32_t launch_cap = CQL_BATCH_LAUNCH_QUERIES;
+  const RankLayout rank_form = rank_layout(launch_types, sum_col_count, wr);
   RankThr* rank_thr = NULL;
   unsigned char* rank_cuts = NULL;
   ranks = ranks && ok && scan_n >= RANK_MIN_QUERIES && (mode == BATCH_RUN || mode == BATCH_PREPARE || mode == BATCH_SOURCE);
@@ -2314,7 +2375,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     uint32_t nq = scan_n < launch_cap ? scan_n : launch_cap;
     uint32_t ns;
     SLICE_SHAPES(0, nq, ns);
-    char* src = ranks ? batch_source_ranks(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, wr)
+    char* src = ranks ? batch_source_ranks(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rank_form)
                       : launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, persistent_source);
     ok = src != NULL;
     if (ok && mode == BATCH_SOURCE)
@@ -2324,13 +2385,13 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
       if (src_out && src_cap) snprintf(src_out, src_cap, "%s", src);
       if (src_out && n + 1 > src_cap) ok = 0;
     }
-    else if (ok) ok = kernel_ready(src);
+    else if (ok) ok = ranks ? rank_kernel(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rank_form) != NULL : kernel_ready(src) != NULL;
     free(src);
     if (ok && mode == BATCH_PREPARE && ranks && view)
     {
       /* a batch of the catalog's shapes whose cuts do not fit takes the register form */
       src = launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, 0);
-      ok = src && kernel_ready(src);
+      ok = src && kernel_ready(src) != NULL;
       free(src);
     }
   }
@@ -2357,8 +2418,8 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
      16-byte boundary */
   uint32_t slices = (scan_n + launch_cap - 1) / launch_cap;
   const uint64_t off_thr = 256;
-  const uint64_t off_qc = off_thr + (uint64_t)scan_n * BATCH_MAX_SITES * sizeof(Thr);
-  const uint64_t off_qs = off_qc + (uint64_t)scan_n * BATCH_MAX_CONSTS * 8;
+  const uint64_t off_qc = off_thr + (uint64_t)scan_n * BATCH_MAX_SITES * (ranks ? sizeof(RankThr) : sizeof(Thr));
+  const uint64_t off_qs = off_qc + (ranks ? 0 : (uint64_t)scan_n * BATCH_MAX_CONSTS * 8);
   const uint64_t off_begin = off_qs + (((uint64_t)scan_n * 4 + 15) & ~15ull);
   const uint64_t begin_stride = ((BATCH_MAX_SHAPES + 1) * 4 + 15) & ~15ull;
   const uint64_t off_cuts = off_begin + (uint64_t)slices * begin_stride;
@@ -2379,7 +2440,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     }
     else
       memcpy(params + off_thr, thr_o, (size_t)scan_n * BATCH_MAX_SITES * sizeof(Thr));
-    memcpy(params + off_qc, qc_o, (size_t)scan_n * BATCH_MAX_CONSTS * 8);
+    if (!ranks) memcpy(params + off_qc, qc_o, (size_t)scan_n * BATCH_MAX_CONSTS * 8);
     memcpy(params + off_qs, qs_o, (size_t)scan_n * 4);
     for (uint32_t i = 0; i < cube_n; i++)
     {
@@ -2393,7 +2454,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
       memcpy(params + off_cmeta + (uint64_t)i * 4, &meta, 4);
     }
   }
-  uint32_t per_sm = ranks ? rank_layout(launch_types, sum_col_count, wr).per_sm
+  uint32_t per_sm = ranks ? rank_form.per_sm
                           : (rows_per_thread ? register_ctas_per_sm(block) : tiled_layout(launch_types, sum_col_count).per_sm);
   uint64_t ctas = (uint64_t)(sm_count ? sm_count : 152) * per_sm;
   uint32_t widest = scan_n < launch_cap ? scan_n : launch_cap;
@@ -2425,19 +2486,13 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     CqlKernel* k = shared_k;
     if (!k)
     {
-      char* src = ranks ? batch_source_ranks(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, wr)
-                        : launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, 0);
-      if (!src)
+      if (ranks) k = rank_kernel(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rank_form);
+      else
       {
-        ok = 0;
-        break;
+        char* src = launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, 0);
+        k = src ? kernel_ready(src) : NULL;
+        free(src);
       }
-      char name[64];
-      snprintf(name, sizeof(name), "qk_batch_%016llx", (unsigned long long)fnv_str(src));
-      size_t nlen = strlen(name);
-      k = cqlcuda_kernel_alloc(name, nlen);
-      if (!k) k = cqlcuda_kernel_alloc_from_image(name, nlen, src, strlen(src));
-      free(src);
       if (!k)
       {
         ok = 0;
