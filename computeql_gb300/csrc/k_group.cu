@@ -160,7 +160,7 @@ static int launch_hll_rows(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaS
 // reductions; f64 reductions would cost one but round per row.
 //
 // What it replaced, per 10M rows: member lists (assign 640 us, scatter 575, reduce 460, prefix sums and ranges 100)
-// for 1000 groups of two keys, this form 187. For 1M groups of one key, assign 337, scatter 143, reduce 122, ranges,
+// for 1000 groups of two keys, this form 164 (187 while the types were tested for every row). For 1M groups of one key, assign 337, scatter 143, reduce 122, ranges,
 // sums and compaction 230, this form 295 with the listing of the groups.
 #define EXACT_ROWS 4
 #define EXACT_EMPTY 0xffffffffffffffffull
@@ -205,42 +205,52 @@ __device__ __forceinline__ uint32_t exact_hash(unsigned long long id, uint32_t s
   return (uint32_t)((id * 0x9E3779B97F4A7C15ull) >> 32) >> (__clz(slots) + 1);
 }
 
-// One key's digit for a row; EXACT_EMPTY and `bad` for a key the numbering does not hold.
-__device__ __forceinline__ unsigned long long exact_digit(uint32_t type, unsigned long long raw, unsigned long long kmin, unsigned long long range, bool* bad)
+// A key of a thread's rows: its digits appended to the groups' numbers; `bad` gets the rows whose key the numbering
+// does not hold. The key's type is fixed (8 for both 64-bit integers).
+template <int TYPE>
+__device__ __forceinline__ void exact_key(const void* col, unsigned long long kmin, unsigned long long range, const uint32_t (&row)[EXACT_ROWS],
+                                          unsigned long long (&id)[EXACT_ROWS], uint32_t* bad)
 {
-  unsigned long long v = raw;
-  if (type == 7) v = (unsigned long long)(long long)(int)(uint32_t)raw;
-  else if (type == CQL_EXACT_KEY_U64_AS_F64) v = (unsigned long long)__double_as_longlong((double)raw);
-  else if (type == CQL_EXACT_KEY_I64_AS_F64) v = (unsigned long long)__double_as_longlong((double)(long long)raw);
-  else if (type == 3) { if ((v & 0x7fffffffull) > 0x7f800000ull || v == 0x80000000ull) *bad = true; }
-  else if (type == 4) { if ((v & 0x7fffffffffffffffull) > 0x7ff0000000000000ull || v == 0x8000000000000000ull) *bad = true; }
-  v -= kmin;
-  if (range && v >= range) *bad = true;
-  return v;
+  constexpr bool WIDE = !(TYPE == 1 || TYPE == 3 || TYPE == 7);
+  unsigned long long raw[EXACT_ROWS];
+#pragma unroll
+  for (uint32_t i = 0; i < EXACT_ROWS; i++)
+    raw[i] = WIDE ? __ldcs((const unsigned long long*)col + row[i]) : (unsigned long long)__ldcs((const uint32_t*)col + row[i]);
+#pragma unroll
+  for (uint32_t i = 0; i < EXACT_ROWS; i++)
+  {
+    unsigned long long v = raw[i];
+    bool off = false;
+    if (TYPE == 7) v = (unsigned long long)(long long)(int)(uint32_t)v;
+    if (TYPE == CQL_EXACT_KEY_U64_AS_F64) v = (unsigned long long)__double_as_longlong((double)v);
+    if (TYPE == CQL_EXACT_KEY_I64_AS_F64) v = (unsigned long long)__double_as_longlong((double)(long long)v);
+    if (TYPE == 3) off = (v & 0x7fffffffull) > 0x7f800000ull || v == 0x80000000ull;
+    if (TYPE == 4) off = (v & 0x7fffffffffffffffull) > 0x7ff0000000000000ull || v == 0x8000000000000000ull;
+    v -= kmin;
+    if (off || (range && v >= range)) *bad |= 1u << i;
+    id[i] = id[i] * range + v;
+  }
 }
 
 // Adds (or subtracts) m * 2^pos, m < 2^53, to a 128-bit two's-complement number of four words `stride` apart that
 // threads share.
 __device__ __forceinline__ void exact_add_local(uint32_t* word, uint32_t stride, unsigned long long m, uint32_t pos, bool negative)
 {
-  uint32_t j = pos >> 5, sh = pos & 31u;
-  unsigned long long low = m << sh;
-  uint32_t piece[3] = { (uint32_t)low, (uint32_t)(low >> 32), sh ? (uint32_t)(m >> (64 - sh)) : 0u };
+  const uint32_t j = pos >> 5, sh = pos & 31u, keep = negative ? 0u : 0xffffffffu;
+  const unsigned long long low = m << sh;
+  const uint32_t piece[3] = { (uint32_t)low, (uint32_t)(low >> 32), (uint32_t)((m >> 32) >> (32u - sh)) };   // a shift by 32 gives 0
+  uint32_t* at = word + j * stride;
   uint32_t carry = 0;
 #pragma unroll
   for (uint32_t k = 0; k < 4; k++)
   {
-    unsigned long long t = (unsigned long long)(k < 3 ? piece[k] : 0u) + carry;
-    if (k >= 2 && t == 0) break;
+    if (k >= 2 && piece[2] == 0 && carry == 0) break;   // the second word may hold nothing yet, the third mostly does not
     if (j + k > 3) break;
-    carry = (uint32_t)(t >> 32);
-    uint32_t add = (uint32_t)t;
-    if (add)
-    {
-      uint32_t* at = word + (j + k) * stride;
-      if (negative) carry += atomicSub(at, add) < add ? 1u : 0u;
-      else carry += atomicAdd(at, add) > 0xffffffffu - add ? 1u : 0u;
-    }
+    uint32_t add = (k < 3 ? piece[k] : 0u) + carry;
+    carry = add < carry ? 1u : 0u;
+    // the word's old value, or its complement, below what is subtracted or added: a borrow or a carry
+    if (add) carry += (atomicAdd(at, negative ? 0u - add : add) ^ keep) < add ? 1u : 0u;
+    at += stride;
   }
 }
 
@@ -275,6 +285,94 @@ __device__ __forceinline__ uint32_t exact_slot(unsigned long long* key, uint32_t
     h = (h + 1) & (slots - 1);
   }
   return slots;
+}
+
+struct ExactColumn
+{
+  const void* data;
+  uint32_t type, what;
+  int base, scale;
+  uint32_t low_bits, number;
+};
+
+// One column of a thread's rows into their slots (0xffffffff: none). KIND: 0 whole numbers and decimals, 4 f64, 3
+// f32, 8 64-bit integers met as doubles.
+template <bool LOCAL, int KIND>
+__device__ __forceinline__ void exact_column(const ExactColumn& v, const uint32_t (&row)[EXACT_ROWS], const uint32_t (&sl)[EXACT_ROWS], uint32_t* words, uint32_t S,
+                                             unsigned long long* part, uint32_t T, unsigned long long* mn, unsigned long long* mx, uint32_t* flags,
+                                             uint32_t pos_max, uint32_t* wrong)
+{
+  const uint32_t type = v.type, what = v.what;
+  const bool wide = KIND == 4 || KIND == 8 || (KIND == 0 && (type == 2 || type == 4 || type == 8));
+  unsigned long long raw[EXACT_ROWS];
+#pragma unroll
+  for (uint32_t i = 0; i < EXACT_ROWS; i++)
+    raw[i] = wide ? __ldcs((const unsigned long long*)v.data + row[i]) : (unsigned long long)__ldcs((const uint32_t*)v.data + row[i]);
+#pragma unroll
+  for (uint32_t i = 0; i < EXACT_ROWS; i++)
+  {
+    const uint32_t s = sl[i];
+    if (s == 0xffffffffu) continue;
+    // the value's magnitude and place, and its double's bits
+    unsigned long long m, b;
+    bool negative, finite = true;
+    uint32_t pos = 0;
+    if (KIND == 0)
+    {
+      const long long q = (what & CQL_EXACT_DECIMAL) ? (long long)fix_scaled(fix_decode_f64(raw[i]), v.scale)
+                                                     : type == 7 ? (long long)(int)(uint32_t)raw[i] : (long long)raw[i];
+      negative = q < 0;
+      m = (unsigned long long)(negative ? -q : q);
+      b = (what & (CQL_EXACT_MIN | CQL_EXACT_MAX)) ? cql_int_bits(q) : 0ull;
+    }
+    else
+    {
+      b = KIND == 3 ? cql_f32_bits((uint32_t)raw[i])
+                    : KIND == 4 ? raw[i] : (unsigned long long)__double_as_longlong(type == 8 ? (double)(long long)raw[i] : (double)raw[i]);
+      const uint32_t top = (uint32_t)(b >> 32);
+      const int e = (int)((top >> 20) & 0x7ffu);
+      finite = e != 0x7ff;
+      negative = (b >> 63) != 0;
+      m = ((unsigned long long)((top & 0xfffffu) | (e ? 0x100000u : 0u)) << 32) | (uint32_t)b;
+      int at = max(e, 1) - 1075 - v.base;
+      if ((what & CQL_EXACT_SUM) && (uint32_t)at > pos_max && finite && m)
+      {
+        // below the window's last bit: exact only where those bits are zero
+        if (at >= 0 || at <= -53 || (m & ((1ull << -at) - 1ull))) *wrong |= CQL_EXACT_RANGE;
+        else m >>= -at;
+        at = 0;
+      }
+      pos = (uint32_t)at;
+    }
+    if (what & CQL_EXACT_SUM)
+    {
+      if (!finite)
+        atomicOr(&flags[s], ((b & 0xfffffffffffffull) ? 1u : negative ? 4u : 2u) << (3 * v.number));
+      else if (m)
+      {
+        if (LOCAL) exact_add_local(words + s, S, m, pos, negative);
+        else if (KIND == 0) atomicAdd(&part[s], negative ? 0ull - m : m);
+        else exact_add_parts(part + s, T, v.low_bits, (unsigned __int128)m << pos, negative);
+      }
+    }
+    if (what & (CQL_EXACT_MIN | CQL_EXACT_MAX))
+    {
+      // NaN is left out; -0.0 compares equal to +0.0
+      unsigned long long o = (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+      const bool nan = KIND != 0 && (b << 1) > 0xffe0000000000000ull;
+      if ((b << 1) == 0) o = 0x8000000000000000ull;
+      if (LOCAL)
+      {
+        if ((what & CQL_EXACT_MIN) && o < mn[s] && !nan) atomicMin(&mn[s], o);
+        if ((what & CQL_EXACT_MAX) && o > mx[s] && !nan) atomicMax(&mx[s], o);
+      }
+      else if (!nan)
+      {
+        if (what & CQL_EXACT_MIN) atomicMin(&mn[s], o);
+        if (what & CQL_EXACT_MAX) atomicMax(&mx[s], o);
+      }
+    }
+  }
 }
 
 template <bool LOCAL, bool DIRECT, int THREADS>
@@ -313,28 +411,26 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group_exact(CqlLaun
   {
     if (*(volatile uint32_t*)&s_stop) break;
     unsigned long long id[EXACT_ROWS];
-    uint32_t bad = 0;
+    uint32_t bad = 0, row[EXACT_ROWS];   // a row past the end reads the last one and is left out below
 #pragma unroll
-    for (uint32_t i = 0; i < EXACT_ROWS; i++) id[i] = 0;
+    for (uint32_t i = 0; i < EXACT_ROWS; i++)
+    {
+      id[i] = 0;
+      row[i] = (uint32_t)min(r0 + i * step, rows - 1);
+    }
 #pragma unroll 1
     for (uint32_t k = 0; k < p.key_count; k++)
     {
-      uint32_t type = p.key_type[k];
-      bool wide = !(type == 1 || type == 3 || type == 7);
-      unsigned long long kmin = p.key_min[k], range = p.key_range[k], raw[EXACT_ROWS];
-#pragma unroll
-      for (uint32_t i = 0; i < EXACT_ROWS; i++)
+      const unsigned long long kmin = p.key_min[k], range = p.key_range[k];
+      switch (p.key_type[k])
       {
-        uint64_t r = min(r0 + i * step, rows - 1);
-        raw[i] = wide ? __ldcs((const unsigned long long*)a.buf[k] + r) : (unsigned long long)__ldcs((const uint32_t*)a.buf[k] + r);
-      }
-#pragma unroll
-      for (uint32_t i = 0; i < EXACT_ROWS; i++)
-      {
-        bool off = false;
-        unsigned long long d = exact_digit(type, raw[i], kmin, range, &off);
-        if (off) bad |= 1u << i;
-        id[i] = id[i] * range + d;
+        case 1: exact_key<1>(a.buf[k], kmin, range, row, id, &bad); break;
+        case 3: exact_key<3>(a.buf[k], kmin, range, row, id, &bad); break;
+        case 4: exact_key<4>(a.buf[k], kmin, range, row, id, &bad); break;
+        case 7: exact_key<7>(a.buf[k], kmin, range, row, id, &bad); break;
+        case CQL_EXACT_KEY_U64_AS_F64: exact_key<CQL_EXACT_KEY_U64_AS_F64>(a.buf[k], kmin, range, row, id, &bad); break;
+        case CQL_EXACT_KEY_I64_AS_F64: exact_key<CQL_EXACT_KEY_I64_AS_F64>(a.buf[k], kmin, range, row, id, &bad); break;
+        default: exact_key<8>(a.buf[k], kmin, range, row, id, &bad); break;
       }
     }
     uint32_t sl[EXACT_ROWS];
@@ -381,99 +477,16 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group_exact(CqlLaun
 #pragma unroll 1
     for (uint32_t c = 0; c < p.column_count; c++)
     {
-      uint32_t type = p.col_type[c], what = p.col_what[c];
-      const void* col = a.buf[4 + c];
-      bool wide = type == 2 || type == 4 || type == 8;
-      unsigned long long raw[EXACT_ROWS];
-#pragma unroll
-      for (uint32_t i = 0; i < EXACT_ROWS; i++)
-      {
-        uint64_t r = min(r0 + i * step, rows - 1);
-        raw[i] = wide ? __ldcs((const unsigned long long*)col + r) : (unsigned long long)__ldcs((const uint32_t*)col + r);
-      }
-      int base = p.col_base[c];
-#pragma unroll
-      for (uint32_t i = 0; i < EXACT_ROWS; i++)
-      {
-        uint32_t s = sl[i];
-        if (s == 0xffffffffu) continue;
-        // the value's magnitude and place, and its double's bits
-        unsigned long long m, b;
-        bool negative;
-        uint32_t pos = 0;
-        bool finite = true;
-        if (what & (CQL_EXACT_WHOLE | CQL_EXACT_DECIMAL))
-        {
-          long long q = (what & CQL_EXACT_DECIMAL) ? (long long)fix_scaled(fix_decode_f64(raw[i]), (int)p.col_scale[c])
-                                                   : type == 7 ? (long long)(int)(uint32_t)raw[i] : (long long)raw[i];
-          negative = q < 0;
-          m = (unsigned long long)(negative ? -q : q);
-          b = (what & (CQL_EXACT_MIN | CQL_EXACT_MAX)) ? cql_int_bits(q) : 0ull;
-        }
-        else
-        {
-          b = type == 3 ? cql_f32_bits((uint32_t)raw[i])
-                        : type == 4 ? raw[i]
-                                    : (unsigned long long)__double_as_longlong(type == 8 ? (double)(long long)raw[i] : (double)raw[i]);
-          int e = (int)((b >> 52) & 0x7ffu);
-          finite = e != 0x7ff;
-          negative = (b >> 63) != 0;
-          m = b & 0xfffffffffffffull;
-          if (e) m |= 1ull << 52;
-          else e = 1;
-          int at = e - 1075 - base;
-          if ((what & CQL_EXACT_SUM) && finite && m)
-          {
-            if (at < 0)
-            {
-              // below the window's last bit: exact only where those bits are zero
-              if (at <= -53 || (m & ((1ull << -at) - 1ull))) wrong |= CQL_EXACT_RANGE;
-              else m >>= -at;
-              at = 0;
-            }
-            if ((uint32_t)at > pos_max)
-            {
-              wrong |= CQL_EXACT_RANGE;
-              at = 0;
-            }
-            pos = (uint32_t)at;
-          }
-        }
-        if (what & CQL_EXACT_SUM)
-        {
-          if (!finite)
-          {
-            uint32_t f = ((b & 0xfffffffffffffull) ? 1u : negative ? 4u : 2u) << (3 * c);
-            atomicOr(LOCAL ? &lflags[s] : &t.flags[s], f);
-          }
-          else if (m)
-          {
-            if (LOCAL) exact_add_local(lsum + (uint64_t)p.col_sum[c] * 4 * S + s, S, m, pos, negative);
-            else if (what & (CQL_EXACT_WHOLE | CQL_EXACT_DECIMAL)) atomicAdd(&t.part[(uint64_t)p.col_sum[c] * 3 * T + s], negative ? 0ull - m : m);
-            else exact_add_parts(t.part + (uint64_t)p.col_sum[c] * 3 * T + s, T, p.low_bits, (unsigned __int128)m << pos, negative);
-          }
-        }
-        if (what & (CQL_EXACT_MIN | CQL_EXACT_MAX))
-        {
-          if (finite || !(b & 0xfffffffffffffull))   // NaN is left out
-          {
-            if ((b << 1) == 0) b = 0;   // -0.0 compares equal to +0.0
-            unsigned long long o = (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
-            if (LOCAL)
-            {
-              unsigned long long* mn = lmn + p.col_min[c] * S + s;
-              unsigned long long* mx = lmx + p.col_max[c] * S + s;
-              if ((what & CQL_EXACT_MIN) && o < *mn) atomicMin(mn, o);
-              if ((what & CQL_EXACT_MAX) && o > *mx) atomicMax(mx, o);
-            }
-            else
-            {
-              if (what & CQL_EXACT_MIN) atomicMin(&t.mn[(uint64_t)p.col_min[c] * T + s], o);
-              if (what & CQL_EXACT_MAX) atomicMax(&t.mx[(uint64_t)p.col_max[c] * T + s], o);
-            }
-          }
-        }
-      }
+      const ExactColumn v = { a.buf[4 + c], p.col_type[c], p.col_what[c], p.col_base[c], (int)p.col_scale[c], p.low_bits, c };
+      unsigned long long* part = t.part + (uint64_t)p.col_sum[c] * 3 * T;
+      unsigned long long* mn = LOCAL ? lmn + p.col_min[c] * S : t.mn + (uint64_t)p.col_min[c] * T;
+      unsigned long long* mx = LOCAL ? lmx + p.col_max[c] * S : t.mx + (uint64_t)p.col_max[c] * T;
+      uint32_t* flags = LOCAL ? lflags : t.flags;
+      uint32_t* words = lsum + (uint64_t)p.col_sum[c] * 4 * S;
+      if (v.what & (CQL_EXACT_WHOLE | CQL_EXACT_DECIMAL)) exact_column<LOCAL, 0>(v, row, sl, words, S, part, T, mn, mx, flags, pos_max, &wrong);
+      else if (v.type == 4) exact_column<LOCAL, 4>(v, row, sl, words, S, part, T, mn, mx, flags, pos_max, &wrong);
+      else if (v.type == 3) exact_column<LOCAL, 3>(v, row, sl, words, S, part, T, mn, mx, flags, pos_max, &wrong);
+      else exact_column<LOCAL, 8>(v, row, sl, words, S, part, T, mn, mx, flags, pos_max, &wrong);
     }
     if (wrong) *(volatile uint32_t*)&s_stop = 1;
   }
