@@ -848,7 +848,6 @@ static char* batch_source_tiled(char** shape_exprs, const uint32_t* shape_sites,
 #define RANK_TABLE (RANK_CUTS + 1u)                                     /* a column's cuts, padded to a power of two */
 #define RANK_CUT_BYTES (CQLOPS_MAX_BINDINGS * RANK_TABLE * 8u + 64u)    /* a launch's cuts, then each column's search steps */
 #define RANK_QUERIES 160u       /* a launch's queries: its accumulators leave room for three CTAs an SM */
-#define RANK_MIN_LAUNCH 48u     /* launches are halved down to this many while their cuts do not fit */
 #define RANK_MIN_QUERIES 2u     /* two queries: 54 -> 47 us over 300 thousand rows, 454 -> 346 over 50M; one: equal */
 #define FORM_REGISTERS (1u << 24)   /* with a form: not as ranks */
 #define RANK_BAD (1ull << 44)   /* added to the first query's count by a CTA that met a summand outside its planes */
@@ -1228,66 +1227,62 @@ static uint32_t cut_rank(const uint64_t* cuts, uint32_t n, uint64_t key)
   return lo;
 }
 
-static int cut_order(const void* x, const void* y)
+/* adds a cut to a column's; 0 when they are RANK_CUTS already */
+static int cut_add(uint64_t* cuts, uint32_t* n, uint64_t key)
 {
-  const uint64_t a = *(const uint64_t*)x, b = *(const uint64_t*)y;
-  return a < b ? -1 : a > b;
+  const uint32_t at = cut_rank(cuts, *n, key);
+  if (at && cuts[at - 1] == key) return 1;
+  if (*n == RANK_CUTS) return 0;
+  memmove(cuts + at + 1, cuts + at, (*n - at) * sizeof(uint64_t));
+  cuts[at] = key;
+  (*n)++;
+  return 1;
 }
 
-/* The cuts of a launch's thresholds and the thresholds as bounds of ranks; 0 when a column has more than
-   RANK_CUTS. A key is in [lo, hi] when its rank is at least lo's and below hi + 1's. */
-static int rank_thresholds(const Thr* thr, uint32_t queries, const int* slot_type, RankThr* out, unsigned char* cut_bytes)
+/* The next launch: as many of the queries, in order, as leave every column at most RANK_CUTS cuts (one query has at
+   most 32), their thresholds as bounds of ranks, the cuts and the search steps. A key is in [lo, hi] when its rank is
+   at least lo's and below hi + 1's. Returns the number of queries. */
+static uint32_t rank_launch(const Thr* thr, uint32_t queries, const int* slot_type, RankThr* out, unsigned char* cut_bytes)
 {
-  const uint64_t n = (uint64_t)queries * BATCH_MAX_SITES;
-  uint64_t* cuts = (uint64_t*)malloc((2 * n + 1) * sizeof(uint64_t));
-  uint32_t* list = (uint32_t*)malloc((n + 1) * sizeof(uint32_t));
+  uint64_t cuts[CQLOPS_MAX_BINDINGS][RANK_TABLE];
+  uint32_t n[CQLOPS_MAX_BINDINGS] = { 0 };
+  uint64_t lo, hi;
+  uint32_t taken = 0;
+  if (queries > RANK_QUERIES) queries = RANK_QUERIES;
+  for (; taken < queries; taken++)
+  {
+    int fits = 1;
+    /* a query's comparisons come first among its places; a column it overfills keeps cuts no taken query needs */
+    for (const Thr* t = thr + (uint64_t)taken * BATCH_MAX_SITES; fits && t < thr + ((uint64_t)taken + 1) * BATCH_MAX_SITES && t->site; t++)
+    {
+      const uint32_t c = (uint32_t)(t->site & 0xffu) - 1u;
+      const uint64_t top = slot_type[c] == CQLOPS_TYPE_F64 ? ~0ull : 0xffffffffull;
+      rank_interval(t, &lo, &hi);
+      fits = (lo == 0 || cut_add(cuts[c], &n[c], lo)) && (hi >= top || cut_add(cuts[c], &n[c], hi + 1));
+    }
+    if (!fits) break;
+  }
   uint64_t* table = (uint64_t*)cut_bytes;
   uint32_t* steps = (uint32_t*)(cut_bytes + (uint64_t)CQLOPS_MAX_BINDINGS * RANK_TABLE * 8u);
-  int ok = cuts && list;
-  memset(out, 0, n * sizeof(RankThr));
   memset(cut_bytes, 0, RANK_CUT_BYTES);
-  /* the comparisons of all queries (a query's come first among its places) */
-  uint32_t sites = 0;
-  for (uint32_t q = 0; ok && q < queries; q++)
-    for (uint32_t i = q * BATCH_MAX_SITES; i < (q + 1) * BATCH_MAX_SITES && thr[i].site; i++) list[sites++] = i;
-  for (int c = 0; ok && c < CQLOPS_MAX_BINDINGS; c++)
+  for (uint32_t c = 0; c < CQLOPS_MAX_BINDINGS; c++)
   {
-    if (!slot_type[c]) continue;
     const uint64_t top = slot_type[c] == CQLOPS_TYPE_F64 ? ~0ull : 0xffffffffull;
-    uint64_t k = 0, lo, hi;
-    for (uint32_t i = 0; i < sites; i++)
-    {
-      const Thr* t = &thr[list[i]];
-      if ((t->site & 0xffu) != (uint64_t)c + 1u) continue;
-      rank_interval(t, &lo, &hi);
-      if (lo > 0) cuts[k++] = lo;
-      if (hi < top) cuts[k++] = hi + 1;
-    }
-    qsort(cuts, k, sizeof(uint64_t), cut_order);
-    uint32_t u = 0;
-    for (uint64_t i = 0; i < k; i++)
-      if (u == 0 || cuts[u - 1] != cuts[i]) cuts[u++] = cuts[i];
-    if (u > RANK_CUTS)
-    {
-      ok = 0;
-      break;
-    }
-    while ((1u << steps[c]) <= u) steps[c]++;
-    for (uint32_t i = 0; i < RANK_TABLE; i++) table[(uint32_t)c * RANK_TABLE + i] = i < u ? cuts[i] : top;
-    for (uint32_t i = 0; i < sites; i++)
-    {
-      const Thr* t = &thr[list[i]];
-      if ((t->site & 0xffu) != (uint64_t)c + 1u) continue;
-      const int inv = rank_interval(t, &lo, &hi);
-      const uint32_t rl = lo > 0 ? cut_rank(cuts, u, lo) : 0u, rh = hi < top ? cut_rank(cuts, u, hi + 1) : 128u;
-      out[list[i]].lo = rl * 0x01010101u;
-      out[list[i]].hi = rh * 0x01010101u;
-      out[list[i]].inv = inv ? 0x80808080u : 0u;
-    }
+    while ((1u << steps[c]) <= n[c]) steps[c]++;
+    for (uint32_t i = 0; i < RANK_TABLE; i++) table[c * RANK_TABLE + i] = i < n[c] ? cuts[c][i] : top;
   }
-  free(cuts);
-  free(list);
-  return ok;
+  memset(out, 0, (size_t)taken * BATCH_MAX_SITES * sizeof(RankThr));
+  for (uint32_t i = 0; i < taken * BATCH_MAX_SITES; i++)
+  {
+    if (!thr[i].site) continue;
+    const uint32_t c = (uint32_t)(thr[i].site & 0xffu) - 1u;
+    const uint64_t top = slot_type[c] == CQLOPS_TYPE_F64 ? ~0ull : 0xffffffffull;
+    const int inv = rank_interval(&thr[i], &lo, &hi);
+    out[i].lo = (lo > 0 ? cut_rank(cuts[c], n[c], lo) : 0u) * 0x01010101u;
+    out[i].hi = (hi < top ? cut_rank(cuts[c], n[c], hi + 1) : 128u) * 0x01010101u;
+    out[i].inv = inv ? 0x80808080u : 0u;
+  }
+  return taken;
 }
 
 /* a rank form's kernel, found by what its source is made from - the source itself, some 40 KB, is written
@@ -2256,34 +2251,41 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     }
   uint64_t* folded = ok && mode == BATCH_RUN ? (uint64_t*)malloc((size_t)nalloc * 24) : NULL;
   ok = ok && (folded || mode != BATCH_RUN);
-  /* the rank form, where every predicate is comparisons with literals and the launches' cuts fit, in
-     launches of fewer queries if need be */
-  uint32_t launch_cap = CQL_BATCH_LAUNCH_QUERIES;
+  /* the launches' first queries: the rank form's, where every predicate is comparisons with literals, as many as their
+     cuts allow, else CQL_BATCH_LAUNCH_QUERIES each */
   const RankLayout rank_form = rank_layout(launch_types, sum_col_count, wr);
+  uint32_t* slice_at = (uint32_t*)malloc(((size_t)scan_n + 2) * sizeof(uint32_t));
+  uint32_t slices = 0, widest = 0;
   RankThr* rank_thr = NULL;
   unsigned char* rank_cuts = NULL;
+  ok = ok && slice_at;
   ranks = ranks && ok && scan_n >= RANK_MIN_QUERIES && (mode == BATCH_RUN || mode == BATCH_PREPARE || mode == BATCH_SOURCE);
   for (uint32_t sh = 0; ranks && sh < launch_shapes; sh++) ranks = rank_expr(launch_exprs[sh]);
   for (uint32_t c = 0; ranks && mode == BATCH_RUN && c < column_count; c++)
     ranks = !(((uint64_t)(uintptr_t)cqlcuda_buffer_device_pointer(columns[c].buffer)) & 15u);
-  if (ranks)
+  if (ranks) rank_thr = (RankThr*)malloc((size_t)scan_n * BATCH_MAX_SITES * sizeof(RankThr));
+  ranks = ranks && rank_thr;
+  for (uint32_t first = 0; ok && first < scan_n; slices++)
   {
-    rank_thr = (RankThr*)malloc((size_t)scan_n * BATCH_MAX_SITES * sizeof(RankThr));
-    rank_cuts = (unsigned char*)malloc((size_t)(scan_n / RANK_MIN_LAUNCH + 1) * RANK_CUT_BYTES);
-    int fits = 0;
-    launch_cap = RANK_QUERIES;
-    for (; rank_thr && rank_cuts && !fits && launch_cap >= RANK_MIN_LAUNCH; launch_cap /= fits ? 1 : 2)
+    uint32_t n = scan_n - first < CQL_BATCH_LAUNCH_QUERIES ? scan_n - first : CQL_BATCH_LAUNCH_QUERIES;
+    if (ranks)
     {
-      fits = 1;
-      for (uint32_t first = 0; fits && first < scan_n; first += launch_cap)
-        fits = rank_thresholds(thr_o + (uint64_t)first * BATCH_MAX_SITES, scan_n - first < launch_cap ? scan_n - first : launch_cap, launch_types,
-                               rank_thr + (uint64_t)first * BATCH_MAX_SITES, rank_cuts + (uint64_t)(first / launch_cap) * RANK_CUT_BYTES);
+      unsigned char* more = (unsigned char*)realloc(rank_cuts, (size_t)(slices + 1) * RANK_CUT_BYTES);
+      if (!more)
+      {
+        ok = 0;
+        break;
+      }
+      rank_cuts = more;
+      n = rank_launch(thr_o + (uint64_t)first * BATCH_MAX_SITES, scan_n - first, launch_types, rank_thr + (uint64_t)first * BATCH_MAX_SITES,
+                      rank_cuts + (uint64_t)slices * RANK_CUT_BYTES);
     }
-    ranks = fits;
-    if (!fits) launch_cap = CQL_BATCH_LAUNCH_QUERIES;
+    slice_at[slices] = first;
+    slice_at[slices + 1] = first + n;
+    if (n > widest) widest = n;
+    first += n;
   }
-  /* one launch per slice of at most launch_cap queries: its shapes (all of the catalog's, with a catalog)
-     and where each starts */
+  /* one launch per slice: its shapes (all of the catalog's, with a catalog) and where each starts */
   uint32_t begin[BATCH_MAX_SHAPES + 1];
   char* slice_exprs[BATCH_MAX_SHAPES];
   uint32_t slice_sites[BATCH_MAX_SHAPES];
@@ -2372,7 +2374,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   }
   if (ok && (mode == BATCH_SOURCE || mode == BATCH_PREPARE) && (scan_n || view))
   {
-    uint32_t nq = scan_n < launch_cap ? scan_n : launch_cap;
+    uint32_t nq = slices ? slice_at[1] : 0;
     uint32_t ns;
     SLICE_SHAPES(0, nq, ns);
     char* src = ranks ? batch_source_ranks(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rank_form)
@@ -2416,7 +2418,6 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
      integers at 16..), the scan's thresholds, literals and summed columns in shape order, each slice's shape
      starts, the rank form's cuts per slice, then the cube queries' thresholds, literals and (shape, cube, summed column); each part on a
      16-byte boundary */
-  uint32_t slices = (scan_n + launch_cap - 1) / launch_cap;
   const uint64_t off_thr = 256;
   const uint64_t off_qc = off_thr + (uint64_t)scan_n * BATCH_MAX_SITES * (ranks ? sizeof(RankThr) : sizeof(Thr));
   const uint64_t off_qs = off_qc + (ranks ? 0 : (uint64_t)scan_n * BATCH_MAX_CONSTS * 8);
@@ -2457,7 +2458,6 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   uint32_t per_sm = ranks ? rank_form.per_sm
                           : (rows_per_thread ? register_ctas_per_sm(block) : tiled_layout(launch_types, sum_col_count).per_sm);
   uint64_t ctas = (uint64_t)(sm_count ? sm_count : 152) * per_sm;
-  uint32_t widest = scan_n < launch_cap ? scan_n : launch_cap;
   const uint64_t cube_out_bytes = 16 + (uint64_t)cube_n * 24;   /* the error word, then (count, lo, hi) per cube query */
   uint64_t* cube_out = launch && cube_n ? (uint64_t*)malloc(cube_out_bytes) : NULL;
   if (launch && cube_n && !cube_out) ok = 0;
@@ -2477,8 +2477,8 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   CqlKernel* shared_k = NULL;
   for (uint32_t sl = 0; launch && ok && sl < slices; sl++)
   {
-    uint32_t first = sl * launch_cap;
-    uint32_t nq = scan_n - first < launch_cap ? scan_n - first : launch_cap;
+    uint32_t first = slice_at[sl];
+    uint32_t nq = slice_at[sl + 1] - first;
     uint32_t ns;
     SLICE_SHAPES(first, nq, ns);
     memcpy(params + off_begin + sl * begin_stride, begin, (ns + 1) * 4);
@@ -2541,8 +2541,8 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     }
     for (uint32_t sl = 0; sl < slices; sl++)
     {
-      uint32_t first = sl * launch_cap;
-      uint32_t nq = scan_n - first < launch_cap ? scan_n - first : launch_cap;
+      uint32_t first = slice_at[sl];
+      uint32_t nq = slice_at[sl + 1] - first;
       CqlKernel* k = kernels[sl];
       cqlcuda_kernel_set_arg_buffer_range(k, 0, param_buf, 0, 256);
       cqlcuda_kernel_set_arg_buffer_range(k, 1, param_buf, off_thr, off_qc - off_thr);
@@ -2575,7 +2575,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   /* a summand outside the rank form's planes (a value outside its column's stated range): the batch runs
      again in the register form */
   int again = 0;
-  for (uint32_t first = 0; ranks && launch && ok && first < scan_n; first += launch_cap) again |= folded[first * 3] >= RANK_BAD;
+  for (uint32_t sl = 0; ranks && launch && ok && sl < slices; sl++) again |= folded[slice_at[sl] * 3] >= RANK_BAD;
   if (again)
     ok = batch_run(catalog, programs, query_count, columns, column_count, sum_columns, rows_per_thread | FORM_REGISTERS, out_counts, out_sums,
                    out_shapes, BATCH_RUN, NULL, 0, NULL, allow_cubes);
@@ -2665,6 +2665,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   free(qs_o);
   free(rank_thr);
   free(rank_cuts);
+  free(slice_at);
   free(folded);
   return ok;
 }
