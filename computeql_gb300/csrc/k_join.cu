@@ -6,6 +6,9 @@
 //  join_pack_key          src/gpu/vulkan/shaders/join_pack_key.comp:1-52          two whole-number keys folded into one f64 key
 //  join_probe_native      src/gpu/vulkan/shaders/join_probe_native.comp:1-238     fact-side probe fused with per-dim-row aggregates
 //
+// Of GB300's own: cql_join_unique_* (an equi-join whose build keys are unique) and cql_join_hash_* (a join-aggregate
+// whose table carries each key's group), below.
+//
 // Keys are f64 values (or raw strings) hashed from their bit patterns exactly as the reference does, so a
 // build row lands in the same bucket. GB300 design: persistent grid-stride launches; the fused probe keeps
 // eight keys and their Bloom words in flight per thread and bounds every open-addressing walk by the

@@ -20,6 +20,8 @@
  *  4. One warp owns its accumulators in shared memory (a 32-bit count and a 64-bit sum per query, no
  *     atomics); a CTA folds its warps into 128-bit sums, a second kernel folds the CTAs in order. At
  *     most CQL_BATCH_LAUNCH_QUERIES queries go into one launch.
+ *  5. Batches whose conditions are comparisons with literals run in the rank form: a byte a row and column
+ *     says where the value lies among the launch's literals, and decides every comparison.
  */
 #define _POSIX_C_SOURCE 200809L
 #include "cqlops.h"

@@ -3,7 +3,7 @@
  * host memory in selection order (selection_gather.comp modes 0/1, qe_selection_gather_column,
  * src/query_exec/query_exec.c:4371-4410, which the reference runs one column and one batch at a time).
  *
- * Here one batch uploads the selection once, gathers up to 13 columns a launch into one destination
+ * Here one batch uploads the selection once, gathers every column in one launch into one destination
  * buffer (each column in a 16-byte-aligned section) and reads every section straight into the caller's
  * array. Raw strings take two batches: their lengths and an exclusive scan of them (the output offsets),
  * then a warp per row copies the bytes.

@@ -9,6 +9,9 @@
  *   4a. whole-number arguments: aggregate_hash_reduce_fixed, per-row atomics            :11611-11790
  *   4b. otherwise: csr_scatter into member lists, aggregate_reduce per 4096-row chunk,
  *       HyperLogLog registers and t-digest centroids, folded on the host in chunk order :11826-12275
+ *   4c. of GB300's own, before 1-4 where they apply: one pass into tables of exact sums over numbered keys
+ *       (cql_group_exact), a small-range key (cql_group_small), a wide dense key (cql_group_direct), and the
+ *       sketch registers straight from the columns (cql_hll_rows)
  *   5. qe_hll_estimate_cardinality (:6711-6737, rounded :12230) and
  *      qe_tdigest_estimate_percentile (:6748-6790)
  */

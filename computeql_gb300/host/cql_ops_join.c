@@ -4,12 +4,15 @@
  *  cqlops_hash_join       qe_hash_join_impl (src/query_exec/query_exec.c:14541-15358): build-side bucket
  *                         histogram, three-pass prefix sum, scatter into bucket lists, probe emitting
  *                         (probe row, build row) pairs, LEFT JOIN unmatched rows, output capacity
- *                         max(probe, build) + probe (qe_join_output_capacity :14368-14381) grown once
+ *                         max(probe, build) + probe (qe_join_output_capacity :14368-14381) grown once;
+ *                         numeric build keys that prove unique take one table and need no sort
  *  cqlops_join_aggregate  qe_aggregate_join_pushdown (:8442-8776): the fact table reduced to totals per
  *                         join key - densely when the fact key's range is small (qe_dense_stream_core),
  *                         else by probing a CPU-built linear-probing table of the dim keys behind a Bloom
  *                         filter (qe_join_probe_stream_core :8080-8420) - then every (filtered) dim row
- *                         meets its key's totals and is folded into a group of its group columns on the host
+ *                         meets its key's totals and is folded into a group of its group columns on the host;
+ *                         unique keys spread wider with one whole-number group value take a hash table that
+ *                         carries the group
  */
 #include "cqlops.h"
 #include "cql_ops_internal.h"

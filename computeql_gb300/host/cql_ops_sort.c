@@ -1,7 +1,8 @@
 /*
  * cql_ops_sort.c - ORDER BY up to 4 numeric keys, ties by input position (qe_sort_rows,
  * src/query_exec/query_exec.c:5376-6155; the tie rule of the generated sort, query_kernel.c:2156-2177),
- * as a stable LSD radix sort on the GPU: the last key first, each key 8 bits per pass.
+ * as a stable LSD radix sort on the GPU: the last key first, each key 8 bits per pass. Keys of more than
+ * 32 bits together are sorted by a 32-bit prefix of them, then within the runs that share it.
  */
 #include "cqlops.h"
 #include "cql_ops_internal.h"

@@ -251,8 +251,11 @@ int cqlops_group_dense(const CqlColumn* key, uint64_t rows, uint32_t expr_count,
    shared scan (exact scaled-integer sums), MIN/MAX and each group's first row from one more pass (groups in
    key order, each represented by its first row; automatic takes it when it
    applies and some argument is not a decimal of at most 6 places, which path 2 finalizes as the
-   reference does). Per dense group g: out_repr_row[g] (a row of the group), out_counts[g],
-   out_results[g*expr_count + e]. out_path receives the path taken (1, 2 or 3). */
+   reference does). Automatic also answers numeric keys that number in one 64-bit word from tables of
+   exact sums in one pass, and APPROX_COUNT_DISTINCT of the whole table or of a key of up to 8192 values
+   from one pass over the column; out_path then receives the path they stand for. Per dense group g:
+   out_repr_row[g] (a row of the group), out_counts[g], out_results[g*expr_count + e]. out_path receives
+   the path taken (1, 2, 3, or 4: tables indexed by a whole-number key of a wide dense range). */
 int cqlops_group_hash(const CqlColumn* keys, uint32_t key_count, uint32_t expr_count, const uint32_t* funcs, const CqlColumn* const* args,
                       const double* params, uint64_t group_hint, uint32_t path, uint64_t max_groups, uint64_t* out_group_count,
                       uint64_t* out_repr_row, uint64_t* out_counts, double* out_results, uint32_t* out_path);
@@ -271,6 +274,8 @@ double cqlops_tdigest_percentile(float* means, float* weights, uint64_t count, d
    GPU path, src/query_exec/query_exec.c:14541-15358: the build side hashed into buckets (a power of
    two >= its rows), bucket lists by prefix sum and scatter, every probe row emitting its
    (probe row, build row) pairs; a LEFT join also emits (probe row, 0xffffffff) for an unmatched row.
+   Numeric build keys that turn out unique are joined by a table of the keys in probe order, without the
+   bucket lists and without sorting the pairs; the answer is the same.
    hint_pairs > 0 sizes the output for that many pairs. Writes the pair count and up to
    out_capacity pairs, sorted, as (probe, build) u32 pairs. */
 int cqlops_hash_join(const CqlColumn* build_key, const CqlColumn* probe_key, int left_join, uint64_t hint_pairs, uint64_t* out_count,
@@ -294,7 +299,9 @@ typedef struct CqlJoinAgg
   uint32_t strategy;                  /* 0 automatic, 1 dense over the fact key's range, 2 probe a hash table of the dim keys,
                                          3 a lookup table over the fact key's range (unique dim keys, at most one
                                          whole-number GROUP BY value spanning < 65536, no dim-side aggregates, a key
-                                         range up to 2^24; automatic picks it for ranges above 65536 when it applies) */
+                                         range up to 2^24; automatic picks it for ranges above 65536 when it applies).
+                                         Automatic answers unique dim keys spread wider, grouped by one whole-number
+                                         value, from a hash table that carries each key's group (reported as 2) */
   /* Optional: the dim table resident on the device - its key column (dim_table_rows rows, the keys of
      dim_keys) and its one GROUP BY column (whole numbers spanning at most 65536 values, the values of
      dim_group_values). With them, a dense join's dim-row pass runs on the device instead of the host. */
@@ -348,7 +355,8 @@ int cqlops_group_dense_fixed(const CqlColumn* key, uint32_t expr_count, const ui
 
 /* ORDER BY up to 4 numeric keys (desc[k] != 0 for DESC), keys compared as F64 values with ties broken
    by input position - qe_sort_rows (src/query_exec/query_exec.c:5376-6155, compare :4859-4882) with a
-   stable LSD radix sort in place of the bitonic sorts. Without a selection the input is the columns' rows
+   stable LSD radix sort in place of the bitonic sorts (keys of more than 32 bits from 16384 rows on by a
+   32-bit prefix, the short runs that share one then put in order by the full keys). Without a selection the input is the columns' rows
    and the output their row numbers; with one (selection_count u32 row numbers in a device buffer, the
    row set of a filter) the input is those rows in selection order and the output is their row numbers.
    Writes up to out_capacity row numbers in sorted order. */
@@ -411,7 +419,11 @@ int cqlops_window_rank(const CqlColumn* keys, uint32_t key_count, const uint32_t
    depend on the form, so every form gives the same sums. rows_per_thread picks the form of the generated
    kernel: 4, 8 or 16 rows a thread in registers (plus 1 << 9 for 512-thread CTAs instead of 256), 0 the
    shared-memory tile form, or CQLOPS_BATCH_AUTOTUNE: the form timed fastest for the batch's plan shape,
-   each candidate timed on the shape's first batches. out_shapes (optional) receives the shape count.
+   each candidate timed on the shape's first batches. With 8 in 256 threads (the default of the callers
+   here) a batch of two queries or more whose conditions are comparisons of columns with literals, joined
+   by AND and OR, runs over the columns' ranks among the literals instead: the fastest form where it
+   applies (16-byte aligned columns, summed values inside their stated range; else 8 rows a thread).
+   out_shapes (optional) receives the shape count.
    Refuses programs with string comparisons. */
 int cqlops_batch_filter_aggregate(const CqlProgram* const* programs, uint32_t query_count, const CqlColumn* columns, uint32_t column_count,
                                   const int32_t* sum_columns, uint32_t rows_per_thread, uint64_t* out_counts, double* out_sums,
