@@ -2287,7 +2287,8 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     if (n > widest) widest = n;
     first += n;
   }
-  /* one launch per slice: its shapes (all of the catalog's, with a catalog) and where each starts */
+  /* one launch per slice: its shapes and where each starts. With a catalog, and in the rank form, whose slices depend
+     on the literals, all the shapes there are: one kernel whatever the batch's literals */
   uint32_t begin[BATCH_MAX_SHAPES + 1];
   char* slice_exprs[BATCH_MAX_SHAPES];
   uint32_t slice_sites[BATCH_MAX_SHAPES];
@@ -2295,7 +2296,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   do                                                                                  \
   {                                                                                   \
     ns = 0;                                                                           \
-    if (view && launch_exprs == view->exprs)                                          \
+    if (ranks || (view && launch_exprs == view->exprs))                               \
     {                                                                                 \
       uint32_t at_ = 0;                                                               \
       for (uint32_t s_ = 0; s_ < launch_shapes; s_++)                                 \
@@ -2500,7 +2501,7 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
         ok = 0;
         break;
       }
-      if (view && launch_exprs == view->exprs) shared_k = k;
+      if (ranks || (view && launch_exprs == view->exprs)) shared_k = k;
     }
     kernels[sl] = k;
   }

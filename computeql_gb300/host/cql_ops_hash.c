@@ -1067,7 +1067,8 @@ static int group_exact(const CqlColumn* keys, uint32_t key_count, uint64_t rows,
     CqlBuffer* ob = pooled("group_exact_out", out_bytes, CQLCUDA_BUFFER_READ_WRITE);
     CqlBuffer* bits = listed ? pooled("group_exact_bits", ((table_slots + 31) / 32) * 4, CQLCUDA_BUFFER_READ_WRITE) : NULL;
     CqlBuffer* list = listed ? pooled("group_exact_list", cap * 4, CQLCUDA_BUFFER_READ_WRITE) : NULL;
-    if (!tab || !ob || (listed && (!bits || !list))) return 0;
+    /* no room for the tables (up to EXACT_TABLE_BYTES): the member lists, which take less of few rows */
+    if (!tab || !ob || (listed && (!bits || !list))) return -1;
     cqlcuda_kernel_set_arg_buffer(k, 12, pb);
     cqlcuda_kernel_set_arg_buffer(k, 13, tab);
     cqlcuda_kernel_set_arg_buffer_range(k, 14, ob, 16, 4);

@@ -151,3 +151,33 @@ def test_catalog_prepared_for_both_forms(ops):
             m = t["d"] > q + 0.5
             assert c[q] == m.sum() and abs(s[q] - t["v"][m].sum()) <= 1e-12 * t["v"].sum()
     cat.close()
+
+
+@pytest.mark.parametrize("rows", [3, 4099])
+def test_bool_column(ops, rows):
+    """a column of one byte a row, compared and summed"""
+    r = np.random.default_rng(rows)
+    b, v = r.integers(0, 2, rows, dtype=np.uint8), r.random(rows)
+    cols = {"b": ops.Column(6, rows, ops.DeviceBuffer(rows, b), zone=(0.0, 1.0), zone_map=False), "v": ops.Column.from_numpy(v)}
+    qs = [("(= b 1)", "v"), ("(and (!= b 1) (< v 0.25))", "v"), ("(or (>= b 1) (> v 0.5))", "b")]
+    _, c, s = _agree(ops, cols, qs)
+    want = [b == 1, (b != 1) & (v < 0.25), (b >= 1) | (v > 0.5)]
+    assert [int(x) for x in c] == [int(w.sum()) for w in want] and s[2] == b[want[2]].sum()
+
+
+def test_new_literals_compile_nothing(ops):
+    """a batch of several launches and known shapes, with other literals and so other launches, reuses its kernel"""
+    from computeql_gb300 import native
+    t = _table(20_000, 12)
+    cols = _columns(ops, t)
+    n = native.C.c_uint64()
+    compiled = []
+    for seed in (1, 2, 3):
+        r = np.random.default_rng(seed)
+        qs = [(w, "v") for k in range(200) for w in (f"(> d {r.normal() * 1e3:.6f})", f"(and (< u {r.integers(1 << 32)}) (<= d {r.normal():.6f}))")]
+        progs = [ops.Program(w, cols) for w, _ in qs]
+        c, _, shapes = ops.batch_aggregate(progs, ["v"] * len(qs))
+        assert shapes == 2 and c[0] == (t["d"] > float(qs[0][0].split()[-1][:-1])).sum()
+        native.load_cuda().cqlcuda_generated_kernel_stats(native.C.byref(n), None)
+        compiled.append(n.value)
+    assert compiled[0] == compiled[1] == compiled[2]
