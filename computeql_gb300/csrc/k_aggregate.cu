@@ -445,194 +445,54 @@ static int launch_aggregate_global(const CqlLaunch& a, uint32_t gws, uint32_t lw
 #define FUNC_MIN   3u
 #define FUNC_MAX   4u
 
-struct DenseDecode
+// A column's quads of rows as they are stored: 16 bytes of whole words, 8 of 2-byte codes, 4 of 1-byte codes, nothing of
+// a sequence; a narrow column's value is base + code.
+struct DenseColumn
 {
-  const uint32_t* col[5];  // key, arg0..3
-  uint32_t log2w[5], bits[5], mask[5], base[5];
-  bool seq[5];
-  uint32_t chunk_start;
+  const void* data;
+  uint32_t width, base;   // 4, 2, 1, or 3: a sequence, base + row
 };
 
-__device__ __forceinline__ uint32_t dense_read(const DenseDecode& d, int c, uint64_t row)
+__device__ __forceinline__ uint4 quad_load(const DenseColumn& c, uint64_t quad)
 {
-  if (d.seq[c]) return d.base[c] + d.chunk_start + (uint32_t)row;
-  uint32_t l = d.log2w[c];
-  uint32_t w = d.col[c][row >> l];
-  uint32_t sh = (uint32_t)((row & ((1u << l) - 1u)) * d.bits[c]) & 31u;
-  return d.base[c] + ((w >> sh) & d.mask[c]);
+  if (c.width == 4) return __ldcs((const uint4*)c.data + quad);
+  if (c.width == 2)
+  {
+    const uint2 q = __ldcs((const uint2*)c.data + quad);
+    return make_uint4(q.x, q.y, 0, 0);
+  }
+  if (c.width == 1) return make_uint4(__ldcs((const uint32_t*)c.data + quad), 0, 0, 0);
+  return make_uint4((uint32_t)quad * 4u, 0, 0, 0);
 }
 
-struct DenseLayout
+__device__ __forceinline__ uint4 quad_values(const DenseColumn& c, uint4 q)
 {
-  uint32_t groups;        // groups in this pass
-  uint32_t exprs;
-  uint32_t nsum, nmm;     // expressions needing a sum slot / a min+max slot
-  uint32_t copies;        // privatised copies of the table
-  uint32_t copy_words;    // 32-bit words per copy (sums are 2 words, 8-byte aligned)
-  uint32_t sum_off, mm_off;
-  uint32_t sum_slot[8], mm_slot[8];
-};
-
-// words per group of one copy: count, then 2 words per summed expr, then 2 words per min/max expr
-__host__ __device__ inline uint32_t dense_group_words(uint32_t nsum, uint32_t nmm) { return 1 + 2 * nsum + 2 * nmm; }
-
-template <bool WIDE_VEC>
-__global__ void __launch_bounds__(1024) k_aggregate_dense(CqlLaunch a, DenseLayout L, uint32_t group_base, uint64_t rows)
-{
-  extern __shared__ __align__(16) uint32_t smem[];
-  DenseDecode d;
-  uint32_t widths = cql_word(a, 1);
-  uint32_t arg_base[4] = { cql_word(a, 3), cql_word(a, 5), cql_word(a, 9), cql_word(a, 11) };
-  for (int c = 0; c < 5; c++)
-  {
-    uint32_t w = (widths >> (4 * c)) & 0xfu;
-    d.col[c] = (const uint32_t*)a.buf[c];
-    d.log2w[c] = w == 1 ? 2 : (w == 2 ? 1 : 0);
-    d.bits[c] = w == 1 ? 8 : (w == 2 ? 16 : 32);
-    d.mask[c] = w == 1 ? 0xffu : (w == 2 ? 0xffffu : 0xffffffffu);
-    if (c == 0) d.base[c] = (w == 1 || w == 2) ? cql_word(a, 10) : 0u;
-    else d.base[c] = (w == 1 || w == 2 || w == 3) ? arg_base[c - 1] : 0u;
-    d.seq[c] = c > 0 && w == 3;
-  }
-  d.chunk_start = cql_word(a, 15);
-  uint32_t func_codes = cql_word(a, 4);
-  uint32_t arg_index = cql_word(a, 6);
-  uint32_t arg_signed = cql_word(a, 7);
-  int min_key = (int)cql_word(a, 10);
-
-  // per copy: [count | sums (8-byte aligned) | min,max] for each group
-  uint32_t G = L.groups;
-  uint32_t total = L.copies * L.copy_words;
-  for (uint32_t i = threadIdx.x; i < total; i += blockDim.x)
-  {
-    uint32_t in_copy = i % L.copy_words;
-    uint32_t v = 0;
-    if (in_copy >= L.mm_off)
-    {
-      uint32_t k = in_copy - L.mm_off;
-      v = (k & 1u) ? 0x80000000u : 0x7fffffffu;  // min then max per (group, expr)
-    }
-    smem[i] = v;
-  }
-  __syncthreads();
-
-  uint32_t copy = (threadIdx.x >> 5) % L.copies;
-  uint32_t* cnt = smem + copy * L.copy_words;
-  unsigned long long* sums = (unsigned long long*)(smem + copy * L.copy_words + L.sum_off);
-  int* mm = (int*)(smem + copy * L.copy_words + L.mm_off);
-
-  auto count_row = [&](uint64_t row, uint32_t key) {
-    int id = (int)key - min_key - (int)group_base;
-    if (id < 0 || (uint32_t)id >= G) return;
-    atomicAdd(&cnt[id], 1u);
-    for (uint32_t e = 0; e < L.exprs; e++)
-    {
-      uint32_t f = (func_codes >> (e * 4)) & 0xfu;
-      if (f == FUNC_COUNT) continue;
-      uint32_t ai = (arg_index >> (e * 4)) & 0x3u;  // at most 4 argument columns are bound
-      uint32_t word = dense_read(d, 1 + (int)ai, row);
-      if (f == FUNC_SUM || f == FUNC_AVG)
-      {
-        bool is_signed = ((arg_signed >> ai) & 1u) != 0u;
-        unsigned long long add = is_signed ? (unsigned long long)(long long)(int)word : (unsigned long long)word;
-        atomicAdd(&sums[(uint32_t)id * L.nsum + L.sum_slot[e]], add);
-      }
-      else if (f == FUNC_MIN)
-        atomicMin(&mm[((uint32_t)id * L.nmm + L.mm_slot[e]) * 2], (int)word);
-      else if (f == FUNC_MAX)
-        atomicMax(&mm[((uint32_t)id * L.nmm + L.mm_slot[e]) * 2 + 1], (int)word);
-    }
-  };
-
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (WIDE_VEC)
-  {
-    // whole-word key: four keys per 16-byte load, two vectors in flight
-    const uint4* kv = (const uint4*)d.col[0];
-    uint64_t vec_count = rows / 4;
-    uint64_t i = t;
-    for (; i + stride < vec_count; i += 2 * stride)
-    {
-      uint4 q0 = __ldcs(kv + i);
-      uint4 q1 = __ldcs(kv + i + stride);
-      uint64_t r0 = i * 4, r1 = (i + stride) * 4;
-      count_row(r0 + 0, q0.x);
-      count_row(r0 + 1, q0.y);
-      count_row(r0 + 2, q0.z);
-      count_row(r0 + 3, q0.w);
-      count_row(r1 + 0, q1.x);
-      count_row(r1 + 1, q1.y);
-      count_row(r1 + 2, q1.z);
-      count_row(r1 + 3, q1.w);
-    }
-    for (; i < vec_count; i += stride)
-    {
-      uint4 q = __ldcs(kv + i);
-      uint64_t r = i * 4;
-      count_row(r + 0, q.x);
-      count_row(r + 1, q.y);
-      count_row(r + 2, q.z);
-      count_row(r + 3, q.w);
-    }
-    uint64_t tail = vec_count * 4;
-    if (t < rows - tail) count_row(tail + t, d.col[0][tail + t]);
-  }
-  else
-  {
-    for (uint64_t row = t; row < rows; row += stride) count_row(row, dense_read(d, 0, row));
-  }
-  __syncthreads();
-
-  // fold the copies and merge into the global arrays, skipping groups this CTA never saw
-  uint32_t* info = (uint32_t*)a.buf[5];
-  unsigned long long* gsum = (unsigned long long*)a.buf[6];
-  int* gmin = (int*)a.buf[7];
-  int* gmax = (int*)a.buf[8];
-  uint64_t info_cap = a.bytes[5] / 4, sum_cap = a.bytes[6] / 8, mm_cap_min = a.bytes[7] / 4, mm_cap_max = a.bytes[8] / 4;
-  for (uint32_t g = threadIdx.x; g < G; g += blockDim.x)
-  {
-    uint32_t count = 0;
-    for (uint32_t c = 0; c < L.copies; c++) count += smem[c * L.copy_words + g];
-    if (count == 0) continue;
-    uint64_t gg = (uint64_t)group_base + g;
-    if (gg * 2 + 1 < info_cap) atomicAdd(&info[gg * 2 + 1], count);
-    for (uint32_t e = 0; e < L.exprs; e++)
-    {
-      uint32_t f = (func_codes >> (e * 4)) & 0xfu;
-      uint64_t index = gg * L.exprs + e;
-      if (f == FUNC_SUM || f == FUNC_AVG)
-      {
-        unsigned long long s = 0;
-        for (uint32_t c = 0; c < L.copies; c++)
-          s += ((unsigned long long*)(smem + c * L.copy_words + L.sum_off))[g * L.nsum + L.sum_slot[e]];
-        if (index < sum_cap) atomicAdd(&gsum[index], s);
-      }
-      else if (f == FUNC_MIN || f == FUNC_MAX)
-      {
-        int best = f == FUNC_MIN ? 0x7fffffff : (int)0x80000000;
-        for (uint32_t c = 0; c < L.copies; c++)
-        {
-          int v = ((int*)(smem + c * L.copy_words + L.mm_off))[(g * L.nmm + L.mm_slot[e]) * 2 + (f == FUNC_MAX ? 1 : 0)];
-          best = f == FUNC_MIN ? min(best, v) : max(best, v);
-        }
-        if (f == FUNC_MIN && index < mm_cap_min) atomicMin(&gmin[index], best);
-        if (f == FUNC_MAX && index < mm_cap_max) atomicMax(&gmax[index], best);
-      }
-    }
-  }
+  if (c.width == 4) return q;
+  if (c.width == 2) return make_uint4(c.base + (q.x & 0xffffu), c.base + (q.x >> 16), c.base + (q.y & 0xffffu), c.base + (q.y >> 16));
+  if (c.width == 1) return make_uint4(c.base + (q.x & 0xffu), c.base + ((q.x >> 8) & 0xffu), c.base + ((q.x >> 16) & 0xffu), c.base + (q.x >> 24));
+  return make_uint4(c.base + q.x, c.base + q.x + 1u, c.base + q.x + 2u, c.base + q.x + 3u);
 }
 
+__device__ __forceinline__ uint32_t row_value(const DenseColumn& c, uint64_t row)
+{
+  if (c.width == 4) return ((const uint32_t*)c.data)[row];
+  if (c.width == 2) return c.base + ((const uint16_t*)c.data)[row];
+  if (c.width == 1) return c.base + ((const uint8_t*)c.data)[row];
+  return c.base + (uint32_t)row;
+}
 
-// Fast path for whole-word keys and argument columns (the full-width u32/i32 case): per-expression
+// One pass over the key and the argument columns: per-expression
 // metadata unrolled into registers, key and argument vectors loaded together (16 bytes each), 32-bit
 // shared atomics with a carry into the high word as aggregate_dense_native.comp:184-200 does, one
 // private table per warp when the groups are few. KEYARG: the one argument column is the key column
 // itself (GROUP BY amount ... SUM(amount)), read once.
 // DEPTH: key vectors (and vectors of every argument column) in flight per thread. 2 where several CTAs share an
 // SM; 4 for the one-CTA-an-SM tables (1024 threads, a table of thousands of groups), whose warps alone must keep
-// enough loads in flight.
-template <int NE, int NA, bool KEYARG = false, int DEPTH = 2>
+// enough loads in flight, and for narrow columns, whose vectors are short.
+// NARROW: the key or an argument is narrow or a sequence, the widths looked at once a vector (a uniform branch). Such
+// columns had a kernel of their own, a row a thread and 64-bit shared sums: 1549 us for 282M rows of 1-byte keys and
+// u32 arguments (1.4 GB), 446 here; 300M rows of 20000 groups 4942 and 997.
+template <int NE, int NA, bool KEYARG = false, int DEPTH = 2, bool NARROW = false>
 __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint32_t G, uint32_t group_base, uint64_t rows,
                                                                uint32_t copies, uint32_t copy_words, uint32_t nsum)
 {
@@ -641,12 +501,13 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
   uint32_t arg_index = cql_word(a, 6);
   uint32_t arg_signed = cql_word(a, 7);
   int min_key = (int)cql_word(a, 10);
+  const uint32_t exprs = NARROW ? cql_word(a, 2) : (uint32_t)NE;   // (narrow: 5 to 8 of them share a kernel of 8)
   uint32_t f[NE], ai[NE], sg[NE], slot[NE];
   uint32_t ns = 0, nm = 0;
 #pragma unroll
   for (int e = 0; e < NE; e++)
   {
-    f[e] = (func_codes >> (4 * e)) & 0xfu;
+    f[e] = !NARROW || (uint32_t)e < exprs ? (func_codes >> (4 * e)) & 0xfu : FUNC_COUNT;
     ai[e] = (arg_index >> (4 * e)) & 0x3u;
     sg[e] = (arg_signed >> ai[e]) & 1u;
     slot[e] = 0;
@@ -706,6 +567,20 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
   uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   constexpr int NC = NA > 0 ? NA : 1;
+  // column 0 the key (narrow: its codes count from the smallest key), then the arguments
+  DenseColumn dc[NC + 1];
+  if constexpr (NARROW)
+  {
+    const uint32_t widths = cql_word(a, 1);
+#pragma unroll
+    for (int c = 0; c <= NC; c++)
+    {
+      const uint32_t w = (widths >> (4 * c)) & 0xfu;
+      dc[c].data = a.buf[c];
+      dc[c].width = w == 1 || w == 2 || (w == 3 && c > 0) ? w : 4u;
+      dc[c].base = c == 0 ? (uint32_t)min_key : cql_word(a, c == 1 ? 3 : c == 2 ? 5 : c == 3 ? 9 : 11) + (w == 3 ? cql_word(a, 15) : 0u);
+    }
+  }
   uint64_t i = t;
   // DEPTH key vectors and DEPTH vectors of every argument column in flight per thread
   for (; i + (uint64_t)(DEPTH - 1) * stride < vec_count; i += DEPTH * stride)
@@ -714,18 +589,26 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
 #pragma unroll
     for (int dd = 0; dd < DEPTH; dd++)
     {
-      kk[dd] = __ldcs(kv + i + dd * stride);
+      if constexpr (NARROW) kk[dd] = quad_load(dc[0], i + dd * stride);
+      else kk[dd] = __ldcs(kv + i + dd * stride);
 #pragma unroll
       for (int c = 0; c < NC; c++)
       {
         if (KEYARG) qq[dd][c] = kk[dd];
-        else if (c < NA) qq[dd][c] = __ldcs((const uint4*)a.buf[1 + c] + i + dd * stride);
-        else qq[dd][c] = make_uint4(0, 0, 0, 0);
+        else if (c >= NA) qq[dd][c] = make_uint4(0, 0, 0, 0);
+        else if constexpr (NARROW) qq[dd][c] = quad_load(dc[1 + c], i + dd * stride);
+        else qq[dd][c] = __ldcs((const uint4*)a.buf[1 + c] + i + dd * stride);
       }
     }
 #pragma unroll
     for (int dd = 0; dd < DEPTH; dd++)
     {
+      if constexpr (NARROW)
+      {
+        kk[dd] = quad_values(dc[0], kk[dd]);
+#pragma unroll
+        for (int c = 0; c < NA; c++) qq[dd][c] = quad_values(dc[1 + c], qq[dd][c]);
+      }
       uint32_t v[NC];
 #pragma unroll
       for (int c = 0; c < NC; c++) v[c] = qq[dd][c].x;
@@ -743,10 +626,19 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
   }
   for (; i < vec_count; i += stride)
   {
-    uint4 k0 = __ldcs(kv + i);
-    uint4 q0[NC];
+    uint4 k0, q0[NC];
+    if constexpr (NARROW)
+    {
+      k0 = quad_values(dc[0], quad_load(dc[0], i));
 #pragma unroll
-    for (int c = 0; c < NC; c++) q0[c] = c < NA ? (KEYARG ? k0 : __ldcs((const uint4*)a.buf[1 + c] + i)) : make_uint4(0, 0, 0, 0);
+      for (int c = 0; c < NC; c++) q0[c] = c < NA ? quad_values(dc[1 + c], quad_load(dc[1 + c], i)) : make_uint4(0, 0, 0, 0);
+    }
+    else
+    {
+      k0 = __ldcs(kv + i);
+#pragma unroll
+      for (int c = 0; c < NC; c++) q0[c] = c < NA ? (KEYARG ? k0 : __ldcs((const uint4*)a.buf[1 + c] + i)) : make_uint4(0, 0, 0, 0);
+    }
     uint32_t v[NC];
 #pragma unroll
     for (int c = 0; c < NC; c++) v[c] = q0[c].x;
@@ -767,8 +659,8 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
     uint64_t r = tail + t;
     uint32_t v[NC];
 #pragma unroll
-    for (int c = 0; c < NC; c++) v[c] = c < NA ? ((const uint32_t*)a.buf[1 + c])[r] : 0u;
-    row(((const uint32_t*)a.buf[0])[r], v);
+    for (int c = 0; c < NC; c++) v[c] = c >= NA ? 0u : NARROW ? row_value(dc[1 + c], r) : ((const uint32_t*)a.buf[1 + c])[r];
+    row(NARROW ? row_value(dc[0], r) : ((const uint32_t*)a.buf[0])[r], v);
   }
   __syncthreads();
 
@@ -787,7 +679,7 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
 #pragma unroll
     for (int e = 0; e < NE; e++)
     {
-      uint64_t index = gg * NE + e;
+      uint64_t index = gg * exprs + e;
       if (KEYARG && f[e] != FUNC_COUNT)
       {
         uint32_t key = (uint32_t)(min_key + (int)gg);
@@ -835,29 +727,36 @@ static const DenseWideFn k_dense_keyarg_table[8] = { k_aggregate_dense_wide<1, 1
                                                      k_aggregate_dense_wide<5, 1, true>, k_aggregate_dense_wide<6, 1, true>,
                                                      k_aggregate_dense_wide<7, 1, true>, k_aggregate_dense_wide<8, 1, true> };
 #undef DW_ROW
+#define DWN_ROW(NE, D)                                                                                                                \
+  { k_aggregate_dense_wide<NE, 0, false, D, true>, k_aggregate_dense_wide<NE, 1, false, D, true>, k_aggregate_dense_wide<NE, 2, false, D, true>, \
+    k_aggregate_dense_wide<NE, 4, false, 2, true> }
+static const DenseWideFn k_dense_narrow_table[5][4] = { DWN_ROW(1, 4), DWN_ROW(2, 4), DWN_ROW(3, 4), DWN_ROW(4, 4), DWN_ROW(8, 2) };
+#undef DWN_ROW
 
-// Whole-word key and arguments: one pass per tile of groups that fits shared memory.
-static int launch_dense_wide(const CqlLaunch& a, uint64_t rows, uint32_t exprs, uint32_t groups, uint32_t nsum, uint32_t nmm, cudaStream_t stream)
+// One pass per tile of groups that fits shared memory.
+static int launch_dense_wide(const CqlLaunch& a, uint64_t rows, uint32_t exprs, uint32_t groups, uint32_t nsum, uint32_t nmm, bool narrow, cudaStream_t stream)
 {
   uint32_t per_group = 1 + 2 * nsum + 2 * nmm;
   uint32_t budget_words = (uint32_t)(std::min(g_cql_max_smem_optin, 200 * 1024) / 4);
   uint32_t tile = std::min<uint32_t>(groups, budget_words / per_group);
   if (tile == 0) return (int)cudaErrorInvalidValue;
+  if (exprs == 0) exprs = 1;   // only the rows are counted: a COUNT
   // distinct argument columns are bound at 1..n in order (qe_dense_stream_core, query_exec.c:7863-7867)
   uint32_t funcs = cql_word(a, 4), arg_index = cql_word(a, 6), na = 0;
   for (uint32_t e = 0; e < exprs; e++)
   {
     uint32_t f = (funcs >> (4 * e)) & 0xfu;
-    if (f != FUNC_COUNT) na = std::max(na, ((arg_index >> (4 * e)) & 0x3u) + 1);
+    if (f != FUNC_COUNT && e < cql_word(a, 2)) na = std::max(na, ((arg_index >> (4 * e)) & 0x3u) + 1);
   }
-  bool keyarg = na == 1 && a.buf[1] == a.buf[0];
+  bool keyarg = !narrow && na == 1 && a.buf[1] == a.buf[0];
   for (uint32_t base = 0; base < groups; base += tile)
   {
     uint32_t G = std::min(tile, groups - base);
     uint32_t copy_words = (G * per_group + 3) & ~3u;
     uint32_t threads = copy_words * 4 > 48 * 1024 ? 1024 : 512;
     DenseWideFn fn = keyarg ? k_dense_keyarg_table[exprs - 1] : k_dense_wide_table[exprs - 1][na <= 2 ? na : 3];
-    if (threads == 1024 && keyarg && exprs <= 2) fn = k_dense_keyarg_deep[exprs - 1];
+    if (narrow) fn = k_dense_narrow_table[std::min(exprs, 5u) - 1][na <= 2 ? na : 3];
+    else if (threads == 1024 && keyarg && exprs <= 2) fn = k_dense_keyarg_deep[exprs - 1];
     else if (threads == 1024 && !keyarg && exprs <= 4 && na <= 2) fn = k_dense_wide_deep[exprs - 1][na];
     uint32_t copies = 1;
     while (copies < threads / 32 && (uint64_t)copy_words * 4 * copies * 2 <= 32 * 1024) copies *= 2;
@@ -884,71 +783,20 @@ static int launch_aggregate_dense(const CqlLaunch& a, uint32_t gws, uint32_t lws
   uint32_t groups = cql_word(a, 8);
   if (exprs > 8 || groups == 0 || rows == 0) return 0;
 
-  DenseLayout L;
-  L.exprs = exprs;
-  L.nsum = 0;
-  L.nmm = 0;
-  for (uint32_t e = 0; e < 8; e++)
-  {
-    L.sum_slot[e] = 0;
-    L.mm_slot[e] = 0;
-  }
+  uint32_t nsum = 0, nmm = 0;
   for (uint32_t e = 0; e < exprs; e++)
   {
     uint32_t f = (funcs >> (e * 4)) & 0xfu;
-    if (f == FUNC_SUM || f == FUNC_AVG) L.sum_slot[e] = L.nsum++;
-    if (f == FUNC_MIN || f == FUNC_MAX) L.mm_slot[e] = L.nmm++;
+    if (f == FUNC_SUM || f == FUNC_AVG) nsum++;
+    if (f == FUNC_MIN || f == FUNC_MAX) nmm++;
   }
-  // whole-word key and arguments take the fast path
-  bool all_wide = true;
+  bool narrow = false;
   for (uint32_t c = 0; c < 5; c++)
   {
     uint32_t w = (widths >> (4 * c)) & 0xfu;
-    if (!(w == 0 || w == 4)) all_wide = false;
+    if (!(w == 0 || w == 4)) narrow = true;
   }
-  if (all_wide) return launch_dense_wide(a, rows, exprs, groups, L.nsum, L.nmm, stream);
-
-  uint32_t per_group_words = dense_group_words(L.nsum, L.nmm);
-  uint32_t budget_words = (uint32_t)(std::min(g_cql_max_smem_optin, 200 * 1024) / 4);
-  uint32_t tile = groups;
-  if ((uint64_t)tile * per_group_words + 4 > budget_words) tile = (budget_words - 4) / per_group_words;
-  if (tile == 0) return (int)cudaErrorInvalidValue;
-
-  bool wide = (widths & 0xfu) == 0 || (widths & 0xfu) == 4;
-  for (uint32_t base = 0; base < groups; base += tile)
-  {
-    uint32_t G = std::min(tile, groups - base);
-    L.groups = G;
-    // words of one copy: counts (padded to even), sums (2 words each), min/max pairs
-    uint32_t cnt_words = (G + 1) & ~1u;
-    L.sum_off = cnt_words;
-    L.mm_off = L.sum_off + 2 * G * L.nsum;
-    L.copy_words = L.mm_off + 2 * G * L.nmm;
-    L.copy_words = (L.copy_words + 3) & ~3u;
-    // few groups: one copy per warp so 32 lanes of 16 warps do not serialise on the same words
-    uint32_t threads = L.copy_words * 4 > 64 * 1024 ? 1024 : 512;
-    uint32_t warps = threads / 32;
-    uint32_t copies = 1;
-    while (copies < warps && (uint64_t)L.copy_words * 4 * copies * 2 <= 48 * 1024 && G <= 4096) copies *= 2;
-    L.copies = copies;
-    size_t smem = (size_t)L.copy_words * 4 * copies;
-    int per_sm = 1;
-    if (smem <= 24 * 1024) per_sm = threads == 512 ? 4 : 2;
-    else if (smem <= 48 * 1024) per_sm = threads == 512 ? 3 : 2;
-    else if (smem <= 100 * 1024) per_sm = 2;
-    if (threads == 1024 && per_sm > 2) per_sm = 2;
-    if (smem > 48 * 1024)
-    {
-      if (wide) cudaFuncSetAttribute(k_aggregate_dense<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      else cudaFuncSetAttribute(k_aggregate_dense<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    }
-    uint64_t need = (rows / (wide ? 4 : 1) + threads - 1) / threads;
-    uint32_t grid = cql_stream_grid(need ? need : 1, per_sm);
-    if (wide) k_aggregate_dense<true><<<grid, threads, smem, stream>>>(a, L, base, rows);
-    else k_aggregate_dense<false><<<grid, threads, smem, stream>>>(a, L, base, rows);
-    CQL_LAUNCH_CHECK();
-  }
-  return 0;
+  return launch_dense_wide(a, rows, exprs, groups, nsum, nmm, narrow, stream);
 }
 
 // aggregate_global_f32.comp:1-13 has the same bindings and slots 0-2 but no type words: every column is F32
