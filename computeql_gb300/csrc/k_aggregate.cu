@@ -579,6 +579,8 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
       dc[c].data = a.buf[c];
       dc[c].width = w == 1 || w == 2 || (w == 3 && c > 0) ? w : 4u;
       dc[c].base = c == 0 ? (uint32_t)min_key : cql_word(a, c == 1 ? 3 : c == 2 ? 5 : c == 3 ? 9 : 11) + (w == 3 ? cql_word(a, 15) : 0u);
+      // a column that does not start on its vectors' boundary: every row by itself, below
+      if ((c == 0 || c <= NA) && dc[c].width != 3 && ((uintptr_t)dc[c].data & (4 * dc[c].width - 1))) vec_count = 0;
     }
   }
   uint64_t i = t;
@@ -653,10 +655,8 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
     for (int c = 0; c < NC; c++) v[c] = q0[c].w;
     row(k0.w, v);
   }
-  uint64_t tail = vec_count * 4;
-  if (t < rows - tail)
+  for (uint64_t r = vec_count * 4 + t; r < rows; r += stride)
   {
-    uint64_t r = tail + t;
     uint32_t v[NC];
 #pragma unroll
     for (int c = 0; c < NC; c++) v[c] = c >= NA ? 0u : NARROW ? row_value(dc[1 + c], r) : ((const uint32_t*)a.buf[1 + c])[r];
