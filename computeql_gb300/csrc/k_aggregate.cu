@@ -572,10 +572,15 @@ __global__ void __launch_bounds__(1024) k_aggregate_dense_wide(CqlLaunch a, uint
   if constexpr (NARROW)
   {
     const uint32_t widths = cql_word(a, 1);
+    // the arguments there are; a kernel of more has none in the others, whose bindings are not columns of these rows
+    uint32_t used = 0;
+#pragma unroll
+    for (int e = 0; e < NE; e++)
+      if (f[e] != FUNC_COUNT) used = max(used, ai[e] + 1u);
 #pragma unroll
     for (int c = 0; c <= NC; c++)
     {
-      const uint32_t w = (widths >> (4 * c)) & 0xfu;
+      const uint32_t w = (uint32_t)c > used ? 3u : (widths >> (4 * c)) & 0xfu;
       dc[c].data = a.buf[c];
       dc[c].width = w == 1 || w == 2 || (w == 3 && c > 0) ? w : 4u;
       dc[c].base = c == 0 ? (uint32_t)min_key : cql_word(a, c == 1 ? 3 : c == 2 ? 5 : c == 3 ? 9 : 11) + (w == 3 ? cql_word(a, 15) : 0u);
