@@ -1036,7 +1036,8 @@ static int group_exact(const CqlColumn* keys, uint32_t key_count, uint64_t rows,
     if (local)
     {
       uint64_t n = p.direct ? product : expected ? expected : 1300;
-      while (expected && p.copies_log2 < 5 && (n << (p.copies_log2 + 1)) <= 512 && (p.direct || product >> 58 == 0)) p.copies_log2++;
+      /* (a hashed copy's number stands below the group's: only numbers of at most 58 bits leave room, and 0 means 2^64) */
+      while (expected && p.copies_log2 < 5 && (n << (p.copies_log2 + 1)) <= 512 && (p.direct || (product && product >> 58 == 0))) p.copies_log2++;
       uint64_t s = p.direct ? n << p.copies_log2 : pow2_from((n << p.copies_log2) * 3 / 2);
       if (!p.direct && s < 256) s = 256;
       uint64_t bytes = s * slot_bytes;
