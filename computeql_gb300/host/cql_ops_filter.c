@@ -182,19 +182,14 @@ static int program_buffers(const CqlProgram* prog, CqlBuffer** out_code, CqlBuff
 }
 
 /* The program written into its buffers, in the batch of the kernel that reads it: a batch of its own cost a wait for the
-   device (13 us of a 1M-row query's 138) before the kernel was even launched. The generated kernels read no bytecode. */
+   device (13 us of a 1M-row query's 138) before the kernel was even launched. The batch takes the bytes as late as its end, so
+   they are the program's own, which outlives it; the kernels read the pool's strings byte by byte, so that nothing past
+   it is needed. The generated kernels read no bytecode. */
 static void upload_program(CqlBatch* batch, const CqlProgram* prog, int bytecode, CqlBuffer* code, CqlBuffer* consts, CqlBuffer* strs)
 {
   if (bytecode && prog->word_count) cqlcuda_batch_buffer_write(batch, code, prog->words, (uint64_t)prog->word_count * 4);
   if (prog->const_count) cqlcuda_batch_buffer_write(batch, consts, prog->consts, (uint64_t)prog->const_count * 8);
-  if (prog->str_pool_size)
-  {
-    uint8_t pad[CQLOPS_MAX_STR_POOL + 4];
-    uint64_t str_bytes = (prog->str_pool_size + 3u) & ~3u;
-    memset(pad + prog->str_pool_size, 0, str_bytes - prog->str_pool_size);
-    memcpy(pad, prog->str_pool, prog->str_pool_size);
-    cqlcuda_batch_buffer_write(batch, strs, pad, str_bytes);
-  }
+  if (prog->str_pool_size) cqlcuda_batch_buffer_write(batch, strs, prog->str_pool, prog->str_pool_size);
 }
 
 /* scan_simple over the program's leaves, columns remapped to the leaf columns */
