@@ -38,11 +38,13 @@ class _ResultBlocks:
     A fresh large array is mapped anew, and its first touch costs more than the copy into it: on Grace's 64 KB pages
     about 3 us a page (8 MB of join pairs: 400 us, against 50 us for the copy). `take` gives an array over a block that an
     earlier result has left, or over a new one; the block comes back when the last array over it is gone, whichever
-    thread drops it. Free blocks are kept up to LIMIT touched bytes, the longest unused dropped first; results below
-    SMALL, which malloc reuses by itself, are ordinary arrays.
+    thread drops it. Free blocks are kept up to LIMIT touched and MAPPED mapped bytes, the longest unused dropped first, as
+    soon as a block comes back; results below SMALL, which malloc reuses by itself, are ordinary arrays. No result
+    keeps more than SHARE times its own bytes in memory: a block that holds more is not taken for it, and `cut` copies
+    what is little of a block (and anything below COPIED, whose copy costs a few us).
     """
 
-    LIMIT, SMALL = 256 << 20, 1 << 20
+    LIMIT, MAPPED, SMALL, COPIED, SHARE = 256 << 20, 16 << 30, 1 << 20, 64 << 10, 8
 
     class _Lease:
         def __init__(self, blocks, memory, touched, count, dtype):
@@ -51,36 +53,59 @@ class _ResultBlocks:
 
         def __del__(self):
             self.blocks.returned.append((self.memory, self.touched))     # deque.append takes no lock
+            self.memory = None
+            self.blocks._settle()
 
     def __init__(self):
         self.lock = threading.Lock()
         self.returned = collections.deque()
         self.free = []                          # (memory, touched bytes), the longest unused first
 
+    def _sort_in(self):
+        """with the lock: the returned blocks among the free ones, within the limits"""
+        while self.returned:
+            self.free.append(self.returned.popleft())
+        touched, mapped = sum(t for _, t in self.free), sum(m.nbytes for m, _ in self.free)
+        while touched > self.LIMIT or mapped > self.MAPPED:
+            memory, held = self.free.pop(0)
+            touched, mapped = touched - held, mapped - memory.nbytes
+
+    def _settle(self):
+        # Runs in destructors too, so it never waits: who holds the lock looks again once it is free.
+        while self.returned and self.lock.acquire(blocking=False):
+            try:
+                self._sort_in()
+            finally:
+                self.lock.release()
+
     def take(self, count, dtype, used=None):
         """An uninitialized array of `count` values. `used` (optional): a list that receives a function to call with
-        the bytes the result took, when it is less than the array."""
+        the bytes the result took, when it is less than the array; it returns the bytes the block holds in memory."""
         dtype = np.dtype(dtype)
         size = count * dtype.itemsize
         if size < self.SMALL:
             return np.empty(count, dtype=dtype)
         with self.lock:
-            while self.returned:
-                self.free.append(self.returned.popleft())
-            kept = sum(t for _, t in self.free)
-            while kept > self.LIMIT:
-                kept -= self.free.pop(0)[1]
-            fits = [i for i, (m, _) in enumerate(self.free) if m.nbytes >= size]
+            self._sort_in()
+            fits = [i for i, (m, t) in enumerate(self.free) if m.nbytes >= size and t <= self.SHARE * size]
             at = min(fits, key=lambda i: self.free[i][0].nbytes, default=None)
             memory, touched = self.free.pop(at) if at is not None else (None, 0)
+        self._settle()
         if memory is None:
             memory = np.empty(size + size // 8, dtype=np.uint8)          # a little more: the next result may be larger
-        lease = self._Lease(self, memory, memory.nbytes, count, dtype)
+        lease = self._Lease(self, memory, max(touched, size), count, dtype)
         if used is not None:
             def note(nbytes):
                 lease.touched = max(touched, nbytes)
+                return lease.touched
             used.append(note)
         return np.asarray(lease)
+
+    def cut(self, array, count, used):
+        """The first `count` values of an array from `take`, all that was written of it."""
+        part = array[:count]
+        held = max([note(part.nbytes) for note in used], default=array.nbytes)
+        return part.copy() if part.nbytes < self.COPIED or part.nbytes * self.SHARE < held else part
 
 
 _results = _ResultBlocks()
@@ -231,9 +256,7 @@ def scan_simple(columns, leaves, want_rows=False, max_rows=None):
         out_ptr = N.ptr(rows)
     _check(N.load_ops().cqlops_scan_simple(arr, len(columns), lv, len(leaves), C.byref(count), out_ptr, cap), "cqlops_scan_simple")
     if want_rows:
-        rows = rows[: min(count.value, cap)]     # a view: what is past the rows was never touched
-        for note in used:
-            note(rows.nbytes)
+        rows = _results.cut(rows, min(count.value, cap), used)     # what is past the rows was never touched
     return count.value, rows
 
 
@@ -401,9 +424,7 @@ def scan_filter(program, strategy=SCAN_AUTO, want_rows=False, max_rows=None):
     _check(ok, "cqlops_scan_filter")
     if not want_rows:
         return count.value, None, ran.value
-    rows = rows_arr[: min(count.value, cap)]     # a view: what is past the rows was never touched
-    for note in used:
-        note(rows.nbytes)
+    rows = _results.cut(rows_arr, min(count.value, cap), used)     # what is past the rows was never touched
     return count.value, rows, ran.value
 
 
@@ -579,12 +600,12 @@ def hash_join(build_key, probe_key, left=False, hint_pairs=0, want_pairs=True):
         _check(N.load_ops().cqlops_hash_join(C.byref(bc), C.byref(pc_), 1 if left else 0, hint_pairs, C.byref(count),
                                              N.ptr(out) if want_pairs else None, cap), "cqlops_hash_join")
         n = count.value
-        for note in used:
-            note(min(n, cap) * 8)
+        if want_pairs:
+            out = _results.cut(out, 2 * min(n, cap), used)
         if not want_pairs or n <= cap:
             break
         cap = hint_pairs = n          # the host array was too small: once more with room for every pair
-    return n, (out[: 2 * n].reshape(-1, 2) if want_pairs else None)
+    return n, (out.reshape(-1, 2) if want_pairs else None)
 
 
 def join_aggregate(fact_key, funcs, fact_args, dim_keys, dim_rows=None, group_values=(), dim_args=None, strategy=0, dim_key_col=None,
