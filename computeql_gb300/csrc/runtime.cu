@@ -722,6 +722,14 @@ extern "C" CqlBuffer* cqlcuda_buffer_alloc_pooled(const char* name, uint64_t nam
   return b;
 }
 
+extern "C" void cqlcuda_pool_idle(const char* name, uint64_t name_len)
+{
+  CqlState& s = S();
+  std::lock_guard<std::recursive_mutex> g(s.lock);
+  CqlPooled* slot = pool_find(L().pool_tag + std::string(name, name_len));
+  if (slot) slot->last_epoch = 0;   // before every epoch: pool_evict's first choice
+}
+
 // Host memory is pinned and mapped read-only; on a GB300 node (NVLink-C2C, ATS) the GPU could also
 // read pageable memory directly, which is the fallback when registration is refused.
 extern "C" CqlBuffer* cqlcuda_buffer_import_host_readonly(const void* host_ptr, uint64_t size)

@@ -62,6 +62,11 @@ static CqlBuffer* pooled(const char* name, uint64_t size, uint32_t flags)
   return cqlcuda_buffer_alloc_pooled(name, (uint64_t)strlen(name), size ? size : 4, flags, NULL);
 }
 
+static void idle(const char* name)
+{
+  cqlcuda_pool_idle(name, (uint64_t)strlen(name));
+}
+
 static CqlKernel* kernel(const char* name)
 {
   return cqlcuda_kernel_alloc(name, (uint64_t)strlen(name));
@@ -998,9 +1003,9 @@ static int exact_units(CqlGroupPlan* p, const CqlColumn* const* cols, uint64_t r
 }
 
 /* 1 done, 0 failed, -1 the query does not fit (or its data does not: the caller's general path answers it) */
-static int group_exact(const CqlColumn* keys, uint32_t key_count, uint64_t rows, uint32_t expr_count, const uint32_t* funcs,
-                       const CqlColumn* const* args, int use_fixed, uint32_t fixed_scales, uint64_t group_hint, uint64_t max_groups,
-                       uint64_t* out_group_count, uint64_t* out_repr_row, uint64_t* out_counts, double* out_results)
+static int group_exact_run(const CqlColumn* keys, uint32_t key_count, uint64_t rows, uint32_t expr_count, const uint32_t* funcs,
+                           const CqlColumn* const* args, int use_fixed, uint32_t fixed_scales, uint64_t group_hint, uint64_t max_groups,
+                           uint64_t* out_group_count, uint64_t* out_repr_row, uint64_t* out_counts, double* out_results)
 {
   CqlGroupPlan p;
   memset(&p, 0, sizeof(p));
@@ -1011,12 +1016,13 @@ static int group_exact(const CqlColumn* keys, uint32_t key_count, uint64_t rows,
     return -1;
   while ((1ull << p.low_bits) < rows) p.low_bits++;
   p.low_bits++;
-  if (!exact_units(&p, cols, rows)) return 0;
+  if (!exact_units(&p, cols, rows)) return -1;
   CqlKernel* k = kernel("cql_group_exact");
   CqlKernel* ke = kernel("cql_group_exact_emit");
   CqlKernel* kb = kernel("cql_group_direct_bits");
   CqlBuffer* pb = pooled("group_exact_plan", sizeof(CqlGroupPlan), CQLCUDA_BUFFER_READ_WRITE);
-  if (!k || !ke || !kb || !pb) return 0;
+  if (!k || !ke || !kb) return 0;
+  if (!pb) return -1;
   for (uint32_t i = 0; i < CQL_EXACT_KEYS; i++) cqlcuda_kernel_set_arg_buffer(k, i, keys[i < key_count ? i : 0].buffer);
   for (uint32_t i = 0; i < CQL_EXACT_COLUMNS; i++) cqlcuda_kernel_set_arg_buffer(k, 4 + i, i < p.column_count ? cols[i]->buffer : keys[0].buffer);
   /* how many groups: the hint, or the ranges' product where that is less */
@@ -1148,6 +1154,20 @@ static int group_exact(const CqlColumn* keys, uint32_t key_count, uint64_t rows,
     else table_slots *= 8;
   }
   return -1;
+}
+
+static int group_exact(const CqlColumn* keys, uint32_t key_count, uint64_t rows, uint32_t expr_count, const uint32_t* funcs,
+                       const CqlColumn* const* args, int use_fixed, uint32_t fixed_scales, uint64_t group_hint, uint64_t max_groups,
+                       uint64_t* out_group_count, uint64_t* out_repr_row, uint64_t* out_counts, double* out_results)
+{
+  int r = group_exact_run(keys, key_count, rows, expr_count, funcs, args, use_fixed, fixed_scales, group_hint, max_groups, out_group_count,
+                          out_repr_row, out_counts, out_results);
+  /* room for the form that may follow */
+  idle("group_exact_table");
+  idle("group_exact_out");
+  idle("group_exact_bits");
+  idle("group_exact_list");
+  return r;
 }
 
 int cqlops_group_hash(const CqlColumn* keys, uint32_t key_count, uint32_t expr_count, const uint32_t* funcs, const CqlColumn* const* args,

@@ -42,7 +42,12 @@ static CqlKernel* kernel(const char* name)
   return cqlcuda_kernel_alloc(name, (uint64_t)strlen(name));
 }
 
-/* a join key as the join kernels read it: f64 values (widened on the device) or raw strings */
+/* the scratch of a form that is done: room for the form that may follow it */
+static void idle(const char* name)
+{
+  cqlcuda_pool_idle(name, (uint64_t)strlen(name));
+}
+
 /* a join key as the buckets read it: raw bytes and offsets, or room for f64 values (join_key_widen fills it) */
 static int join_key(const CqlColumn* col, const char* name, CqlBuffer** data, CqlBuffer** off, int* is_str)
 {
@@ -71,8 +76,9 @@ static void join_key_widen(CqlBatch* b, CqlKernel* widen, const CqlColumn* col, 
 
 /* ---- the join of a build side whose keys do not repeat (cql_join_unique_build, _probe, _emit) ----
    One table of the build keys, one probe, and the pairs written in the probe rows' order: no bucket lists and no sort.
-   Gives way (-1) when a build key repeats, or a key is NaN, -0.0 or an integer past 2^53; the probe and the emit
-   leave at once then, so a build side with repeated keys pays for the table alone (35 us of 1M rows' millisecond). */
+   Gives way (-1) when a build key repeats, a key is NaN, -0.0 or an integer past 2^53, or there is no room for the table
+   and the pairs; the probe and the emit leave at once where a build key repeats, so that such a build side pays for the
+   table alone (35 us of 1M rows' millisecond). */
 static int unique_join_key(const CqlColumn* c)
 {
   return c->width == 0 && c->buffer && c->type != CQLOPS_TYPE_STRING8 &&
@@ -80,8 +86,8 @@ static int unique_join_key(const CqlColumn* c)
           c->type == CQLOPS_TYPE_U64 || c->type == CQLOPS_TYPE_I64);
 }
 
-static int unique_join(const CqlColumn* build_key, const CqlColumn* probe_key, int left_join, uint64_t* out_count, uint32_t* out_pairs,
-                       uint64_t out_capacity)
+static int unique_join_run(const CqlColumn* build_key, const CqlColumn* probe_key, int left_join, uint64_t* out_count, uint32_t* out_pairs,
+                           uint64_t out_capacity)
 {
   uint64_t brows = build_key->rows, prows = probe_key->rows;
   if (!unique_join_key(build_key) || !unique_join_key(probe_key) || brows > (1ull << 28)) return -1;
@@ -101,7 +107,8 @@ static int unique_join(const CqlColumn* build_key, const CqlColumn* probe_key, i
   CqlKernel* kb = kernel("cql_join_unique_build");
   CqlKernel* kp = kernel("cql_join_unique_probe");
   CqlKernel* ke = kernel("cql_join_unique_emit");
-  if (!table || !match || !pairs || !counts || !head || !kb || !kp || !ke) return 0;
+  if (!table || !match || !pairs || !counts || !head) return -1;
+  if (!kb || !kp || !ke) return 0;
   cqlcuda_kernel_set_arg_buffer(kb, 0, build_key->buffer);
   cqlcuda_kernel_set_arg_buffer(kp, 0, probe_key->buffer);
   CqlKernel* both[2] = { kb, kp };
@@ -144,6 +151,16 @@ static int unique_join(const CqlColumn* build_key, const CqlColumn* probe_key, i
   }
   *out_count = n;
   return 1;
+}
+
+static int unique_join(const CqlColumn* build_key, const CqlColumn* probe_key, int left_join, uint64_t* out_count, uint32_t* out_pairs,
+                       uint64_t out_capacity)
+{
+  int r = unique_join_run(build_key, probe_key, left_join, out_count, out_pairs, out_capacity);
+  idle("join_unique_table");
+  idle("join_unique_match");
+  idle("join_unique_pairs");
+  return r;
 }
 
 /* the bits of the row numbers below `rows` */
@@ -1122,8 +1139,8 @@ static int join_slots_finish(const CqlJoinAgg* q, uint32_t core_count, const uin
    is built on the device, each fact row's match is its group, and the totals are kept per group, so nothing is
    kept per dim row. The group values' range comes from the resident column's zone or from the values themselves
    (on the device past JHASH_HOST_VISITS of them: the host reads about a value a nanosecond, a launch and its wait cost
-   some 20 us). Gives way (-1) for duplicate keys, other group values, dim-side aggregates, narrow fact columns, and
-   more groups than a CTA's shared memory holds. */
+   some 20 us). Gives way (-1) for duplicate keys, other group values, dim-side aggregates, narrow fact columns,
+   more groups than a CTA's shared memory holds, and where there is no room for its tables. */
 #define JHASH_SMEM_BYTES (96u * 1024u)
 #define JHASH_SMEM_WANTED (32u * 1024u)
 #define JHASH_HOST_VISITS 16384u
@@ -1136,9 +1153,9 @@ static double order_key_value(uint64_t k)
   return v;
 }
 
-static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const uint32_t* core_funcs, const CqlColumn* const* core_cols,
-                               const uint32_t* core_of_expr, uint64_t max_groups, uint64_t* out_groups, uint64_t* out_group_dim_row,
-                               double* out_results)
+static int hash_join_aggregate_run(const CqlJoinAgg* q, uint32_t core_count, const uint32_t* core_funcs, const CqlColumn* const* core_cols,
+                                   const uint32_t* core_of_expr, uint64_t max_groups, uint64_t* out_groups, uint64_t* out_group_dim_row,
+                                   double* out_results)
 {
   const CqlColumn* fk = q->fact_key;
   uint64_t rows = fk->rows, D = q->dim_table_rows, visits = q->dim_rows ? q->dim_count : D;
@@ -1192,7 +1209,7 @@ static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const u
   CqlBuffer* vbuf = pooled("join_hash_visits", visit_list ? visits * 4 : 4, CQLCUDA_BUFFER_WRITE);
   CqlBuffer* kbuf = dev_keys ? dkc->buffer : pooled("join_hash_dim_keys", D * 4, CQLCUDA_BUFFER_WRITE);
   CqlBuffer* gbuf = dev_groups ? dgc->buffer : pooled("join_hash_group_values", gv ? D * 8 : 8, CQLCUDA_BUFFER_WRITE);
-  int ok = vbuf && kbuf && gbuf;
+  int room = vbuf && kbuf && gbuf, ok = room;
   /* the groups: the values from the smallest on */
   double vmin = 0.0, vmax = 0.0;
   int fits = 1, uploaded = 0;
@@ -1218,7 +1235,8 @@ static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const u
     CqlBuffer* rb = pooled("join_hash_range", 24, CQLCUDA_BUFFER_READ_WRITE);
     CqlKernel* kr = kernel("cql_join_group_range");
     uint64_t range[3] = { ~0ull, 0, 0 };
-    ok = rb && kr;
+    room = rb != NULL;
+    ok = room && kr;
     if (ok)
     {
       cqlcuda_kernel_set_arg_buffer(kr, 0, vbuf);
@@ -1242,7 +1260,7 @@ static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const u
   if (!ok || !fits || !(vmax - vmin <= 65535.0))
   {
     free(visit_list);
-    return ok ? -1 : 0;
+    return ok || !room ? -1 : 0;
   }
   uint64_t slots = gv ? (uint64_t)(vmax - vmin) + 1 : 1, E = core_count;
   uint32_t copies_log2 = 5;
@@ -1270,7 +1288,7 @@ static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const u
   {
     free(visit_list);
     free(host);
-    return 0;
+    return !table || !visit_group || !out ? -1 : 0;
   }
   uint64_t group_min_bits;
   memcpy(&group_min_bits, &vmin, 8);
@@ -1324,6 +1342,20 @@ static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const u
                                       out_group_dim_row, out_results);
   free(host);
   return result;
+}
+
+static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const uint32_t* core_funcs, const CqlColumn* const* core_cols,
+                               const uint32_t* core_of_expr, uint64_t max_groups, uint64_t* out_groups, uint64_t* out_group_dim_row,
+                               double* out_results)
+{
+  int r = hash_join_aggregate_run(q, core_count, core_funcs, core_cols, core_of_expr, max_groups, out_groups, out_group_dim_row, out_results);
+  idle("join_hash_table");
+  idle("join_hash_visit_groups");
+  idle("join_hash_visits");
+  idle("join_hash_dim_keys");
+  idle("join_hash_group_values");
+  idle("join_hash_slots");
+  return r;
 }
 
 /* -1 when the query does not take this path (the host pass then runs), else 0 / 1 */

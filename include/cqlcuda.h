@@ -94,6 +94,10 @@ void     cqlcuda_pool_begin_epoch(void);                       /* gpu_backend.h:
    (src/gpu/vulkan/gpu_vulkan.c:1577-1617), which the reference's failure tests call to start each run
    cold (src/tests/bench_alloc_fault.c:236-241). Does nothing while a batch is open or a lane is open. */
 uint64_t cqlcuda_pool_evict(uint64_t bytes_wanted);
+/* The pooled buffer of this name (of the calling thread's lane) holds nothing its operator still needs: it may be
+   evicted to make room at once, not only from the next epoch on. A lookup takes it back into use. For the scratch of
+   operator forms that another form may follow in the same query (no reference counterpart). */
+void     cqlcuda_pool_idle(const char* name, uint64_t name_len);
 CqlMemoryStats cqlcuda_memory_stats(void);                     /* gpu_backend.h:30 */
 uint32_t cqlcuda_sm_count(void);                               /* device property the kernels size grids by */
 

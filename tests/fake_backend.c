@@ -131,6 +131,12 @@ CqlBuffer* cqlcuda_buffer_alloc_pooled(const char* name, uint64_t name_len, uint
   b->size = size;
   return b;
 }
+void cqlcuda_pool_idle(const char* name, uint64_t name_len)
+{
+  char key[64];
+  snprintf(key, sizeof(key), "%.*s", (int)name_len, name);
+  note("idle", key);
+}
 CqlBuffer* cqlcuda_buffer_alloc_host_mapped(uint64_t size, void** out_host)
 {
   CqlBuffer* b = cqlcuda_buffer_alloc(size, 0, NULL);
