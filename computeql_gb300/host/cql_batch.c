@@ -2261,8 +2261,11 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
   RankThr* rank_thr = NULL;
   unsigned char* rank_cuts = NULL;
   ok = ok && slice_at;
-  ranks = ranks && ok && scan_n >= RANK_MIN_QUERIES && (mode == BATCH_RUN || mode == BATCH_PREPARE || mode == BATCH_SOURCE);
+  ranks = ranks && ok && (mode == BATCH_RUN || mode == BATCH_PREPARE || mode == BATCH_SOURCE);
   for (uint32_t sh = 0; ranks && sh < launch_shapes; sh++) ranks = rank_expr(launch_exprs[sh]);
+  /* whether batches of these shapes run as ranks from RANK_MIN_QUERIES queries on: this one may have fewer */
+  const int rank_shapes = ranks;
+  ranks = ranks && scan_n >= RANK_MIN_QUERIES;
   for (uint32_t c = 0; ranks && mode == BATCH_RUN && c < column_count; c++)
     ranks = !(((uint64_t)(uintptr_t)cqlcuda_buffer_device_pointer(columns[c].buffer)) & 15u);
   if (ranks) rank_thr = (RankThr*)malloc((size_t)scan_n * BATCH_MAX_SITES * sizeof(RankThr));
@@ -2394,11 +2397,14 @@ static int batch_run(CqlBatchCatalog* catalog, const CqlProgram* const* programs
     free(src);
     if (ok && mode == BATCH_PREPARE && ranks && view)
     {
-      /* a batch of the catalog's shapes whose cuts do not fit takes the register form */
+      /* a batch of the catalog's shapes with one query, or with a value outside its column's range, takes the register form */
       src = launch_source(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rows_per_thread, block, 0);
       ok = src && kernel_ready(src) != NULL;
       free(src);
     }
+    /* and one with more queries than were prepared together the rank form */
+    if (ok && mode == BATCH_PREPARE && rank_shapes && !ranks && view)
+      ok = rank_kernel(slice_exprs, slice_sites, ns, launch_types, sum_cols, sum_col_count, rank_form) != NULL;
   }
   if (ok && (mode == BATCH_SOURCE || mode == BATCH_PREPARE) && out_shapes) *out_shapes = shapes;
   if (mode == BATCH_PERSIST)

@@ -59,7 +59,10 @@ void fake_reset(void)
 {
   g_logged = 0;
   g_fail_name[0] = 0;
+  for (uint32_t i = 0; i < g_kernel_count; i++)   /* the generated kernels are compiled anew */
+    if (!strncmp(g_kernels[i].name, "qk_", 3)) g_kernels[i].name[0] = 0;
 }
+void fake_clear_log(void) { g_logged = 0; }
 void fake_fail_name(const char* name) { snprintf(g_fail_name, sizeof(g_fail_name), "%s", name); }
 uint32_t fake_log_count(void) { return g_logged; }
 const char* fake_log(uint32_t i) { return i < g_logged ? g_log[i] : ""; }

@@ -19,7 +19,7 @@ def load(directory):
                         *sources, "-lm", "-lpthread"], check=True)
         _lib = C.CDLL(path)
         N._bind(_lib, N.OPS_API)
-        for name, res, args in [("fake_reset", None, []), ("fake_fail_name", None, [C.c_char_p]), ("fake_log_count", C.c_uint32, []),
+        for name, res, args in [("fake_reset", None, []), ("fake_clear_log", None, []), ("fake_fail_name", None, [C.c_char_p]), ("fake_log_count", C.c_uint32, []),
                                 ("fake_log", C.c_char_p, [C.c_uint32]), ("fake_pooled_data", C.c_void_p, [C.c_char_p]),
                                 ("cqlcuda_buffer_alloc", C.c_void_p, [C.c_uint64, C.c_uint32, C.c_void_p])]:
             f = getattr(_lib, name)
