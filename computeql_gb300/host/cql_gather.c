@@ -3,7 +3,7 @@
  * host memory in selection order (selection_gather.comp modes 0/1, qe_selection_gather_column,
  * src/query_exec/query_exec.c:4371-4410, which the reference runs one column and one batch at a time).
  *
- * Here one batch uploads the selection once, gathers every column in one launch into one destination
+ * Here one batch uploads the selection once, gathers every column in one launch (65535 of them at most) into one destination
  * buffer (each column in a 16-byte-aligned section) and reads every section straight into the caller's
  * array. Raw strings take two batches: their lengths and an exclusive scan of them (the output offsets),
  * then a warp per row copies the bytes.
@@ -16,6 +16,7 @@
 #include <string.h>
 
 #define QE_GPU_WORKGROUP_SIZE 256
+#define GATHER_COLUMNS 65535u   /* a launch's columns: the grid's second dimension */
 
 static int refuse(const char* why)
 {
@@ -102,7 +103,6 @@ int cqlops_gather_rows(const CqlColumn* columns, uint32_t column_count, const ui
   if (column_count == 0 || count == 0) return 1;
   if (!columns || !out_values) return refuse("columns and outputs are required");
   if (!cqlops_rows_fit(count)) return 0;
-  if (column_count > 65535) return refuse("at most 65535 columns");
   uint32_t* params = (uint32_t*)calloc((size_t)column_count * 8, sizeof(uint32_t));
   uint64_t* section = (uint64_t*)malloc((size_t)column_count * sizeof(uint64_t));
   uint32_t* sizes = (uint32_t*)malloc((size_t)column_count * sizeof(uint32_t));
@@ -151,12 +151,16 @@ int cqlops_gather_rows(const CqlColumn* columns, uint32_t column_count, const ui
     {
       cqlcuda_batch_buffer_write(b, pbuf, params, (uint64_t)column_count * 32);
       cqlcuda_kernel_set_arg_buffer(k, 0, sel ? sel : pbuf);
-      cqlcuda_kernel_set_arg_buffer(k, 1, pbuf);
       cqlcuda_kernel_set_arg_buffer(k, 2, dest);
       cqlcuda_kernel_set_arg_u64(k, 0, count);
       cqlcuda_kernel_set_arg_u64(k, 1, given);
-      cqlcuda_kernel_set_arg_u64(k, 2, column_count);
-      cqlcuda_batch_kernel_execute(b, k, (uint32_t)count, QE_GPU_WORKGROUP_SIZE);
+      for (uint32_t first = 0; first < column_count; first += GATHER_COLUMNS)
+      {
+        uint32_t n = column_count - first < GATHER_COLUMNS ? column_count - first : GATHER_COLUMNS;
+        cqlcuda_kernel_set_arg_buffer_range(k, 1, pbuf, (uint64_t)first * 32, (uint64_t)n * 32);
+        cqlcuda_kernel_set_arg_u64(k, 2, n);
+        cqlcuda_batch_kernel_execute(b, k, (uint32_t)count, QE_GPU_WORKGROUP_SIZE);
+      }
       /* outputs laid out as the device sections are (one host block, each column at its section's offset):
          one read of the whole block; else a read a column */
       int contiguous = 1;
