@@ -1025,7 +1025,8 @@ static int group_exact_run(const CqlColumn* keys, uint32_t key_count, uint64_t r
   if (!pb) return -1;
   for (uint32_t i = 0; i < CQL_EXACT_KEYS; i++) cqlcuda_kernel_set_arg_buffer(k, i, keys[i < key_count ? i : 0].buffer);
   for (uint32_t i = 0; i < CQL_EXACT_COLUMNS; i++) cqlcuda_kernel_set_arg_buffer(k, 4 + i, i < p.column_count ? cols[i]->buffer : keys[0].buffer);
-  /* how many groups: the hint, or the ranges' product where that is less */
+  /* how many groups: the hint, or the rows or the ranges' product where those are less */
+  if (group_hint > rows) group_hint = rows;
   uint64_t expected = group_hint;
   if (product && (expected == 0 || expected > product)) expected = product <= EXACT_DIRECT_MAX || group_hint ? product : 0;
   if (group_hint && expected > group_hint) expected = group_hint;

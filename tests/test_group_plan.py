@@ -50,3 +50,10 @@ def test_the_number_and_the_copy_fit_64_bits(lib, form, hint):
     # fewer bits leave room for copies, so that the lanes of a warp do not meet
     if form == "u32 sparse" and hint in (1, 2, 50, 256):
         assert local and copies > 0
+
+
+@pytest.mark.parametrize("form", ["f64", "u32 sparse"])
+@pytest.mark.parametrize("hint", [ROWS + 1, 1 << 40, (1 << 62) + 1, (1 << 63) + 1, (1 << 64) - 1])
+def test_a_hint_past_the_rows(lib, form, hint):
+    """a hint of more groups than rows is met as one of as many"""
+    assert plan(lib, keys(lib, form), hint) == plan(lib, keys(lib, form), ROWS)
