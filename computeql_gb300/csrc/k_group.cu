@@ -156,7 +156,8 @@ static int launch_hll_rows(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaS
 // and 63 in the table, L = log2 rows + 1, wide enough that the rows' pieces add without a carry), and rounded
 // once when the group is listed. The sum does not depend on the order of the rows. A value outside that window
 // (over 48 binades below the column's largest for 10M rows) sets the status, and the caller takes the member
-// lists. Two of the three parts hold any value within 2^(62 - 2L) of the largest, so a row mostly costs two 64-bit
+// lists; the other CTAs meet the status a round later and leave too, so that such data costs little beside the lists.
+// Two of the three parts hold any value within 2^(62 - 2L) of the largest, so a row mostly costs two 64-bit
 // reductions; f64 reductions would cost one but round per row.
 //
 // What it replaced, per 10M rows: member lists (assign 640 us, scatter 575, reduce 460, prefix sums and ranges 100)
@@ -410,6 +411,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group_exact(CqlLaun
   for (uint64_t r0 = (uint64_t)blockIdx.x * THREADS + threadIdx.x; r0 < rows; r0 += step * EXACT_ROWS)
   {
     if (*(volatile uint32_t*)&s_stop) break;
+    const uint32_t stopped = threadIdx.x == 0 ? *(volatile uint32_t*)status : 0u;   // another CTA's; needed at the round's end
     unsigned long long id[EXACT_ROWS];
     uint32_t bad = 0, row[EXACT_ROWS];   // a row past the end reads the last one and is left out below
 #pragma unroll
@@ -488,7 +490,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group_exact(CqlLaun
       else if (v.type == 3) exact_column<LOCAL, 3>(v, row, sl, words, S, part, T, mn, mx, flags, pos_max, &wrong);
       else exact_column<LOCAL, 8>(v, row, sl, words, S, part, T, mn, mx, flags, pos_max, &wrong);
     }
-    if (wrong) *(volatile uint32_t*)&s_stop = 1;
+    if (wrong | stopped) *(volatile uint32_t*)&s_stop = 1;
   }
   if (wrong) atomicOr(status, wrong);
   if (!LOCAL) return;
