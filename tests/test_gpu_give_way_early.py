@@ -44,3 +44,49 @@ def test_group_by_values_outside_the_window(gpu, groups):
     row = k[r["repr_row"].astype(np.int64)]
     assert np.array_equal(r["counts"], counts[row]) and len(row) == (counts > 0).sum()
     assert np.allclose(r["results"][:, 1], sums[row], rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("where", ["all over", "first", "last"])
+def test_batch_with_values_outside_their_range(gpu, where):
+    from computeql_gb300 import ops
+    lib = gpu.load_cuda()
+    rng = np.random.default_rng(3)
+    w, v = rng.random(N), rng.random(N)      # (conditions on whole numbers of small range would be answered from a table)
+    bad = v.copy()
+    if where == "all over":
+        bad[::1009] = np.nan
+    else:
+        bad[0 if where == "first" else N - 1] = 1e9
+    wc = ops.Column.from_numpy(w)
+    cols = [{"w": wc, "v": ops.Column(ops.TYPE_F64, N, ops.DeviceBuffer(a.nbytes, a), zone=(0.0, 1.0), zone_map=False)} for a in (v, bad)]
+    progs = [[ops.Program(f"(< w {(q + 1) / 70!r})", c) for q in range(64)] for c in cols]
+    run = lambda p, form=8: ops.batch_aggregate(p, ["v"] * 64, form)
+    for p in progs:
+        run(p)
+    _, whole = nanoseconds(lib, gpu, "qk_batch_rank", lambda: run(progs[0]))
+    (c, s, _), early = nanoseconds(lib, gpu, "qk_batch_rank", lambda: run(progs[1]))
+    c8, s8, _ = run(progs[1], 8 | (1 << 24))
+    assert np.array_equal(c, c8) and np.array_equal(s.view(np.uint64), s8.view(np.uint64))
+    assert np.array_equal(c, [(w < (q + 1) / 70).sum() for q in range(64)])
+    assert whole > 0 and early > 0
+    if where != "last":
+        assert early < whole / 2, (early, whole)
+
+
+def test_batch_over_a_range_that_is_not_finite(gpu):
+    """a column of NaN and numbers, its range taken from it: the register form at once"""
+    from computeql_gb300 import ops
+    lib = gpu.load_cuda()
+    rng = np.random.default_rng(4)
+    n = 100_003
+    w, v = rng.random(n), rng.random(n)
+    v[::97] = np.nan
+    cols = {"w": ops.Column.from_numpy(w), "v": ops.Column.from_numpy(v), "d": ops.Column.from_numpy(rng.random(n))}
+    progs = [ops.Program(f"(< w {(q + 1) / 20!r})", cols) for q in range(16)]
+    (c, s, _), ranked = nanoseconds(lib, gpu, "qk_batch_rank", lambda: ops.batch_aggregate(progs, ["v"] * 16))
+    c8, s8, _ = ops.batch_aggregate(progs, ["v"] * 16, 8 | (1 << 24))
+    assert ranked == 0
+    assert np.array_equal(c, c8) and np.array_equal(s.view(np.uint64), s8.view(np.uint64))
+    # the other columns' batches still run as ranks
+    (c, s, _), ranked = nanoseconds(lib, gpu, "qk_batch_rank", lambda: ops.batch_aggregate(progs, ["d"] * 16))
+    assert ranked > 0 and np.array_equal(c, c8)
