@@ -1144,6 +1144,7 @@ static int join_slots_finish(const CqlJoinAgg* q, uint32_t core_count, const uin
 #define JHASH_SMEM_BYTES (96u * 1024u)
 #define JHASH_SMEM_WANTED (32u * 1024u)
 #define JHASH_HOST_VISITS 16384u
+#define JHASH_HOST_SAMPLE 1024u
 
 static double order_key_value(uint64_t k)
 {
@@ -1218,19 +1219,23 @@ static int hash_join_aggregate_run(const CqlJoinAgg* q, uint32_t core_count, con
     vmin = dgc->zone_min;
     vmax = dgc->zone_max;
   }
-  else if (ok && gv && visits <= JHASH_HOST_VISITS)
+  else if (ok && gv)
   {
+    /* on the host, all of few values; of more the first, since a column of other values mostly shows there, before the
+       values are uploaded (100003 keys and fractions: 2770 us by the host pass alone, 2860 with the values sent first) */
+    uint64_t looked = visits <= JHASH_HOST_VISITS ? visits : JHASH_HOST_SAMPLE;
     vmin = HUGE_VAL;
     vmax = -HUGE_VAL;
-    for (uint64_t v = 0; v < visits && fits; v++)
+    for (uint64_t v = 0; v < looked && fits; v++)
     {
       double x = gv[visit_list ? visit_list[v] : v];
       if (!(x >= -9.0e15 && x <= 9.0e15) || x != (double)(int64_t)x || (x == 0.0 && signbit(x))) fits = 0;
       if (x < vmin) vmin = x;
       if (x > vmax) vmax = x;
     }
+    if (!(vmax - vmin <= 65535.0)) fits = 0;
   }
-  else if (ok && gv)
+  if (ok && gv && !dev_groups && fits && visits > JHASH_HOST_VISITS)
   {
     CqlBuffer* rb = pooled("join_hash_range", 24, CQLCUDA_BUFFER_READ_WRITE);
     CqlKernel* kr = kernel("cql_join_group_range");

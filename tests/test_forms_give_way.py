@@ -36,13 +36,13 @@ def test_join_of_unique_keys(lib, name):
     assert "hash_join_build_count" in fake_backend.log(lib, "run")
 
 
-def join_aggregate(lib, dims, listed):
+def join_aggregate(lib, dims, listed, fraction=0.0):
     rng = np.random.default_rng(1)
     keys = rng.choice(2 ** 32, dims, replace=False).astype(np.uint32)
     fact = fake_backend.column(lib, ops.TYPE_U32, keys[rng.integers(0, dims, ROWS)], (0.0, 2.0 ** 32 - 1))
     value = fake_backend.column(lib, ops.TYPE_U32, np.ones(ROWS, np.uint32), (0.0, 1.0))
     funcs, fargs = np.array([0, 1], np.uint32), (C.c_void_p * 2)(None, C.addressof(value))
-    seg = (np.arange(dims) % 20).astype(np.float64)
+    seg = (np.arange(dims) % 20).astype(np.float64) + fraction
     gv = (C.c_void_p * 1)(seg.ctypes.data)
     visit = np.arange(0, dims, 2, dtype=np.uint64) if listed else None
     q = N.CqlJoinAgg(C.addressof(fact), 2, funcs.ctypes.data, C.addressof(fargs), None, keys.ctypes.data, dims, visit.ctypes.data if listed else None,
@@ -64,6 +64,13 @@ def test_join_aggregate_by_hash(lib, dims, listed, name):
     lib.fake_fail_name(name.encode())
     assert join_aggregate(lib, dims, listed), lib.cqlops_last_error()
     assert fake_backend.log(lib, "refused") == [name]
+    assert not {"cql_join_group_range", "cql_join_hash_probe"} & set(fake_backend.log(lib, "run"))
+
+
+@pytest.mark.parametrize("dims,listed", [(2003, True), (40_003, False), (40_003, True)])
+def test_group_values_that_are_fractions_are_not_sent(lib, dims, listed):
+    """such a column is met by the host pass: the values that show it are looked at before any is uploaded"""
+    assert join_aggregate(lib, dims, listed, 0.5), lib.cqlops_last_error()
     assert not {"cql_join_group_range", "cql_join_hash_probe"} & set(fake_backend.log(lib, "run"))
 
 
