@@ -62,6 +62,9 @@ static CqlBuffer* pooled(const char* name, uint64_t size, uint32_t flags)
   return cqlcuda_buffer_alloc_pooled(name, (uint64_t)strlen(name), size ? size : 4, flags, NULL);
 }
 
+/* scratch of fewer rows is a few MB: not worth the lookups, some us of a small call */
+#define IDLE_ROWS 65536u
+
 static void idle(const char* name)
 {
   cqlcuda_pool_idle(name, (uint64_t)strlen(name));
@@ -1163,11 +1166,13 @@ static int group_exact(const CqlColumn* keys, uint32_t key_count, uint64_t rows,
 {
   int r = group_exact_run(keys, key_count, rows, expr_count, funcs, args, use_fixed, fixed_scales, group_hint, max_groups, out_group_count,
                           out_repr_row, out_counts, out_results);
-  /* room for the form that may follow */
-  idle("group_exact_table");
-  idle("group_exact_out");
-  idle("group_exact_bits");
-  idle("group_exact_list");
+  if (rows >= IDLE_ROWS)   /* room for the form that may follow */
+  {
+    idle("group_exact_table");
+    idle("group_exact_out");
+    idle("group_exact_bits");
+    idle("group_exact_list");
+  }
   return r;
 }
 

@@ -42,7 +42,10 @@ static CqlKernel* kernel(const char* name)
   return cqlcuda_kernel_alloc(name, (uint64_t)strlen(name));
 }
 
-/* the scratch of a form that is done: room for the form that may follow it */
+/* The scratch of a form that is done: room for the form that may follow it. That of fewer rows is a few MB, not worth the
+   lookups, some us of a small call. */
+#define IDLE_ROWS 65536u
+
 static void idle(const char* name)
 {
   cqlcuda_pool_idle(name, (uint64_t)strlen(name));
@@ -157,9 +160,12 @@ static int unique_join(const CqlColumn* build_key, const CqlColumn* probe_key, i
                        uint64_t out_capacity)
 {
   int r = unique_join_run(build_key, probe_key, left_join, out_count, out_pairs, out_capacity);
-  idle("join_unique_table");
-  idle("join_unique_match");
-  idle("join_unique_pairs");
+  if (build_key->rows >= IDLE_ROWS || probe_key->rows >= IDLE_ROWS)
+  {
+    idle("join_unique_table");
+    idle("join_unique_match");
+    idle("join_unique_pairs");
+  }
   return r;
 }
 
@@ -1354,12 +1360,15 @@ static int hash_join_aggregate(const CqlJoinAgg* q, uint32_t core_count, const u
                                double* out_results)
 {
   int r = hash_join_aggregate_run(q, core_count, core_funcs, core_cols, core_of_expr, max_groups, out_groups, out_group_dim_row, out_results);
-  idle("join_hash_table");
-  idle("join_hash_visit_groups");
-  idle("join_hash_visits");
-  idle("join_hash_dim_keys");
-  idle("join_hash_group_values");
-  idle("join_hash_slots");
+  if (q->dim_table_rows >= IDLE_ROWS || (q->dim_rows && q->dim_count >= IDLE_ROWS))
+  {
+    idle("join_hash_table");
+    idle("join_hash_visit_groups");
+    idle("join_hash_visits");
+    idle("join_hash_dim_keys");
+    idle("join_hash_group_values");
+    idle("join_hash_slots");
+  }
   return r;
 }
 

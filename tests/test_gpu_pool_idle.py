@@ -15,7 +15,7 @@ def env(gpu):
     probe = ops.Column.from_numpy(rng.integers(0, 1 << 20, N).astype(np.uint32))
     key = ops.Column.from_numpy(rng.integers(0, 2 ** 32, N).astype(np.uint32) % np.uint32(100_003) * np.uint32(40_000))
     value = ops.Column.from_numpy(rng.integers(0, 1000, N).astype(np.uint32))
-    dims = rng.choice(2 ** 32, 3001, replace=False).astype(np.uint32)
+    dims = rng.choice(2 ** 32, 70_001, replace=False).astype(np.uint32)
     fact = ops.Column.from_numpy(dims[rng.integers(0, len(dims), N)])
     seg = rng.integers(0, 20, len(dims)).astype(np.float64)
 
@@ -36,7 +36,7 @@ def test_scratch_is_evictable_after_the_call(env, name):
     want = queries[name]()
     before = lib.cqlcuda_memory_stats()
     freed = lib.cqlcuda_pool_evict(2 ** 64 - 1)            # the same epoch: only what is idle goes
-    assert freed >= 3001 * 2 * 8 and lib.cqlcuda_memory_stats().pool_evictions > before.pool_evictions
+    assert freed >= 50_001 * 2 * 8 and lib.cqlcuda_memory_stats().pool_evictions > before.pool_evictions
     assert queries[name]() == want
 
 
