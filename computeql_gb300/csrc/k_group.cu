@@ -166,7 +166,11 @@ static int launch_hll_rows(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaS
 #define EXACT_ROWS 4
 #define EXACT_EMPTY 0xffffffffffffffffull
 #define EXACT_LOCAL_PROBES 64
+// The slots tried for a group in the table, a constant of the kernel (as a value it cost a hashed table of 333k groups 202 -> 380
+// us): in a half-full table the longest chain stays well below. A row that finds no room tries them one after another, some
+// 0.4 us each, so that a first table, whose size is a guess, takes few.
 #define EXACT_PROBES 256
+#define EXACT_GUESS_PROBES 64
 
 struct ExactTable
 {
@@ -376,7 +380,7 @@ __device__ __forceinline__ void exact_column(const ExactColumn& v, const uint32_
   }
 }
 
-template <bool LOCAL, bool DIRECT, int THREADS>
+template <bool LOCAL, bool DIRECT, int THREADS, uint32_t PROBES = EXACT_PROBES>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group_exact(CqlLaunch a, uint64_t rows)
 {
   extern __shared__ __align__(16) unsigned char local_mem[];
@@ -437,11 +441,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group_exact(CqlLaun
     }
     uint32_t sl[EXACT_ROWS];
 #pragma unroll
+    for (uint32_t i = 0; i < EXACT_ROWS; i++) sl[i] = 0xffffffffu;
+#pragma unroll
     for (uint32_t i = 0; i < EXACT_ROWS; i++)
     {
       uint64_t r = r0 + i * step;
-      sl[i] = 0xffffffffu;
-      if (r >= rows) continue;
+      if (r >= rows || wrong) continue;   // (once a row found no room, the next would look as long)
       if (((bad >> i) & 1u) || (!DIRECT && id[i] == EXACT_EMPTY))
       {
         wrong |= CQL_EXACT_KEY;
@@ -464,7 +469,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group_exact(CqlLaun
       else
       {
         bool claimed = false;
-        uint32_t s = DIRECT ? (uint32_t)id[i] : exact_slot(t.key, T, EXACT_PROBES, id[i], &claimed);
+        uint32_t s = DIRECT ? (uint32_t)id[i] : exact_slot(t.key, T, PROBES, id[i], &claimed);
         if (s >= T)
         {
           wrong |= CQL_EXACT_OVERFLOW;
@@ -507,9 +512,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group_exact(CqlLaun
     uint32_t g = DIRECT ? s >> copies_log2 : exact_slot(t.key, T, EXACT_PROBES, lkey[s] >> copies_log2, &claimed);
     if (g >= T)
     {
+      *(volatile uint32_t*)&s_stop = 1;
       atomicOr(status, CQL_EXACT_OVERFLOW);
-      continue;
     }
+    if (*(volatile uint32_t*)&s_stop) break;   // no room: its other groups would each try every slot again
     atomicAdd(&t.cnt[g], n);
     atomicMin(&t.row[g], lrow[s]);
     if (lflags[s]) atomicOr(&t.flags[g], lflags[s]);
@@ -615,6 +621,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) k_group_exact_emit(CqlLaunch a,
     return;
   }
   uint32_t first = blockIdx.x * GROUP_THREADS, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, mine = 0;
+#pragma unroll 8
   for (uint32_t s = threadIdx.x; s < first; s += GROUP_THREADS) mine += t.cnt[s] != 0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
@@ -635,18 +642,18 @@ __global__ void __launch_bounds__(GROUP_THREADS) k_group_exact_emit(CqlLaunch a,
 }
 
 // The launchers read the plan on the host: the operator layer puts the same plan in binding 12 (1) on the device and
-// names its shape in the words: word 2 local slots, 3 local bytes, word 4 direct, word 6 the table's slots.
-template <bool LOCAL, bool DIRECT, int THREADS>
+// names its shape in the words: word 2 local slots, 3 local bytes, word 4 direct, 5 the table is a guess, word 6 its slots.
+template <bool LOCAL, bool DIRECT, int THREADS, uint32_t PROBES = EXACT_PROBES>
 static int launch_exact_as(const CqlLaunch& a, uint64_t rows, size_t smem, int per_sm, cudaStream_t stream)
 {
-  const void* fn = (const void*)k_group_exact<LOCAL, DIRECT, THREADS>;
+  const void* fn = (const void*)k_group_exact<LOCAL, DIRECT, THREADS, PROBES>;
   if (LOCAL && smem > 40 * 1024)
   {
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
   uint32_t grid = cql_stream_grid((rows + THREADS * EXACT_ROWS - 1) / (THREADS * EXACT_ROWS), per_sm);
-  k_group_exact<LOCAL, DIRECT, THREADS><<<grid, THREADS, smem, stream>>>(a, rows);
+  k_group_exact<LOCAL, DIRECT, THREADS, PROBES><<<grid, THREADS, smem, stream>>>(a, rows);
   CQL_LAUNCH_CHECK();
   return 0;
 }
@@ -660,6 +667,7 @@ static int launch_group_exact(const CqlLaunch& a, uint32_t gws, uint32_t lws, cu
   bool direct = cql_word(a, 4) != 0;
   if (rows == 0) return 0;
   if (rows > 0x7fffffffull || slots == 0 || a.bytes[12] < sizeof(CqlGroupPlan) || a.bytes[14] < 4 || a.bytes[13] < a.push[4]) return (int)cudaErrorInvalidValue;
+  if (local_slots == 0 && !direct && cql_word(a, 5)) return launch_exact_as<false, false, 256, EXACT_GUESS_PROBES>(a, rows, 0, 4, stream);
   if (local_slots == 0)
     return direct ? launch_exact_as<false, true, 256>(a, rows, 0, 4, stream) : launch_exact_as<false, false, 256>(a, rows, 0, 4, stream);
   if (local_bytes > (uint32_t)g_cql_max_smem_optin - 2048) return (int)cudaErrorInvalidValue;

@@ -877,6 +877,10 @@ static int group_direct(const CqlColumn* key, uint32_t expr_count, const uint32_
 #define EXACT_TABLE_BYTES (8ull << 30)
 #define EXACT_EMIT_SLOTS 65536u
 #define EXACT_ONE_READ_BYTES (192ull << 10)
+/* Where the number of groups is unknown, or more than the hint: a table of a 16th of the rows first, a guess (the kernel then
+   gives up on a group soon); where that has no room, one with room for every row if it is small enough to fill in some 20 us,
+   else tables of 8 times as many slots. */
+#define EXACT_WHOLE_BYTES (128ull << 20)
 
 static uint64_t pow2_from(uint64_t n)
 {
@@ -1039,6 +1043,7 @@ static int group_exact_run(const CqlColumn* keys, uint32_t key_count, uint64_t r
   int local = 1;
   uint64_t slot_bytes = (p.direct ? 0 : 8) + 8ull * (p.mins + p.maxs) + 16ull * p.sums + 12;
   uint64_t table_slots = 0;
+  int guess = 0;
   for (int attempt = 0; attempt < 12; attempt++)
   {
     p.local_slots = 0;
@@ -1063,6 +1068,7 @@ static int group_exact_run(const CqlColumn* keys, uint32_t key_count, uint64_t r
     {
       uint64_t want = local ? 2ull * p.local_slots >> p.copies_log2 : expected ? 2 * expected : rows / 16;
       table_slots = pow2_from(want < 1024 ? 1024 : want);
+      guess = !local && !expected;
     }
     if (!p.direct && table_slots > most) table_slots = most;
     if (table_slots > (1ull << 30)) return -1;
@@ -1085,7 +1091,7 @@ static int group_exact_run(const CqlColumn* keys, uint32_t key_count, uint64_t r
     cqlcuda_kernel_set_arg_buffer_range(k, 14, ob, 16, 4);
     cqlcuda_kernel_set_arg_u64(k, 0, rows);
     cqlcuda_kernel_set_arg_u64(k, 1, (uint64_t)p.local_slots | ((uint64_t)p.local_slots * slot_bytes) << 32);
-    cqlcuda_kernel_set_arg_u64(k, 2, p.direct);
+    cqlcuda_kernel_set_arg_u64(k, 2, (uint64_t)p.direct | (uint64_t)(guess && table_slots < most) << 32);
     cqlcuda_kernel_set_arg_u64(k, 3, p.slots);
     cqlcuda_kernel_set_arg_u64(k, 4, ones + zeros);
     cqlcuda_kernel_set_arg_buffer(ke, 0, tab);
@@ -1149,13 +1155,14 @@ static int group_exact_run(const CqlColumn* keys, uint32_t key_count, uint64_t r
     if (status & (CQL_EXACT_RANGE | CQL_EXACT_KEY)) return -1;
     /* more groups than expected: the table in device memory next, then a larger one */
     if (p.direct || (!local && table_slots >= most)) return -1;
+    guess = local;
     if (local)
     {
       local = 0;
       table_slots = pow2_from(4 * expected > rows / 16 ? 4 * expected : rows / 16);
       if (table_slots < 4096) table_slots = 4096;
     }
-    else table_slots *= 8;
+    else table_slots = (ones + zeros) / p.slots * most <= EXACT_WHOLE_BYTES ? most : 8 * table_slots;
   }
   return -1;
 }
