@@ -47,9 +47,11 @@ class _ResultBlocks:
     LIMIT, MAPPED, SMALL, COPIED, SHARE = 256 << 20, 16 << 30, 1 << 20, 64 << 10, 8
 
     class _Lease:
+        __slots__ = ("blocks", "memory", "touched", "__array_interface__")
+
         def __init__(self, blocks, memory, touched, count, dtype):
             self.blocks, self.memory, self.touched = blocks, memory, touched
-            self.__array_interface__ = {"shape": (count,), "typestr": dtype.str, "data": (memory.ctypes.data, False), "version": 3}
+            self.__array_interface__ = {"shape": (count,), "typestr": dtype.str, "data": (memory.__array_interface__["data"][0], False), "version": 3}
 
         def __del__(self):
             self.blocks.returned.append((self.memory, self.touched))     # deque.append takes no lock
@@ -63,16 +65,21 @@ class _ResultBlocks:
 
     def _sort_in(self):
         """with the lock: the returned blocks among the free ones, within the limits"""
+        if not self.returned:
+            return
         while self.returned:
             self.free.append(self.returned.popleft())
-        touched, mapped = sum(t for _, t in self.free), sum(m.nbytes for m, _ in self.free)
+        touched = mapped = 0
+        for memory, held in self.free:
+            touched += held
+            mapped += memory.nbytes
         while touched > self.LIMIT or mapped > self.MAPPED:
             memory, held = self.free.pop(0)
             touched, mapped = touched - held, mapped - memory.nbytes
 
     def _settle(self):
         # Runs in destructors too, so it never waits: who holds the lock looks again once it is free.
-        while self.returned and self.lock.acquire(blocking=False):
+        while self.returned and self.lock.acquire(False):
             try:
                 self._sort_in()
             finally:
@@ -85,12 +92,16 @@ class _ResultBlocks:
         size = count * dtype.itemsize
         if size < self.SMALL:
             return np.empty(count, dtype=dtype)
+        at, memory, touched = -1, None, 0
         with self.lock:
             self._sort_in()
-            fits = [i for i, (m, t) in enumerate(self.free) if m.nbytes >= size and t <= self.SHARE * size]
-            at = min(fits, key=lambda i: self.free[i][0].nbytes, default=None)
-            memory, touched = self.free.pop(at) if at is not None else (None, 0)
-        self._settle()
+            for i, (m, t) in enumerate(self.free):       # the smallest that is large enough and does not hold too much
+                if m.nbytes >= size and t <= self.SHARE * size and (at < 0 or m.nbytes < self.free[at][0].nbytes):
+                    at = i
+            if at >= 0:
+                memory, touched = self.free.pop(at)
+        if self.returned:
+            self._settle()
         if memory is None:
             memory = np.empty(size + size // 8, dtype=np.uint8)          # a little more: the next result may be larger
         lease = self._Lease(self, memory, max(touched, size), count, dtype)
