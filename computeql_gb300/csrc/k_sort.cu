@@ -657,7 +657,7 @@ static int launch_radix_scatter(const CqlLaunch& a, uint32_t gws, uint32_t lws, 
 #define PREFIX_SAMPLE 2048u
 #define RUN_THREADS 256
 #define RUN_TILE 1024
-#define RUN_HALO 64
+#define RUN_HALO 128
 #define WORD_SIGN 0x8000000000000000ull
 
 struct SortPlan
@@ -1031,6 +1031,13 @@ __device__ __noinline__ int sort_compare_rest(const SortCols* c, const SortPlan*
   return 0;
 }
 
+// whether row j of a run belongs behind the row after it, which shares its prefix
+__device__ __forceinline__ bool run_out_of_order(const SortCols* c, const SortPlan* p, const uint32_t* s_row, const unsigned long long* s_word, int j)
+{
+  if (s_word[j] != s_word[j + 1]) return s_word[j] > s_word[j + 1];
+  return p->rest + 1 < c->keys && sort_compare_rest(c, p, s_row[j], s_row[j + 1]) > 0;
+}
+
 // A row of a run: where it belongs, by counting the rows of the run before it. Runs longer than RUN_HALO are only checked.
 __device__ __noinline__ int run_place(const SortCols* c, const SortPlan* p, const uint32_t* s_prefix, const uint32_t* s_row, const unsigned long long* s_word,
                                       int j, int lo, int hi, bool* unsorted)
@@ -1043,9 +1050,7 @@ __device__ __noinline__ int run_place(const SortCols* c, const SortPlan* p, cons
   if (right - left + 1 > RUN_HALO)
   {
     // too long to rank (every row of the run finds so): fine when it is in order as it is
-    if (j + 1 < hi && s_prefix[j + 1] == v &&
-        (s_word[j] > s_word[j + 1] || (s_word[j] == s_word[j + 1] && more && sort_compare_rest(c, p, s_row[j], s_row[j + 1]) > 0)))
-      *unsorted = true;
+    if (j + 1 < hi && s_prefix[j + 1] == v && run_out_of_order(c, p, s_row, s_word, j)) *unsorted = true;
     return j;
   }
   unsigned long long w = s_word[j];
@@ -1130,6 +1135,23 @@ __global__ void __launch_bounds__(RUN_THREADS) k_sort_runs(CqlLaunch a, uint64_t
       s_word[j] = sort_distance_of(c, p, p.rest, s_row[j]);
     }
     __syncthreads();
+    // Runs of equal keys, in order as the passes left them, are most of what a column of few values has: when no row of the tile
+    // and its halo comes before the one ahead of it, each stays (5M rows of 300 values: the kernel 298 us without this)
+    bool off = false;
+    for (uint32_t left = in_run; left && !off; left &= left - 1u)
+    {
+      int u = __ffs(left) - 1, j = u < per ? RUN_HALO + u * RUN_THREADS + (int)threadIdx.x : halo;
+      off = j + 1 < hi && s_prefix[j + 1] == s_prefix[j] && run_out_of_order(&c, &p, s_row, s_word, j);
+    }
+    if (!__syncthreads_or(off))
+    {
+      for (uint32_t left = in_run & ((1u << per) - 1u); left; left &= left - 1u)
+      {
+        int j = RUN_HALO + (__ffs(left) - 1) * RUN_THREADS + (int)threadIdx.x;
+        out[tile + (uint64_t)j - RUN_HALO] = s_row[j];
+      }
+      continue;
+    }
     for (uint32_t left = in_run & ((1u << per) - 1u); left; left &= left - 1u)
     {
       int j = RUN_HALO + (__ffs(left) - 1) * RUN_THREADS + (int)threadIdx.x;
