@@ -81,27 +81,21 @@ double cqlops_hll_estimate(const uint32_t* registers, uint64_t m_count)
   double m = (double)m_count;
   double alpha = m_count == 16 ? 0.673 : m_count == 32 ? 0.697 : m_count == 64 ? 0.709 : 0.7213 / (1.0 + 1.079 / m);
   double sum = 0.0;
-  uint64_t zeros = 0, of[64] = { 0 };
-  /* the terms are powers of two: below 2^-40 apart from 4096 registers on, their sum is exact in any order, so the
-     registers are counted by value (a division a register took 4 us a group of 1024) */
+  uint64_t zeros = 0, whole = 0;
   uint32_t most = 0;
+  /* the terms are powers of two: with none below 2^-40 and 4096 of them their sum is exact in any order, and a whole number
+     of 2^-40 (1024 registers: 0.4 us; 0.75 by a division each, and 2 where counts by value were kept, which wait for one
+     another when most registers are alike) */
   for (uint64_t i = 0; i < m_count; i++)
   {
-    if (registers[i] > most) most = registers[i];
-    of[registers[i] & 63u]++;
+    const uint32_t r = registers[i];
+    most = r > most ? r : most;
+    zeros += r == 0;
+    whole += (1ull << 40) >> (r & 63u);
   }
-  zeros = m_count ? of[0] : 0;
-  if (most <= 40 && m_count <= 4096)
-    for (uint32_t r = 0; r <= most; r++) sum += (double)of[r] / (double)((uint64_t)1 << r);
+  if (most <= 40 && m_count <= 4096) sum = (double)whole / (double)(1ull << 40);
   else
-  {
-    zeros = 0;
-    for (uint64_t i = 0; i < m_count; i++)
-    {
-      sum += 1.0 / (double)((uint64_t)1 << registers[i]);
-      if (registers[i] == 0) zeros++;
-    }
-  }
+    for (uint64_t i = 0; i < m_count; i++) sum += 1.0 / (double)((uint64_t)1 << registers[i]);
   double estimate = alpha * m * m / sum;
   if (estimate <= 2.5 * m && zeros > 0) estimate = m * log(m / (double)zeros);
   return estimate;
