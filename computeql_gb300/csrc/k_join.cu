@@ -1344,11 +1344,14 @@ template <int FORM>
 __global__ void __launch_bounds__(JOIN_THREADS) k_join_unique_build(CqlLaunch a, uint64_t rows)
 {
   unsigned long long* table = (unsigned long long*)a.buf[1];
-  uint32_t log2_size = cql_word(a, 2), mask = (1u << log2_size) - 1u, type = cql_word(a, 6), bad = 0;
+  const volatile uint32_t* status = (const volatile uint32_t*)a.buf[2];
+  uint32_t log2_size = cql_word(a, 2), mask = (1u << log2_size) - 1u, type = cql_word(a, 6), bad = 0, round = 0;
   for (uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += (uint64_t)gridDim.x * blockDim.x)
   {
     unsigned long long key = juniq_key<FORM>(a.buf[0], type, row, &bad);
-    if (FORM != 0 && key == JUNIQ_EMPTY) continue;   // flagged above
+    // a key that repeats, met by any thread, ends the build: the buckets take the rows. 10M rows of 3 a key and 100k probes
+    // 1230 us without; looked for at every row it cost 1M unique rows 32 us instead of 29
+    if (bad || ((round++ & 3u) == 1u && *status)) break;
     uint32_t slot = juniq_slot<FORM>(key, log2_size);
     unsigned long long entry = FORM == 0 ? (row << 32) | key : key;
     for (uint32_t p = 0; p <= mask; p++)   // at most half the slots are taken
@@ -1366,6 +1369,7 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join_unique_build(CqlLaunch a,
       }
       slot = (slot + 1u) & mask;
     }
+    if (bad) break;
   }
   if (bad) atomicOr((uint32_t*)a.buf[2], bad);
 }
@@ -1392,9 +1396,9 @@ template <int FORM>
 __global__ void __launch_bounds__(JUNIQ_THREADS, JUNIQ_CTAS_PER_SM) k_join_unique_probe(CqlLaunch a, uint64_t rows, uint64_t rows_per_cta)
 {
   __shared__ uint32_t s_count;
-  if (*(volatile const uint32_t*)a.buf[2] & 1u) return;   // a build key repeats
   if (threadIdx.x == 0) s_count = 0;
-  __syncthreads();
+  // a build key repeats or is none (another CTA may set the word for a probe key meanwhile: one thread looks for all)
+  if (__syncthreads_or(threadIdx.x == 0 && *(volatile const uint32_t*)a.buf[2] != 0u)) return;
   const unsigned long long* table = (const unsigned long long*)a.buf[1];
   uint32_t* match_out = (uint32_t*)a.buf[3];
   uint32_t log2_size = cql_word(a, 2), mask = (1u << log2_size) - 1u, type = cql_word(a, 6), bad = 0, count = 0;

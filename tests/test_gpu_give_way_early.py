@@ -90,3 +90,26 @@ def test_batch_over_a_range_that_is_not_finite(gpu):
     # the other columns' batches still run as ranks
     (c, s, _), ranked = nanoseconds(lib, gpu, "qk_batch_rank", lambda: ops.batch_aggregate(progs, ["d"] * 16))
     assert ranked > 0 and np.array_equal(c, c8)
+
+
+@pytest.mark.parametrize("kind", ["u32", "f64", "i64"])
+def test_join_whose_build_keys_repeat(gpu, kind):
+    from computeql_gb300 import ops
+    lib = gpu.load_cuda()
+    rng = np.random.default_rng(5)
+    n, probes = 10_000_019, 3001
+    unique = rng.permutation(n)
+    repeated = unique % (n // 3)
+    at = rng.integers(0, n, probes)
+    dtype = {"u32": np.uint32, "f64": np.float64, "i64": np.int64}[kind]
+    kinds = {"u32": ops.TYPE_U32, "f64": ops.TYPE_F64, "i64": ops.TYPE_I64}
+    cols = [ops.Column(kinds[kind], len(a), ops.DeviceBuffer(a.nbytes, a), zone_map=False) for a in (unique.astype(dtype), repeated.astype(dtype), at.astype(dtype))]
+    run = lambda b: ops.hash_join(b, cols[2])
+    for b in cols[:2]:
+        run(b)
+    (n0, pairs), whole = nanoseconds(lib, gpu, "cql_join_unique_build", lambda: run(cols[0]))
+    assert n0 == probes and np.array_equal(unique[pairs[:, 1]], at[pairs[:, 0]])
+    (n1, pairs), early = nanoseconds(lib, gpu, "cql_join_unique_build", lambda: run(cols[1]))
+    counts = np.bincount(repeated, minlength=n)
+    assert n1 == counts[at].sum() and np.array_equal(repeated[pairs[:, 1]], at[pairs[:, 0]])
+    assert early < whole / 2, (early, whole)
