@@ -10,7 +10,7 @@
 // cql_hll_rows: the HyperLogLog registers of whole columns, for a table or per value of a small-range key:
 // binding 0 the key (u32 words; the first column again without a key), 1..8 the columns, 9 the registers
 // (u32, zero before) [key value][column][2^10]; word 0 rows, 2 the columns, 4 their CQL types (4 bits each),
-// 6 the key's values (0: no key), 8 its smallest (bits). A row whose key lies outside the values is left out.
+// 6 the key's values (at most 64; 0: no key), 8 its smallest (bits). A row whose key lies outside the values is left out.
 //
 // The update is one max per row on few registers, so the only traffic it needs is the column itself. Without a
 // key a CTA keeps the 1024 registers in shared memory and merges them once (the member reduce read and wrote them
@@ -22,6 +22,7 @@
 #define HLL_P 10
 #define HLL_REGS (1u << HLL_P)
 #define HLL_ROWS 8
+#define HLL_VALUES 64   // what the operators number by a small-range key
 
 template <int TYPE>
 __device__ __forceinline__ unsigned long long value_bits(unsigned long long raw)
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) k_hll_keyed(const uint32_t* key
     {
       uint32_t bucket;
       cql_hll_place(value_bits<TYPE>(raw[i]), HLL_P, &bucket, &rho[i]);
-      at[i] = at[i] < values ? (at[i] * columns + column) * HLL_REGS + bucket : 0xffffffffu;   // values x columns <= 2^16
+      at[i] = at[i] < values ? (at[i] * columns + column) * HLL_REGS + bucket : 0xffffffffu;   // values x columns <= 2^9
     }
 #pragma unroll
     for (uint32_t i = 0; i < HLL_ROWS; i++) held[i] = at[i] != 0xffffffffu ? __ldcg(&out[at[i]]) : 0xffffffffu;
@@ -115,7 +116,7 @@ static int launch_hll_rows(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaS
   uint64_t rows = a.push[0];
   uint32_t columns = cql_word(a, 2), types = cql_word(a, 4), values = cql_word(a, 6), kmin = cql_word(a, 8);
   if (rows == 0 || columns == 0) return 0;
-  if (columns > 8 || rows > 0xffffffffull || values > 8192 || a.bytes[9] < (uint64_t)(values ? values : 1) * columns * HLL_REGS * 4 ||
+  if (columns > 8 || rows > 0xffffffffull || values > HLL_VALUES || a.bytes[9] < (uint64_t)(values ? values : 1) * columns * HLL_REGS * 4 ||
       (values && a.bytes[0] < rows * 4))
     return (int)cudaErrorInvalidValue;
   for (uint32_t j = 0; j < columns; j++)
@@ -161,8 +162,8 @@ static int launch_hll_rows(const CqlLaunch& a, uint32_t gws, uint32_t lws, cudaS
 // reductions; f64 reductions would cost one but round per row.
 //
 // What it replaced, per 10M rows: member lists (assign 640 us, scatter 575, reduce 460, prefix sums and ranges 100)
-// for 1000 groups of two keys, this form 164 (187 while the types were tested for every row). For 1M groups of one key, assign 337, scatter 143, reduce 122, ranges,
-// sums and compaction 230, this form 295 with the listing of the groups.
+// for 1000 groups of two keys, this form 155 and the listing 10. For 1M groups of one key, assign 337, scatter 143, reduce
+// 122, ranges, sums and compaction 230, this form 209 and the listing of the groups 70.
 #define EXACT_ROWS 4
 #define EXACT_EMPTY 0xffffffffffffffffull
 #define EXACT_LOCAL_PROBES 64

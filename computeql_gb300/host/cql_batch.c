@@ -840,7 +840,7 @@ static char* batch_source_tiled(char** shape_exprs, const uint32_t* shape_sites,
    interval compares, mask assembly, predicated 64-bit adds, five reductions every 8 rows). This one spends
    about 8, plus about 290 per 32 rows of 8 columns for the ranks and planes, and is bound by the shared
    memory the queries read (80 % of its wavefronts). Over 50M rows of 4 u32 and 4 f64 columns: 64 queries
-   6.1 -> 1.76 ms, 8 queries 2.0 -> 0.86; over 300 thousand rows 166 -> 107 us and 92 -> 61. Two queries of one
+   6.1 -> 1.77 ms, 8 queries 2.0 -> 0.87; over 300 thousand rows 166 -> 110 us and 92 -> 61. Two queries of one
    column sharing a warp's reads were slower (1.9 to 3.2 ms): the registers they take, or their code in the
    instruction cache, cost more than the reads.
 

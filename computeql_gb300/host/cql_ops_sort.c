@@ -164,8 +164,9 @@ static int sort_enqueue(CqlBatch* b, const CqlColumn* keys, uint32_t key_count, 
    cql_sort_runs, csrc/k_sort.cu) ----
    -1: the keys' rows share prefixes too often (a sample says so, or the runs pass found a long run out of order), and the
    passes over every digit sort them; top_bits then says below which bit each key varies. From SORT_PREFIX_MIN_ROWS rows
-   on: the ranges are read back before the passes are queued, a wait of some 15 us, against four passes saved or more (17000 rows by one
-   f64 key 184 to 155 us, by f64 and u32 251 to 142; 2M rows 364 and 480 to 282 and 288). */
+   on: the ranges are read back before the passes are queued, a wait of some 15 us, against four passes saved or more (17000 rows
+   by one f64 key 172 to 145 us, by f64 and u32 250 to 146; 2M rows 348 and 479 to 276 and 293). Where the sample sends the rows
+   back to the passes, those 20 to 45 us are lost: 300k rows by a price and a u32 252 to 282, 5M rows 735 to 767. */
 #define SORT_PREFIX_MIN_ROWS 16384u
 #define SORT_SAMPLE 2048ull
 #define SORT_RUN_ROWS 16.0   /* the runs pass takes up to 128 rows; 20M rows that share a prefix by 40: 2.5 ms, the passes 3.7 */

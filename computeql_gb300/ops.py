@@ -115,8 +115,9 @@ class _ResultBlocks:
     def cut(self, array, count, used):
         """The first `count` values of an array from `take`, all that was written of it."""
         part = array[:count]
-        held = max([note(part.nbytes) for note in used], default=array.nbytes)
-        return part.copy() if part.nbytes < self.COPIED or part.nbytes * self.SHARE < held else part
+        size = part.nbytes
+        held = used[0](size) if used else array.nbytes
+        return part.copy() if size < self.COPIED or size * self.SHARE < held else part
 
 
 _results = _ResultBlocks()

@@ -252,7 +252,7 @@ int cqlops_group_dense(const CqlColumn* key, uint64_t rows, uint32_t expr_count,
    key order, each represented by its first row; automatic takes it when it
    applies and some argument is not a decimal of at most 6 places, which path 2 finalizes as the
    reference does). Automatic also answers numeric keys that number in one 64-bit word from tables of
-   exact sums in one pass, and APPROX_COUNT_DISTINCT of the whole table or of a key of up to 8192 values
+   exact sums in one pass, and APPROX_COUNT_DISTINCT of the whole table or of a key of up to 64 values
    from one pass over the column; out_path then receives the path they stand for. Per dense group g:
    out_repr_row[g] (a row of the group), out_counts[g], out_results[g*expr_count + e]. out_path receives
    the path taken (1, 2, 3, or 4: tables indexed by a whole-number key of a wide dense range). */
