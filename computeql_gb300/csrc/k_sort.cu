@@ -653,7 +653,8 @@ static int launch_radix_scatter(const CqlLaunch& a, uint32_t gws, uint32_t lws, 
 // to 4000 differ from bit 62 down, but span 2^56, so the prefix holds 28 bits of their fractions and not 21 (20M
 // lognormal rows: most rows in runs, 407 us for the runs, against 125).
 //
-// 20M rows by (f64 DESC, u32): twelve passes over 12- and 8-byte pairs took 2.43 ms of kernels, this form 0.89: ranges 61 us, sample 17, prefixes 74, the four passes 612, runs 125.
+// 20M rows by (f64 DESC, u32): twelve passes over 12- and 8-byte pairs took 2.43 ms of kernels, this form 0.89: ranges
+// 61 us, sample 17, prefixes 74, the four passes 600, runs 133.
 #define PREFIX_SAMPLE 2048u
 #define RUN_THREADS 256
 #define RUN_TILE 1024
@@ -1128,7 +1129,8 @@ __global__ void __launch_bounds__(RUN_THREADS) k_sort_runs(CqlLaunch a, uint64_t
       else if (u < per) out[tile + (uint64_t)j - RUN_HALO] = row[u];
     }
     // most tiles have a few rows in runs: their words are read now, all rows' loads in flight together
-    if (!__syncthreads_or((int)in_run)) continue;
+    const int runners = __syncthreads_count(in_run != 0);   // threads that hold such a row
+    if (runners == 0) continue;
     for (uint32_t left = in_run; left; left &= left - 1u)
     {
       int u = __ffs(left) - 1, j = u < per ? RUN_HALO + u * RUN_THREADS + (int)threadIdx.x : halo;
@@ -1136,14 +1138,15 @@ __global__ void __launch_bounds__(RUN_THREADS) k_sort_runs(CqlLaunch a, uint64_t
     }
     __syncthreads();
     // Runs of equal keys, in order as the passes left them, are most of what a column of few values has: when no row of the tile
-    // and its halo comes before the one ahead of it, each stays (5M rows of 300 values: the kernel 298 us without this)
+    // and its halo comes before the one ahead of it, each stays (5M rows of 300 values: the kernel 298 us without this). Looked
+    // for where nearly every thread holds such a row
     bool off = false;
-    for (uint32_t left = in_run; left && !off; left &= left - 1u)
+    for (uint32_t left = runners >= RUN_THREADS - 6 ? in_run : 0u; left && !off; left &= left - 1u)
     {
       int u = __ffs(left) - 1, j = u < per ? RUN_HALO + u * RUN_THREADS + (int)threadIdx.x : halo;
       off = j + 1 < hi && s_prefix[j + 1] == s_prefix[j] && run_out_of_order(&c, &p, s_row, s_word, j);
     }
-    if (!__syncthreads_or(off))
+    if (runners >= RUN_THREADS - 6 && !__syncthreads_or(off))
     {
       for (uint32_t left = in_run & ((1u << per) - 1u); left; left &= left - 1u)
       {
